@@ -77,7 +77,7 @@ __device__ __forceinline__ void emit_relation(u64 p, u64 M, u64 q, u32 item, Raw
 constexpr u32 kSegWords = 2048;
 constexpr u32 kSieveThreads = 256;
 constexpr u32 kNumPattern = 10;               // 3..31: whole-word patterns, no atomics
-constexpr u32 kNumMedium = 171;               // primes below 1024: all threads share each prime
+constexpr u32 kNumMedium = 171;               // primes below 1024: a warp's lanes share each prime
 
 // Index j >= 0 of the first odd multiple v0 + 2j of q with v0 + 2j >= v0 (v0 odd).
 __device__ __forceinline__ u32 first_odd_multiple(u64 v0, u32 q, u64 rcp) {
@@ -162,17 +162,31 @@ __device__ void sieve_segment(SieveShared<W>& sh, u64 v0, u32 len, u32 n_primes,
             if (i < len) atomicAnd(&sh.bits[i >> 5], ~(1u << (i & 31)));
         }
     }
-    // 2. primes 37..1021: all threads share each prime.
-    for (u32 k = kNumPattern; k < n_med; ++k) {
+    // 2. primes 37..1021: the lanes of a warp share each prime, every eighth
+    // prime a warp (all threads on each prime leaves most of them without a
+    // multiple from q = 256 on, in a segment of 65,536: 2^28 integers at 10^12
+    // took 219 us, now 175).
+    for (u32 k = kNumPattern + warp; k < n_med; k += kSieveThreads / 32) {
         const u32 q = t.sp[k];
-        for (u32 i = sh.med_start[k] + tid * q; i < len; i += kSieveThreads * q)
+        for (u32 i = sh.med_start[k] + lane * q; i < len; i += 32 * q)
             atomicOr(&sh.bits[i >> 5], 1u << (i & 31));
     }
     // 3. primes 1031..65521: one thread per prime.
+    // (the next prime's loads are in flight while this one strikes)
+    u32 q = 0;
+    u64 rcp = 0;
+    if (kNumMedium + tid < n_primes) {
+        q = t.sp[kNumMedium + tid];
+        rcp = t.rcp[kNumMedium + tid];
+    }
     for (u32 k = kNumMedium + tid; k < n_primes; k += kSieveThreads) {
-        const u32 q = t.sp[k];
-        const u64 j = first_strike(v0, q, t.rcp[k]);
+        const u32 next = min(k + kSieveThreads, n_primes - 1);
+        const u32 q_next = t.sp[next];
+        const u64 rcp_next = t.rcp[next];
+        const u64 j = first_strike(v0, q, rcp);
         for (u64 i = j; i < len; i += q) atomicOr(&sh.bits[(u32)i >> 5], 1u << ((u32)i & 31));
+        q = q_next;
+        rcp = rcp_next;
     }
     __syncthreads();
 
@@ -2244,17 +2258,36 @@ size_t bsgs_smem_bytes(u32 tbits, u32 warps_per_block, u32 table_kind) {
 
 bool valid_seg_words(u32 seg_words) { return seg_words == 1024 || seg_words == 2048 || seg_words == 4096; }
 
+// The segment size of one range: halved (down to 256 words) while the range
+// has fewer segments than kFewSegs, so that a small range reaches every SM
+// (2^20 integers at 10^9: 8 blocks, 40 us; now 64 blocks, 15 us.  Switching at
+// 296 segments instead costs 2^24 integers 48 us against 40: a segment has the
+// same set-up for its 6,541 primes whatever its length).
+constexpr u64 kFewSegs = 148;
+u32 range_seg_words(u32 seg_words, u64 n_odds) {
+    while (seg_words > 256 && n_odds < kFewSegs * seg_words * 32) seg_words /= 2;
+    return seg_words;
+}
+
 cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, u64* surv, u32* surv_item, u64 surv_cap,
                          Counters* ctr, cudaStream_t s, u32 seg_words) {
     if (!valid_seg_words(seg_words)) return cudaErrorInvalidValue;
+    seg_words = range_seg_words(seg_words, a.n_odds);
     const u64 seg_odds = (u64)seg_words * 32;
     const u64 segs = (a.n_odds + seg_odds - 1) / seg_odds;
     if (segs == 0 && !a.include_two) return cudaSuccess;
     const u64 grid = segs == 0 ? 1 : min(segs, (u64)148 * 8);
-    if (seg_words == 1024) k_sieve<1024><<<(unsigned)grid, kSieveThreads, 0, s>>>(a, t, surv, surv_item, surv_cap, ctr);
-    else if (seg_words == 4096) k_sieve<4096><<<(unsigned)grid, kSieveThreads, 0, s>>>(a, t, surv, surv_item, surv_cap, ctr);
-    else k_sieve<2048><<<(unsigned)grid, kSieveThreads, 0, s>>>(a, t, surv, surv_item, surv_cap, ctr);
-    return cudaGetLastError();
+    auto go = [&](auto kern) {
+        kern<<<(unsigned)grid, kSieveThreads, 0, s>>>(a, t, surv, surv_item, surv_cap, ctr);
+        return cudaGetLastError();
+    };
+    switch (seg_words) {
+        case 256: return go(k_sieve<256>);
+        case 512: return go(k_sieve<512>);
+        case 1024: return go(k_sieve<1024>);
+        case 4096: return go(k_sieve<4096>);
+        default: return go(k_sieve<2048>);
+    }
 }
 
 cudaError_t launch_sieve_wave(const WaveDesc* w, const SieveTables& t, u64* surv, u32* surv_item, u64 surv_cap,
