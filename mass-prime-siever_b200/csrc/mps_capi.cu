@@ -88,8 +88,11 @@ struct WaveSlot {
     cudaEvent_t evk[kStageEvents] = {};   // around sieve, prep, BSGS, order
     u64* d_surv = nullptr;
     u32* d_surv_item = nullptr;
+    u64* d_surv_split = nullptr;
     u64 surv_cap = 0;
     Entry* d_ent = nullptr;
+    SplitEvent* d_events = nullptr;
+    u32* d_big = nullptr;
     u64 ent_cap = 0;
     RawRelation* d_rel = nullptr;
     RawRelation* h_rel = nullptr;     // pinned
@@ -131,8 +134,11 @@ struct mps_ctx {
     Counters* h_ctr = nullptr;      // pinned
     u64* d_surv = nullptr;
     u64 surv_cap = 0;
-    u32* d_surv_item = nullptr;
+    u64* d_surv_split = nullptr;       // the survivors' split primes (sieved chunks), surv_split_cap of them
+    u64 surv_split_cap = 0;
     Entry* d_ent = nullptr;
+    SplitEvent* d_events = nullptr;  // the split events and BSGS list of d_ent
+    u32* d_big = nullptr;
     u64 ent_cap = 0;
     RawRelation* d_rel = nullptr;
     RawRelation* h_rel = nullptr;   // pinned
@@ -190,6 +196,26 @@ int ensure(mps_ctx* c, T** ptr, u64* cap, u64 need, const char* what) {
     CK(cudaMalloc((void**)ptr, need * sizeof(T)), what);
     *cap = need;
     return MPS_OK;
+}
+
+// The entry buffer with its split events and BSGS list, for need entries.
+int alloc_entries(mps_ctx* c, Entry** ent, SplitEvent** events, u32** big, u64* cap, u64 need) {
+    if (*cap >= need && *ent && *events && *big) return MPS_OK;
+    for (void* p : {(void*)*ent, (void*)*events, (void*)*big})
+        if (p) CK(cudaFree(p), "cudaFree");
+    *ent = nullptr;
+    *events = nullptr;
+    *big = nullptr;
+    *cap = 0;
+    CK(cudaMalloc((void**)ent, need * sizeof(Entry)), "entry buffer");
+    CK(cudaMalloc((void**)events, kSplitClasses * split_event_cap(need) * sizeof(SplitEvent)), "split events");
+    CK(cudaMalloc((void**)big, need * sizeof(u32)), "BSGS list");
+    *cap = need;
+    return MPS_OK;
+}
+
+int ensure_entries(mps_ctx* c, u64 need) {
+    return alloc_entries(c, &c->d_ent, &c->d_events, &c->d_big, &c->ent_cap, need);
 }
 
 int ensure_rel(mps_ctx* c, u64 need) {
@@ -316,6 +342,10 @@ int make_dev_item(mps_ctx* c, const mps_item* it, u32 index, DevItem* d, LaunchC
     return MPS_OK;
 }
 
+// Split primes to look for in a range of an item with K in-class exponents
+// (an explicit split modulus is the whole split).
+u32 split_for(const mps_ctx* c, u64 K) { return c->tun.class_modulus == 0 ? split_primes_for(K) : 0; }
+
 u32 sieve_prime_count(u64 hi) {
     const std::vector<u32>& sp = host_tables().sp;
     u32 n = 0;
@@ -367,7 +397,8 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     const u64 chunk = c->tun.chunk_odds;
     const u64 need_surv = n_odds + 16;
     if (int r = ensure(c, &c->d_surv, &c->surv_cap, std::max<u64>(need_surv, chunk + 16), "survivor buffer")) return r;
-    if (int r = ensure(c, &c->d_ent, &c->ent_cap, std::max<u64>(chunk / 4, 1 << 16), "entry buffer")) return r;
+    if (int r = ensure(c, &c->d_surv_split, &c->surv_split_cap, c->surv_cap, "split primes")) return r;
+    if (int r = ensure_entries(c, std::max<u64>(chunk / 4, 1 << 16))) return r;
     if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
 
     u32 tbits, max_baby;
@@ -381,16 +412,22 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     sa.hi = hi;
     sa.include_two = include_two;
     sa.n_primes = sieve_prime_count(hi);
+    sa.n_split = split_for(c, K);
     sa.item = item;
 
     PrepArgs pa{};
     pa.surv = c->d_surv;
     pa.surv_cap = c->surv_cap;
     pa.surv_item = nullptr;
+    pa.surv_split = c->d_surv_split;
+    pa.tables = c->tables();
     pa.item0 = item;
     pa.items = c->d_items;
     pa.ent = c->d_ent;
     pa.ent_cap = c->ent_cap;
+    pa.events = c->d_events;
+    pa.ev_cap = split_event_cap(c->ent_cap);
+    pa.big = c->d_big;
     pa.rel = c->d_rel;
     pa.rel_cap = c->rel_cap;
     pa.full_mr = c->tun.full_mr;
@@ -400,6 +437,7 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
 
     BsgsArgs ba{};
     ba.ent = c->d_ent;
+    ba.big = c->d_big;
     ba.ent_cap = c->ent_cap;
     ba.rel = c->d_rel;
     ba.rel_cap = c->rel_cap;
@@ -421,7 +459,7 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     cudaStream_t s = c->stream;
     CK(cudaMemsetAsync(c->d_ctr, 0, sizeof(Counters), s), "counter reset");
     CK(cudaEventRecord(c->evk[0], s), "event");
-    CK(launch_sieve(sa, c->tables(), c->d_surv, nullptr, c->surv_cap, c->d_ctr, s, g.seg_words), "sieve launch");
+    CK(launch_sieve(sa, c->tables(), SurvOut{c->d_surv, nullptr, c->d_surv_split, c->surv_cap}, c->d_ctr, s, g.seg_words), "sieve launch");
     CK(cudaEventRecord(c->evk[1], s), "event");
     int bgrid = 0;
     if (int r = bsgs_grid(c, tbits, warps, g.kind, &bgrid)) return r;
@@ -431,18 +469,18 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
         CK(cudaStreamSynchronize(s), "sieve");
         const u64 ns = std::min<u64>(c->h_ctr->survivors, c->surv_cap);
         CK(cudaEventRecord(c->evk[2], s), "event");
-        CK(launch_prep(pa, c->d_ctr, (int)std::max<u64>((ns + 255) / 256, 1), s), "prep launch");
+        CK(launch_prep(pa, c->d_ctr, (int)std::max<u64>((ns + 255) / 256, 1), c->num_sms, s), "prep launch");
         CK(cudaEventRecord(c->evk[3], s), "event");
         CK(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s), "count read");
         CK(cudaStreamSynchronize(s), "prep");
-        const u64 ne = std::min<u64>(c->h_ctr->entries, c->ent_cap);
+        const u64 ne = c->h_ctr->big;
         ba.persistent = 0;
         CK(cudaEventRecord(c->evk[4], s), "event");
         if (ne) CK(launch_bsgs(ba, c->d_ctr, (int)((ne + warps - 1) / warps), s), "bsgs launch");
         CK(cudaEventRecord(c->evk[5], s), "event");
     } else {
         CK(cudaEventRecord(c->evk[2], s), "event");
-        CK(launch_prep(pa, c->d_ctr, grid_for(c, 16), s), "prep launch");
+        CK(launch_prep(pa, c->d_ctr, grid_for(c, 4), c->num_sms, s), "prep launch");
         CK(cudaEventRecord(c->evk[3], s), "event");
         ba.persistent = 1;
         CK(cudaEventRecord(c->evk[4], s), "event");
@@ -455,7 +493,7 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     CK(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s), "count read");
     CK(cudaStreamSynchronize(s), "chunk");
     if (int r = add_stage_times(c, c->evk)) return r;
-    c->stats.kernel_launches += 4;
+    c->stats.kernel_launches += 3 + kPrepLaunches;
     const Counters h = *c->h_ctr;
     if (h.status & (kStatusSurvivorOverflow | kStatusEntryOverflow)) {
         // a denser range than the buffers were sized for: halve the chunk
@@ -520,15 +558,15 @@ int slot_alloc(mps_ctx* c, WaveSlot& w) {
     if (w.surv_cap < chunk + kMaxRuns + 16) {
         if (w.d_surv) CK(cudaFree(w.d_surv), "cudaFree");
         if (w.d_surv_item) CK(cudaFree(w.d_surv_item), "cudaFree");
+        if (w.d_surv_split) CK(cudaFree(w.d_surv_split), "cudaFree");
         w.surv_cap = chunk + kMaxRuns + 16;
         CK(cudaMalloc((void**)&w.d_surv, w.surv_cap * sizeof(u64)), "survivor buffer");
         CK(cudaMalloc((void**)&w.d_surv_item, w.surv_cap * sizeof(u32)), "survivor items");
+        CK(cudaMalloc((void**)&w.d_surv_split, w.surv_cap * sizeof(u64)), "split primes");
         drop_graphs(w);
     }
     if (w.ent_cap < std::max<u64>(chunk / 4, 1 << 16)) {
-        if (w.d_ent) CK(cudaFree(w.d_ent), "cudaFree");
-        w.ent_cap = std::max<u64>(chunk / 4, 1 << 16);
-        CK(cudaMalloc((void**)&w.d_ent, w.ent_cap * sizeof(Entry)), "entry buffer");
+        if (int r = alloc_entries(c, &w.d_ent, &w.d_events, &w.d_big, &w.ent_cap, std::max<u64>(chunk / 4, 1 << 16))) return r;
         drop_graphs(w);
     }
     if (w.rel_cap < (1u << 16)) {
@@ -542,8 +580,8 @@ int slot_alloc(mps_ctx* c, WaveSlot& w) {
 void slot_free(WaveSlot& w) {
     if (w.stream) cudaStreamSynchronize(w.stream);
     drop_graphs(w);
-    for (void* p : {(void*)w.d_surv, (void*)w.d_surv_item, (void*)w.d_ent, (void*)w.d_rel, (void*)w.d_ctr,
-                    (void*)w.d_wave})
+    for (void* p : {(void*)w.d_surv, (void*)w.d_surv_item, (void*)w.d_surv_split, (void*)w.d_ent, (void*)w.d_events, (void*)w.d_big,
+                    (void*)w.d_rel, (void*)w.d_ctr, (void*)w.d_wave})
         if (p) cudaFree(p);
     for (void* p : {(void*)w.h_rel, (void*)w.h_ctr, (void*)w.h_wave})
         if (p) cudaFreeHost(p);
@@ -559,13 +597,15 @@ int slot_enqueue(mps_ctx* c, WaveSlot& w, u32 tbits, const LaunchCfg& g, bool ca
     const u32 warps = g.warps;
     PrepArgs pa{};
     pa.surv = w.d_surv; pa.surv_cap = w.surv_cap; pa.surv_item = w.d_surv_item; pa.item0 = 0;
+    pa.surv_split = w.d_surv_split; pa.tables = c->tables();
     pa.items = c->d_items; pa.ent = w.d_ent; pa.ent_cap = w.ent_cap; pa.rel = w.d_rel; pa.rel_cap = w.rel_cap;
+    pa.events = w.d_events; pa.ev_cap = split_event_cap(w.ent_cap); pa.big = w.d_big;
     pa.full_mr = c->tun.full_mr;
     pa.m_cap = launch_m_cap(c, g, tbits);
     pa.m_round = g.lanes * g.chains;
     pa.prime_below = kSievedPrimeBelow;             // survivors of the sieve
     BsgsArgs ba{};
-    ba.ent = w.d_ent; ba.ent_cap = w.ent_cap; ba.rel = w.d_rel; ba.rel_cap = w.rel_cap; ba.tbits = tbits;
+    ba.ent = w.d_ent; ba.big = w.d_big; ba.ent_cap = w.ent_cap; ba.rel = w.d_rel; ba.rel_cap = w.rel_cap; ba.tbits = tbits;
     ba.warps_per_block = warps; ba.persistent = 1; ba.chains = g.chains;
     ba.table_kind = g.kind; ba.load_shift = g.load_shift; ba.lanes = g.lanes; ba.fill = g.fill;
     ba.max_p = 0;   // per-entry arithmetic
@@ -578,12 +618,12 @@ int slot_enqueue(mps_ctx* c, WaveSlot& w, u32 tbits, const LaunchCfg& g, bool ca
     // external records: a captured graph records these events on every replay
     const unsigned ev_flags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
     CK(cudaEventRecordWithFlags(w.evk[0], s, ev_flags), "event");
-    CK(launch_sieve_wave(w.d_wave, c->tables(), w.d_surv, w.d_surv_item, w.surv_cap, w.d_ctr, grid_for(c, 8), s,
-                         g.seg_words),
+    CK(launch_sieve_wave(w.d_wave, c->tables(), SurvOut{w.d_surv, w.d_surv_item, w.d_surv_split, w.surv_cap}, w.d_ctr,
+                         grid_for(c, 8), s, g.seg_words),
        "sieve launch");
     CK(cudaEventRecordWithFlags(w.evk[1], s, ev_flags), "event");
     CK(cudaEventRecordWithFlags(w.evk[2], s, ev_flags), "event");
-    CK(launch_prep(pa, w.d_ctr, grid_for(c, 16), s), "prep launch");
+    CK(launch_prep(pa, w.d_ctr, grid_for(c, 4), c->num_sms, s), "prep launch");
     CK(cudaEventRecordWithFlags(w.evk[3], s, ev_flags), "event");
     CK(cudaEventRecordWithFlags(w.evk[4], s, ev_flags), "event");
     CK(launch_bsgs(ba, w.d_ctr, bgrid, s), "bsgs launch");
@@ -669,7 +709,7 @@ int slot_finish(mps_ctx* c, WaveSlot& w, std::vector<RawRelation>& out) {
     CK(cudaStreamSynchronize(w.stream), "wave");
     const Counters h = *w.h_ctr;
     if (int r = add_stage_times(c, w.evk)) return r;
-    c->stats.kernel_launches += 5;
+    c->stats.kernel_launches += 4 + kPrepLaunches;
     if (h.status & kStatusOrderFailed) return fail(c, MPS_E_CUDA, "order computation did not factor p - 1");
     if (h.status & kStatusBadLaunch) return fail(c, MPS_E_CUDA, "a BSGS entry did not fit the launch's tables");
     if (h.status & (kStatusSurvivorOverflow | kStatusEntryOverflow | kStatusRelationOverflow)) {
@@ -754,7 +794,7 @@ int run_waves(mps_ctx* c, const std::vector<u64>& lo, const std::vector<u64>& hi
             run.include_two = (a <= 2 && b > 2) ? 1 : 0;
             run.n_primes = sieve_prime_count(b);
             run.item = (u32)i;
-            run.pad = 0;
+            run.n_split = split_for(c, c->item_K[i]);
             run.hi = b;
             cur->ranges.push_back({a, b});
             cur->range_item.push_back((u32)i);
@@ -1069,7 +1109,7 @@ void serve_loop(mps_server* sv) {
                     run.include_two = (a <= 2 && b > 2) ? 1 : 0;
                     run.n_primes = sieve_prime_count(b);
                     run.item = (u32)q->slot;
-                    run.pad = 0;
+                    run.n_split = split_for(c, q->d.K);
                     run.hi = b;
                     w.ranges.push_back({a, b});
                     w.range_item.push_back((u32)q->slot);
@@ -1240,7 +1280,7 @@ int mps_close(mps_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (WaveSlot& w : c->slot) slot_free(w);
     for (void* p : {(void*)c->d_sp, (void*)c->d_rcp, (void*)c->d_inv, (void*)c->d_ctr, (void*)c->d_surv,
-                    (void*)c->d_surv_item, (void*)c->d_ent, (void*)c->d_rel, (void*)c->d_items, (void*)c->d_state})
+                    (void*)c->d_surv_split, (void*)c->d_ent, (void*)c->d_events, (void*)c->d_big, (void*)c->d_rel, (void*)c->d_items, (void*)c->d_state})
         if (p) cudaFree(p);
     if (c->h_ctr) cudaFreeHost(c->h_ctr);
     if (c->h_rel) cudaFreeHost(c->h_rel);
@@ -1323,7 +1363,7 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
     for (size_t off = 0; off < n; off += chunk) {
         const u64 cnt = std::min<u64>(chunk, n - off);
         if (int r = ensure(c, &c->d_surv, &c->surv_cap, std::max<u64>(cnt + 16, chunk + 16), "survivor buffer")) return r;
-        if (int r = ensure(c, &c->d_ent, &c->ent_cap, std::max<u64>(cnt, 1 << 16), "entry buffer")) return r;
+        if (int r = ensure_entries(c, std::max<u64>(cnt, 1 << 16))) return r;
         if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
         u32 tbits, mb;
         table_for(c, g, d.K, &tbits, &mb);
@@ -1338,11 +1378,13 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
         CK(cudaMemcpyAsync(&c->d_ctr->survivors, &h.survivors, sizeof(u64), cudaMemcpyHostToDevice, s), "count upload");
         PrepArgs pa{};
         pa.surv = c->d_surv; pa.surv_cap = c->surv_cap; pa.item0 = 0; pa.items = c->d_items;
+        pa.tables = c->tables();                        // no surv_split: the primes did not come from the sieve
         pa.ent = c->d_ent; pa.ent_cap = c->ent_cap; pa.rel = c->d_rel; pa.rel_cap = c->rel_cap; pa.full_mr = c->tun.full_mr;
+        pa.events = c->d_events; pa.ev_cap = split_event_cap(c->ent_cap); pa.big = c->d_big;
         pa.m_cap = launch_m_cap(c, g, tbits);
         pa.m_round = g.lanes * g.chains;
         BsgsArgs ba{};
-        ba.ent = c->d_ent; ba.ent_cap = c->ent_cap; ba.rel = c->d_rel; ba.rel_cap = c->rel_cap;
+        ba.ent = c->d_ent; ba.big = c->d_big; ba.ent_cap = c->ent_cap; ba.rel = c->d_rel; ba.rel_cap = c->rel_cap;
         ba.tbits = tbits; ba.warps_per_block = warps; ba.persistent = 1; ba.chains = g.chains; ba.table_kind = g.kind;
         ba.load_shift = g.load_shift;
         ba.fill = g.fill;
@@ -1350,7 +1392,7 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
         ba.max_p = *std::max_element(primes + off, primes + off + cnt);
         OrderArgs oa{};
         oa.rel = c->d_rel; oa.rel_cap = c->rel_cap; oa.items = c->d_items; oa.tables = c->tables();
-        CK(launch_prep(pa, c->d_ctr, grid_for(c, 16), s), "prep launch");
+        CK(launch_prep(pa, c->d_ctr, grid_for(c, 4), c->num_sms, s), "prep launch");
         CK(launch_bsgs(ba, c->d_ctr, bgrid, s), "bsgs launch");
         CK(launch_order(oa, c->d_ctr, grid_for(c, 4), s), "order launch");
         CK(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s), "count read");
@@ -1363,7 +1405,7 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
             for (u64 i = 0; i < nr; ++i)
                 if (c->h_rel[i].q != ~0ull) rel.push_back(c->h_rel[i]);
         }
-        c->stats.kernel_launches += 3;
+        c->stats.kernel_launches += 3 + kPrepLaunches;
     }
     if (int r = end_call(c)) return r;
     // flags by p (host-supplied primes may repeat or be unsorted)
@@ -1623,7 +1665,7 @@ int mps_count_primes(mps_ctx* c, uint64_t lo, uint64_t hi, uint64_t* count) {
         sa.lo_odd = lo_odd; sa.n_odds = n_odds; sa.hi = b; sa.include_two = (a <= 2 && b > 2);
         sa.n_primes = sieve_prime_count(b);
         CK(cudaMemsetAsync(c->d_ctr, 0, sizeof(Counters), c->stream), "counter reset");
-        CK(launch_sieve(sa, c->tables(), c->d_surv, nullptr, c->surv_cap, c->d_ctr, c->stream), "sieve launch");
+        CK(launch_sieve(sa, c->tables(), SurvOut{c->d_surv, nullptr, nullptr, c->surv_cap}, c->d_ctr, c->stream), "sieve launch");
         CK(launch_count_primes(c->d_surv, c->surv_cap, c->d_ctr, grid_for(c, 8), c->stream), "count launch");
         CK(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream), "count read");
         CK(cudaStreamSynchronize(c->stream), "count");
@@ -1888,7 +1930,7 @@ int mps_test_survivors(mps_ctx* c, uint64_t lo, uint64_t hi, uint64_t* out, size
     sa.lo_odd = lo_odd; sa.n_odds = n_odds; sa.hi = hi; sa.include_two = 0;
     sa.n_primes = sieve_prime_count(hi);
     CK(cudaMemsetAsync(c->d_ctr, 0, sizeof(Counters), c->stream), "counter reset");
-    CK(launch_sieve(sa, c->tables(), c->d_surv, nullptr, c->surv_cap, c->d_ctr, c->stream), "sieve launch");
+    CK(launch_sieve(sa, c->tables(), SurvOut{c->d_surv, nullptr, nullptr, c->surv_cap}, c->d_ctr, c->stream), "sieve launch");
     CK(cudaMemcpyAsync(c->h_ctr, c->d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream), "count read");
     CK(cudaStreamSynchronize(c->stream), "sieve");
     const u64 ns = c->h_ctr->survivors;

@@ -88,6 +88,7 @@ inline int item_constants(const mps_item* it, u32 class_modulus, u32 index, DevI
     if (x > 1) d->qf_l[d->qf_n++] = (u32)x;
     d->cmQ = (u32)(cm % Q);
     d->nsQ = (u32)(d->n_start % Q);
+    d->split_more = class_modulus == 0;       // an explicit Q is the whole split
     d->item_index = index;
     d->baby_scale = kDefaultBabyScale;
     // the quadratic-character prefilter needs 0 < |b|, |c| < 2^32

@@ -21,6 +21,7 @@
 #include "mps_kernels.cuh"
 
 #include <algorithm>
+#include <cstddef>
 #include <mutex>
 
 namespace mps {
@@ -77,6 +78,7 @@ __device__ __forceinline__ void emit_relation(u64 p, u64 M, u64 q, u32 item, Raw
 constexpr u32 kSegWords = 2048;
 constexpr u32 kSieveThreads = 256;
 constexpr u32 kNumPattern = 10;               // 3..31: whole-word patterns, no atomics
+constexpr u32 kSplitShared = 164;             // split primes below 1024: a warp's lanes share each
 constexpr u32 kNumMedium = 171;               // primes below 1024: a warp's lanes share each prime
 
 // Index j >= 0 of the first odd multiple v0 + 2j of q with v0 + 2j >= v0 (v0 odd).
@@ -102,24 +104,27 @@ struct SieveShared {
     u32 med_start[kNumMedium];
     u32 warp_sum[kSieveThreads / 32];
     unsigned long long block_base;
+    unsigned short before[W];                 // survivors of the segment before each word
+    unsigned short split_start[kSplitPrimes];
 };
 
-__device__ __forceinline__ void emit_two(u32 item, u64* surv, u32* surv_item, u64 cap, Counters* ctr) {
+__device__ __forceinline__ void emit_two(u32 item, const SurvOut& o, Counters* ctr) {
     const u64 slot = atomicAdd(&ctr->survivors, 1ull);
-    if (slot < cap) {
-        surv[slot] = 2;
-        if (surv_item) surv_item[slot] = item;
+    if (slot < o.cap) {
+        o.surv[slot] = 2;
+        if (o.item) o.item[slot] = item;
+        if (o.split) o.split[slot] = 0;
     } else {
         atomicOr(&ctr->status, kStatusSurvivorOverflow);
     }
 }
 
 // One segment of len <= W * 32 odd numbers v0, v0 + 2, ... (v0 odd, >= 3),
-// sieved by the first n_primes odd primes; survivors appended to surv[].
-// Called by all threads of the block.
+// sieved by the first n_primes odd primes; survivors appended to o, with the
+// first n_split split primes l | v - 1 of each.  Called by all threads of the block.
 template <u32 W>
-__device__ void sieve_segment(SieveShared<W>& sh, u64 v0, u32 len, u32 n_primes, u32 item, const SieveTables& t,
-                              u64* surv, u32* surv_item, u64 cap, Counters* ctr) {
+__device__ void sieve_segment(SieveShared<W>& sh, u64 v0, u32 len, u32 n_primes, u32 n_split, u32 item,
+                              const SieveTables& t, const SurvOut& o, Counters* ctr) {
     constexpr u32 kSegOdds = W * 32, kWordsPerThread = W / kSieveThreads;
     const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const u32 n_med = min(n_primes, kNumMedium);
@@ -222,52 +227,89 @@ __device__ void sieve_segment(SieveShared<W>& sh, u64 v0, u32 len, u32 n_primes,
         if (lane == kSieveThreads / 32 - 1) sh.block_base = atomicAdd(&ctr->survivors, (unsigned long long)wincl);
     }
     __syncthreads();
-    u64 pos = sh.block_base + sh.warp_sum[warp] + (incl - mine);
+    const u64 base = sh.block_base;
+    u32 rank = sh.warp_sum[warp] + (incl - mine);
     for (u32 k = 0; k < kWordsPerThread; ++k) {
         const u32 w = w0 + k;
         u32 x = ~sh.bits[w];
         const u32 first = w * 32;
         if (first >= len) x = 0;
         else if (len - first < 32) x &= (1u << (len - first)) - 1u;
+        sh.before[w] = (unsigned short)rank;
         while (x) {
             const u32 b = __ffs(x) - 1;
             x &= x - 1;
-            if (pos < cap) {
-                surv[pos] = v0 + 2ull * (first + b);
-                if (surv_item) surv_item[pos] = item;
+            const u64 pos = base + rank;
+            if (pos < o.cap) {
+                o.surv[pos] = v0 + 2ull * (first + b);
+                if (o.item) o.item[pos] = item;
+                if (o.split) o.split[pos] = 0;
             }
-            ++pos;
+            ++rank;
         }
     }
-    if (pos > cap) atomicOr(&ctr->status, kStatusSurvivorOverflow);
+    if (base + rank > o.cap) atomicOr(&ctr->status, kStatusSurvivorOverflow);
+    if (o.split && n_split) {
+        // 5. the split primes l | v - 1: the bitmap walked once more, from the
+        // first v == 1 (mod l), a warp's lanes sharing each l below 1024 (the
+        // first three classes), one thread each of the others.  A survivor keeps one
+        // l of each size class (a second one of a class, 4% of them, overwrites
+        // the first).  This costs 1/l visits an odd number, about a tenth of
+        // trying the primes on each entry (k_split).
+        for (u32 k = tid; k < n_split; k += kSieveThreads) {
+            const u32 q = t.sp[kSplitBase + k];
+            u32 r = (u32)(v0 - __umul64hi(v0, t.rcp[kSplitBase + k]) * q);
+            if (r >= q) r -= q;
+            const u32 d = r <= 1 ? 1 - r : q + 1 - r;              // 2 j == 1 - v0 (mod q)
+            sh.split_start[k] = (unsigned short)((d & 1u) ? (d + q) >> 1 : d >> 1);
+        }
+        __syncthreads();
+        unsigned short* out = reinterpret_cast<unsigned short*>(o.split);
+        auto visit = [&](u32 i, u32 c, u32 k) {
+            const u32 w = ~sh.bits[i >> 5] << (31 - (i & 31));     // bit i on top
+            if ((int)w < 0) {
+                const u64 pos = base + sh.before[i >> 5] + __popc(w) - 1;
+                if (pos < o.cap) out[4 * pos + c] = (unsigned short)(k + 1);
+            }
+        };
+        const u32 n_shared = min(n_split, kSplitShared);
+        for (u32 k = warp; k < n_shared; k += kSieveThreads / 32) {
+            const u32 q = t.sp[kSplitBase + k], c = split_class(k);
+            for (u32 i = sh.split_start[k] + lane * q; i < len; i += 32 * q) visit(i, c, k);
+        }
+        for (u32 k = kSplitShared + tid; k < n_split; k += kSieveThreads) {
+            const u32 q = t.sp[kSplitBase + k];
+            for (u32 i = sh.split_start[k]; i < len; i += q) visit(i, kSplitClasses - 1, k);
+        }
+    }
     __syncthreads();
 }
+static_assert(kSplitClasses == 4 && split_class(kSplitShared - 1) == 2 && split_class(kSplitShared) == 3, "a survivor's split primes fill one 64-bit word");
 
 template <u32 W>
-__global__ void __launch_bounds__(kSieveThreads) k_sieve(SieveArgs a, SieveTables t, u64* surv, u32* surv_item,
-                                                         u64 cap, Counters* ctr) {
+__global__ void __launch_bounds__(kSieveThreads) k_sieve(SieveArgs a, SieveTables t, SurvOut o, Counters* ctr) {
     constexpr u32 kSegOdds = W * 32;
     __shared__ SieveShared<W> sh;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && a.include_two) emit_two(a.item, surv, surv_item, cap, ctr);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && a.include_two) emit_two(a.item, o, ctr);
     for (u64 seg = blockIdx.x; seg * kSegOdds < a.n_odds; seg += gridDim.x) {
         const u64 base = seg * kSegOdds;
-        sieve_segment(sh, a.lo_odd + 2 * base, (u32)min((u64)kSegOdds, a.n_odds - base), a.n_primes, a.item, t, surv,
-                      surv_item, cap, ctr);
+        sieve_segment(sh, a.lo_odd + 2 * base, (u32)min((u64)kSegOdds, a.n_odds - base), a.n_primes, a.n_split, a.item, t, o,
+                      ctr);
     }
 }
 
 // The same over a wave of runs (ranges of possibly different items), read
 // from device memory so that a captured graph can be replayed per wave.
 template <u32 W>
-__global__ void __launch_bounds__(kSieveThreads) k_sieve_wave(const WaveDesc* w, SieveTables t, u64* surv,
-                                                              u32* surv_item, u64 cap, Counters* ctr) {
+__global__ void __launch_bounds__(kSieveThreads) k_sieve_wave(const WaveDesc* w, SieveTables t, SurvOut o,
+                                                              Counters* ctr) {
     constexpr u32 kSegOdds = W * 32;
     __shared__ SieveShared<W> sh;
     const u32 n_runs = w->n_runs;
     const u64 total = w->total_segs;
     if (blockIdx.x == 0 && threadIdx.x == 0)
         for (u32 r = 0; r < n_runs; ++r)
-            if (w->runs[r].include_two) emit_two(w->runs[r].item, surv, surv_item, cap, ctr);
+            if (w->runs[r].include_two) emit_two(w->runs[r].item, o, ctr);
     for (u64 seg = blockIdx.x; seg < total; seg += gridDim.x) {
         u32 lo = 0, hi = n_runs;                        // last run with seg_begin <= seg
         while (hi - lo > 1) {
@@ -278,8 +320,8 @@ __global__ void __launch_bounds__(kSieveThreads) k_sieve_wave(const WaveDesc* w,
         const SieveRun& run = w->runs[lo];
         const u64 base = (seg - run.seg_begin) * kSegOdds;
         if (base >= run.n_odds) continue;               // (a run with no odd numbers)
-        sieve_segment(sh, run.lo_odd + 2 * base, (u32)min((u64)kSegOdds, run.n_odds - base), run.n_primes, run.item, t,
-                      surv, surv_item, cap, ctr);
+        sieve_segment(sh, run.lo_odd + 2 * base, (u32)min((u64)kSegOdds, run.n_odds - base), run.n_primes, run.n_split,
+                      run.item, t, o, ctr);
     }
 }
 
@@ -298,6 +340,11 @@ struct FieldF {
     __device__ __forceinline__ V mul(V a, V b) const { return f.mul(a, b); }
     __device__ __forceinline__ V canon(V a) const { return f.canon(a); }          // units: (-p, p) -> [0, p)
     __device__ __forceinline__ u64 key(V c) const { return f.bits(c); }
+    // the low word of a unit's canonical integer (|a| < p, a != 0): 2^52 is added to a or to a + p in one step
+    __device__ __forceinline__ u32 key32(V a) const {
+        const double c = 4503599627370496.0;
+        return (u32)__double2loint(__dadd_rn(a, a < 0.0 ? __dadd_rn(c, f.p) : c));
+    }
     __device__ __forceinline__ u64 residue(V a) const { return f.residue(a); }   // any lazy value
     __device__ __forceinline__ V from_u64(u64 x) const { return (double)x; }
     __device__ __forceinline__ V one() const { return 1.0; }
@@ -317,6 +364,7 @@ struct FieldM {
     __device__ __forceinline__ V mul(V a, V b) const { return M.mul(a, b); }
     __device__ __forceinline__ V canon(V a) const { return M.norm(a); }
     __device__ __forceinline__ u64 key(V c) const { return c; }
+    __device__ __forceinline__ u32 key32(V a) const { return (u32)M.norm(a); }
     __device__ __forceinline__ u64 residue(V a) const { return M.from_mont(a); }
     __device__ __forceinline__ V from_u64(u64 x) const { return M.to_mont(x, rr); }
     __device__ __forceinline__ V one() const { return M.one; }
@@ -500,58 +548,126 @@ __device__ bool power_split_pp(const F& f, u64 p, u64 w_res, u64 u_res, const De
     return true;
 }
 
-// Stage 3: n = n_start + cm*k (in class) with n == r (mod d); the BSGS set-up
-// for G0 * B^j == t, G0 = b^n_first, B = b^L, j < jcount.
-template <class F>
-__device__ void bsgs_setup(const F& f, u64 p, u64 b_mod, u64 t, const DevItem& it, u32 d, u32 r, const PrepArgs& a,
-                           Counters* ctr) {
-    typedef typename F::V V;
+// Stage 3: n = n_start + cm*k (in class) with n == r (mod d): the candidates
+// n_first + j*L, j < jcount.  False when there is none.
+__device__ __forceinline__ bool combine_class(u64 p, const DevItem& it, u32 d, u32 r, Entry& e) {
     // the smallest k0 >= 0 with n_start + cm*k0 == r (mod d): k0*cmd == want
     // (mod d) is solvable iff h = gcd(cmd, d) divides want, and then its
     // solutions are k0 + per*i with per = d/h, k0 = (want/h)(cmd/h)^-1 mod per
     const u32 cmd = it.cmQ % d;                        // d | Q
     const u32 want = (r + d - it.nsQ % d) % d;
     const u32 h = gcd32(cmd, d);                       // gcd(0, d) = d
-    if (want % h) return;
+    if (want % h) return false;
     const u32 per = d / h;                             // period of k
     const u32 k0 = (u32)((u64)(want / h) * inv_mod32((cmd / h) % per, per) % per);
-    if (k0 >= it.K) return;
+    if (k0 >= it.K) return false;
     u64 jcount = ((u32)it.K - k0 + per - 1) / per;     // K < 2^32 (N1 - N0 <= 10^7)
     if (jcount > p) jcount = p;                        // ord(B) < p (Math.hpp:398-400)
-    const u64 L = it.cm * per;
-    const u64 n_first = it.n_start + it.cm * k0;
-    // G0 = b^n_first and B = b^L from one chain of squarings of b
-    V sq = f.from_u64(b_mod), gv = f.one(), Bv = f.one();
-    for (u64 e1 = n_first, e2 = L; e1 | e2;) {
-        if (e1 & 1) gv = f.mul(gv, sq);
-        if (e2 & 1) Bv = f.mul(Bv, sq);
-        e1 >>= 1;
-        e2 >>= 1;
-        if (e1 | e2) sq = f.mul(sq, sq);
+    e.jcount = (u32)jcount;
+    e.L = it.cm * per;
+    e.n_first = it.n_start + it.cm * k0;
+    return true;
+}
+
+// ---- the split by larger primes ----
+//
+// A prime l | p - 1 outside Q splits an entry's candidates the same way: with
+// w = b^((p-1)/l) and u = t^((p-1)/l), b^n == t forces w^n == u, so n is known
+// mod l (or, when b is an l-th power residue, t has to be one too).  One
+// discrete logarithm in a group of l elements divides the candidates by l and
+// the baby and giant steps by sqrt(l); a prime has an l of 23 .. 4261 with
+// chance 1/(l-1), about one each.  Finding them costs a second walk of the
+// sieve's bitmap (sieve_segment); a logarithm costs about 720 + 1.6 l lane
+// instructions (k_dlog), so only entries with enough candidates have it.
+// Measured on 2^27 integers of b = 10, c = 111 at 10^12 (1.25 M entries):
+// k_bsgs 3.44 -> 1.62 ms for 0.06 ms of sieve, 0.21 of k_dlog and 0.20 of
+// k_setup (which took the set-up over from k_prep and solves the smallest
+// entries); BSGS steps 2.10e9 -> 0.90e9.
+
+// How many primes of the table an entry with J candidates is split by.
+__host__ __device__ constexpr u32 split_limit(u32 J) {
+    return J < 512 ? 0u : J < 1024 ? 64u : J < 4096 ? 164u : kSplitPrimes;
+}
+u32 split_primes_for(u64 K) { return split_limit((u32)min(K, (u64)~0u)); }
+
+// Queues the split events of the warp's entries (idx, lanes with ok): k[c] is
+// the index + 1 of the entry's l of class c, 0 for none.  One atomic per class
+// and warp; a full list drops the event.
+__device__ __forceinline__ void queue_events(bool ok, u64 idx, const u32 (&k)[kSplitClasses], const PrepArgs& a,
+                                             Counters* ctr) {
+    const u32 lane = threadIdx.x & 31, below = (1u << lane) - 1;
+    u32 bal[kSplitClasses], mine = 0;                  // mine: lane c < kSplitClasses, events of class c
+#pragma unroll
+    for (u32 c = 0; c < kSplitClasses; ++c) {
+        bal[c] = __ballot_sync(FULL, ok && k[c] != 0);
+        if (lane == c) mine = __popc(bal[c]);
     }
-    const u64 G0 = f.residue(gv);
-    if (G0 == t) {                                     // j = 0
-        emit_relation(p, n_first, 0, it.item_index, a.rel, a.rel_cap, ctr);
-        return;
+    u64 at0 = 0;
+    if (mine) at0 = atomicAdd(&ctr->events[lane], (unsigned long long)mine);
+#pragma unroll
+    for (u32 c = 0; c < kSplitClasses; ++c) {
+        const u64 at = __shfl_sync(FULL, at0, c) + __popc(bal[c] & below);
+        if (!ok) continue;
+        const bool in = k[c] != 0 && at < a.ev_cap;
+        if (in) a.events[c * a.ev_cap + at] = SplitEvent{(u32)idx, k[c] - 1};
+        a.ent[idx].ev[c] = in ? k[c] << 16 | kEvUnknown : 0u;
     }
-    if (jcount <= 1) return;
-    u32 m = (u32)isqrt_ceil_dev(jcount);
-    if (it.baby_scale != 256) m = max(1u, (u32)(((u64)m * it.baby_scale + 255) >> 8));
-    // a whole number of baby iterations (lanes x chains per prime): the last
-    // iteration's lanes then all insert, and the extra baby steps save giant steps
-    if (a.m_round > 1) m = (m + a.m_round - 1) / a.m_round * a.m_round;
-    if (m > it.max_baby) m = it.max_baby;
-    if (m > a.m_cap) m = a.m_cap;                      // never more than the launch's tables hold
-    const u64 Bm = f.residue(f.pow(Bv, m));
-    const u64 slot = atomicAdd(&ctr->entries, 1ull);
-    if (slot >= a.ent_cap) {
-        atomicOr(&ctr->status, kStatusEntryOverflow);
-        return;
+}
+
+// Two powers with one exponent, interleaved: a^x and b^x.
+template <class F>
+__device__ __forceinline__ void pow_pair(const F& f, typename F::V a, typename F::V b, u64 x, typename F::V& ra,
+                                         typename F::V& rb) {
+    ra = f.one();
+    rb = f.one();
+    for (; x; x >>= 1) {
+        if (x & 1) {
+            ra = f.mul(ra, a);
+            rb = f.mul(rb, b);
+        }
+        a = f.mul(a, a);
+        b = f.mul(b, b);
     }
-    Entry e;
-    e.p = p; e.t = t; e.G0 = G0; e.B = f.residue(Bv); e.Bm = Bm;
-    e.n_first = n_first; e.L = L; e.jcount = jcount; e.m = m; e.item = it.item_index;
-    a.ent[slot] = e;
+}
+
+// The smallest j in [1, J) with G0 * B^j == t, by one lane (~0: none): kLaneBaby
+// baby steps t * B^i whose low words stay in registers, giant steps G0 *
+// B^(kLaneBaby g) compared with all of them (a compare is one instruction, a
+// product six on the FP64 pipe), a low word that matches resolved exactly.  t canonical.
+constexpr u32 kLaneBaby = 16;
+template <class F>
+__device__ u32 lane_solve(const F& f, typename F::V t, typename F::V G0, typename F::V B, u32 J) {
+    typedef typename F::V V;
+    u32 key[kLaneBaby];
+    V x = t;
+#pragma unroll
+    for (u32 i = 0; i < kLaneBaby; ++i) {
+        key[i] = f.key32(x);
+        x = f.mul(x, B);
+    }
+    V S = f.mul(B, B);
+#pragma unroll
+    for (u32 i = 2; i < kLaneBaby; i <<= 1) S = f.mul(S, S);
+    V g = f.mul(G0, S);
+    for (u32 base = 0; base + 1 < J; base += kLaneBaby) {   // g = G0 B^(base + kLaneBaby): j in (base, base + kLaneBaby]
+        const u32 k = f.key32(g);
+        const V next = f.mul(g, S);
+        bool hit = false;
+#pragma unroll
+        for (u32 i = 0; i < kLaneBaby; ++i) hit |= key[i] == k;
+        if (hit) {
+            const V c = f.canon(g);
+            u32 best = ~0u;
+            x = t;
+            for (u32 i = 0; i < kLaneBaby; ++i) {           // the last i is the smallest j
+                if (f.canon(x) == c) best = base + kLaneBaby - i;
+                x = f.mul(x, B);
+            }
+            if (best != ~0u) return best < J ? best : ~0u;
+        }
+        g = next;
+    }
+    return ~0u;
 }
 
 template <class F>
@@ -591,12 +707,12 @@ constexpr u32 kPrepWarps = kPrepThreads / 32;
 
 struct PrepQueues {
     u64 p1[64];
-    u32 i1[64];
+    u32 i1[64], s1[64];                            // item, survivor index (surv_split's)
     u64 p2[64];
-    u32 i2[64], d2[64], r2[64];
+    u32 i2[64], s2[64], d2[64], r2[64];
     u64 pd[64];
     u64 wd[64], ud[64];                            // stage 2's w and u of a deferred prime
-    u32 id[64];
+    u32 id[64], sd[64];
 };
 
 // Appends the lanes with want to a warp queue of n entries (n warp-uniform).
@@ -623,15 +739,6 @@ __device__ __forceinline__ bool split_pp_in(const DevItem& it, u64 p, u64 w, u64
     return power_split_pp(f, p, w, u, it, d, r);
 }
 
-template <class F>
-__device__ __forceinline__ void setup_in(const DevItem& it, u64 p, u32 d, u32 r, const PrepArgs& a, Counters* ctr) {
-    F f;
-    f.init(p);
-    const u64 bm = residue128(it.babs_hi, it.babs_lo, it.b_neg, p);
-    const u64 t = p - residue128(it.cabs_hi, it.cabs_lo, it.c_neg, p);
-    bsgs_setup(f, p, bm, t, it, d, r, a, ctr);
-}
-
 __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr) {
     __shared__ PrepQueues qs[kPrepWarps];
     PrepQueues& Q = qs[threadIdx.x >> 5];
@@ -641,29 +748,58 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr
     bool inputs = true;
     for (;;) {
         if (n2 >= 32 || (!inputs && n1 == 0 && nd == 0 && n2 > 0)) {
-            // stage 3: class combination and the BSGS set-up
+            // stage 3: class combination, and the entries' way out
             const u32 cnt = min(n2, 32u);
+            Entry e;
+            bool ok = false;
+            u32 sv = 0;
             if (lane < cnt) {
                 const u32 k = n2 - cnt + lane;
-                const u64 p = Q.p2[k];
-                const DevItem& it = a.items[Q.i2[k]];
-                if (p < kFp64Limit) setup_in<FieldF>(it, p, Q.d2[k], Q.r2[k], a, ctr);
-                else setup_in<FieldM>(it, p, Q.d2[k], Q.r2[k], a, ctr);
+                e.p = Q.p2[k];
+                e.item = Q.i2[k];
+                sv = Q.s2[k];
+                ok = combine_class(e.p, a.items[e.item], Q.d2[k], Q.r2[k], e);
             }
             n2 -= cnt;
             __syncwarp();
+            const u32 bal = __ballot_sync(FULL, ok);
+            if (bal) {
+                u64 base = 0;
+                if (lane == 0) base = atomicAdd(&ctr->entries, (unsigned long long)__popc(bal));
+                const u64 slot = __shfl_sync(FULL, base, 0) + __popc(bal & ((1u << lane) - 1));
+                if (ok && slot >= a.ent_cap) {
+                    atomicOr(&ctr->status, kStatusEntryOverflow);
+                    ok = false;
+                }
+                if (ok) {
+                    Entry& d = a.ent[slot];
+                    d.p = e.p; d.n_first = e.n_first; d.L = e.L; d.jcount = e.jcount; d.item = e.item;
+                }
+                if (a.surv_split) {
+                    const u64 found = ok ? a.surv_split[sv] : 0;
+                    const u32 limit = ok && a.items[e.item].split_more ? split_limit(e.jcount) : 0u;
+                    u32 k[kSplitClasses];
+#pragma unroll
+                    for (u32 c = 0; c < kSplitClasses; ++c) {
+                        k[c] = (u32)(found >> (16 * c)) & 0xFFFFu;
+                        if (k[c] > limit) k[c] = 0;
+                    }
+                    queue_events(ok, slot, k, a, ctr);
+                }
+            }
             continue;
         }
         if (nd >= 32 || (!inputs && n1 == 0 && nd > 0)) {
             // stage 2b: long orders, one prime power at a time
             const u32 cnt = min(nd, 32u);
             bool ok = false;
-            u32 d = 1, r = 0, item = 0;
+            u32 d = 1, r = 0, item = 0, sv = 0;
             u64 p = 0;
             if (lane < cnt) {
                 const u32 k = nd - cnt + lane;
                 p = Q.pd[k];
                 item = Q.id[k];
+                sv = Q.sd[k];
                 const DevItem& it = a.items[item];
                 const u64 w = Q.wd[k], u = Q.ud[k];
                 ok = p < kFp64Limit ? split_pp_in<FieldF>(it, p, w, u, d, r) : split_pp_in<FieldM>(it, p, w, u, d, r);
@@ -675,6 +811,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr
             if (ok) {
                 Q.p2[s2] = p;
                 Q.i2[s2] = item;
+                Q.s2[s2] = sv;
                 Q.d2[s2] = d;
                 Q.r2[s2] = r;
             }
@@ -685,12 +822,13 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr
             // stage 2: power-residue split with a short walk
             const u32 cnt = min(n1, 32u);
             int res = 0;
-            u32 d = 1, r = 0, item = 0;
+            u32 d = 1, r = 0, item = 0, sv = 0;
             u64 p = 0, w = 0, u = 0;
             if (lane < cnt) {
                 const u32 k = n1 - cnt + lane;
                 p = Q.p1[k];
                 item = Q.i1[k];
+                sv = Q.s1[k];
                 const DevItem& it = a.items[item];
                 res = p < kFp64Limit ? split_in<FieldF>(it, p, d, r, w, u) : split_in<FieldM>(it, p, d, r, w, u);
             }
@@ -702,6 +840,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr
             if (res == 1) {
                 Q.p2[s2] = p;
                 Q.i2[s2] = item;
+                Q.s2[s2] = sv;
                 Q.d2[s2] = d;
                 Q.r2[s2] = r;
             } else if (res == 2) {
@@ -709,6 +848,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr
                 Q.wd[sd] = w;
                 Q.ud[sd] = u;
                 Q.id[sd] = item;
+                Q.sd[sd] = sv;
             }
             __syncwarp();
             continue;
@@ -739,9 +879,288 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr
         if (keep) {
             Q.p1[s1] = p;
             Q.i1[s1] = item;
+            Q.s1[s1] = (u32)k;
         }
         __syncwarp();
     }
+}
+
+// ---- k_split: the primes l | p - 1 of entries whose primes did not come from the sieve ----
+
+// A warp takes up to 32 entries; the lanes hold the table's primes (kSplitGroups
+// each, in registers for the whole launch) and try them against one entry after
+// another: four integer instructions a prime and no loads.
+__global__ void __launch_bounds__(256, 2) k_split(PrepArgs a, Counters* ctr) {
+    const u32 lane = threadIdx.x & 31;
+    const u64 n_ent = min((u64)*(volatile unsigned long long*)&ctr->entries, a.ent_cap);
+    const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
+    u32 inv_lo[kSplitGroups], inv_hi[kSplitGroups], lim[kSplitGroups];
+#pragma unroll
+    for (u32 g = 0; g < kSplitGroups; ++g) {
+        const u64 inv = a.tables.inv[kSplitBase + 32 * g + lane];
+        inv_lo[g] = (u32)inv;
+        inv_hi[g] = (u32)(inv >> 32);
+        lim[g] = (u32)(a.tables.rcp[kSplitBase + 32 * g + lane] >> 32);
+    }
+    // few entries: fewer than 32 a warp, so that every warp has some
+    const u32 per = (u32)min((u64)32, max((u64)1, n_ent / warps));
+    for (u64 first = ((u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * per; first < n_ent; first += warps * per) {
+        const u64 idx = first + lane;
+        const bool ok = lane < per && idx < n_ent;
+        u32 lo = 0, hi = 0, limit = 0;
+        if (ok) {
+            const Entry& e = a.ent[idx];
+            const u64 pm1 = e.p - 1;
+            lo = (u32)pm1;
+            hi = (u32)(pm1 >> 32);
+            limit = a.items[e.item].split_more ? split_limit(e.jcount) : 0u;
+        }
+        u32 found[kSplitClasses] = {};
+        for (u32 i = 0; i < per; ++i) {
+            const u32 n = __shfl_sync(FULL, limit, i);
+            const u32 xl = __shfl_sync(FULL, lo, i), xh = __shfl_sync(FULL, hi, i);
+            u32 div = 0;
+#pragma unroll
+            for (u32 g = 0; g < kSplitGroups; ++g) {
+                if (32 * g >= n) break;
+                // l | x iff x l^-1 mod 2^64 <= floor((2^64 - 1) / l); the high words
+                // alone let through 2^-32 of the others (k_dlog compares in full)
+                if (__umulhi(xl, inv_lo[g]) + xl * inv_hi[g] + xh * inv_lo[g] <= lim[g]) div |= 1u << g;
+            }
+            u32 bal = __ballot_sync(FULL, div != 0);
+            while (bal) {                                      // one prime of each lane
+                const u32 src = (u32)__ffs((int)bal) - 1;
+                bal &= bal - 1;
+                const u32 k = 32 * ((u32)__ffs((int)__shfl_sync(FULL, div, src)) - 1) + src;
+#pragma unroll
+                for (u32 c = 0; c < kSplitClasses; ++c)
+                    if (lane == i && split_class(k) == c) found[c] = k + 1;
+            }
+        }
+        queue_events(ok, idx, found, a, ctr);
+    }
+}
+
+// ---- k_dlog: the split events ----
+
+// n mod l for the entry's p: dlog of u = t^((p-1)/l) to w = b^((p-1)/l), or kEvUnknown / kEvReject.
+template <class F>
+__device__ __forceinline__ u32 split_solve(u64 p, const DevItem& it, u32 l, u64 l_inv) {
+    typedef typename F::V V;
+    F f;
+    f.init(p);
+    const u64 e = (p - 1) * l_inv;                     // (p - 1) / l
+    if (__umul64hi(e, l) != 0) return kEvUnknown;      // l does not divide p - 1 after all
+    const u64 bm = residue128(it.babs_hi, it.babs_lo, it.b_neg, p);
+    const u64 t = p - residue128(it.cabs_hi, it.cabs_lo, it.c_neg, p);
+    V w, u;
+    pow_pair(f, f.from_u64(bm), f.from_u64(t), e, w, u);
+    const V one = f.one();
+    const bool u1 = f.eq(u, one);
+    if (f.eq(w, one)) return u1 ? kEvUnknown : kEvReject;
+    if (u1) return 0;
+    const u32 x = lane_solve(f, f.canon(u), one, w, l);
+    return x == ~0u ? kEvUnknown : x;                  // (~0: p is not prime; the order stage drops it)
+}
+
+__device__ __noinline__ u32 split_solve_m(u64 p, const DevItem& it, u32 l, u64 l_inv) {
+    return split_solve<FieldM>(p, it, l, l_inv);              // out of line: the FP64 path sets the registers
+}
+
+// One lane per event, the classes of larger l first (longest walks first).
+__global__ void __launch_bounds__(256, 3) k_dlog(PrepArgs a, Counters* ctr) {
+    const u32 lane = threadIdx.x & 31;
+    const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
+    u64 units[kSplitClasses], total = 0;
+#pragma unroll
+    for (u32 c = 0; c < kSplitClasses; ++c) {
+        units[c] = (min((u64)*(volatile unsigned long long*)&ctr->events[c], a.ev_cap) + 31) / 32;
+        total += units[c];
+    }
+    for (u64 u = (u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < total; u += warps) {
+        u64 k = u;
+        u32 c = kSplitClasses - 1;
+#pragma unroll
+        for (u32 i = kSplitClasses - 1; i > 0; --i)
+            if (c == i && k >= units[i]) {
+                k -= units[i];
+                --c;
+            }
+        const u64 idx = k * 32 + lane;
+        if (idx >= min((u64)ctr->events[c], a.ev_cap)) continue;
+        const SplitEvent s = a.events[(u64)c * a.ev_cap + idx];
+        Entry& e = a.ent[s.entry];
+        const u64 p = e.p;
+        const DevItem& it = a.items[e.item];
+        const u32 l = a.tables.sp[kSplitBase + s.k];
+        const u64 l_inv = a.tables.inv[kSplitBase + s.k];
+        const u32 x = p < kFp64Limit ? split_solve<FieldF>(p, it, l, l_inv) : split_solve_m(p, it, l, l_inv);
+        e.ev[c] = (s.k + 1) << 16 | x;
+    }
+}
+
+// ---- k_setup: the solve's set-up, and the solve of primes with few candidates ----
+
+// Applies what k_dlog found to the entry's candidates; false when none is left.
+__device__ __forceinline__ bool apply_events(Entry& e, const SieveTables& t) {
+#pragma unroll
+    for (u32 i = 0; i < kSplitClasses; ++i) {
+        const u32 x = e.ev[i] & 0xFFFFu;
+        if (e.ev[i] == 0 || x == kEvUnknown) continue;
+        if (x == kEvReject) return false;
+        // the j in [0, l) with n_first + j L == x (mod l); L is prime to l unless the class modulus holds l
+        const u32 l = t.sp[kSplitBase + (e.ev[i] >> 16) - 1];
+        const u32 Lm = (u32)(e.L % l), nm = (u32)(e.n_first % l);
+        if (Lm == 0) continue;
+        const u32 j0 = (x >= nm ? x - nm : x + l - nm) * inv_mod32(Lm, l) % l;
+        if (j0 >= e.jcount) return false;
+        e.n_first += (u64)j0 * e.L;
+        e.jcount = (e.jcount - j0 + l - 1) / l;
+        if (e.jcount > 1) e.L *= l;                    // L < N1 - N0 while two candidates are left
+    }
+    return true;
+}
+
+// The set-up of one entry: false when it needs no solve (its only candidate
+// decided, or n_first already a solution).
+template <class F>
+__device__ __forceinline__ bool setup_entry(Entry& e, const DevItem& it, const PrepArgs& a, Counters* ctr, bool small) {
+    typedef typename F::V V;
+    F f;
+    f.init(e.p);
+    const u64 bm = residue128(it.babs_hi, it.babs_lo, it.b_neg, e.p);
+    e.t = e.p - residue128(it.cabs_hi, it.cabs_lo, it.c_neg, e.p);
+    // G0 = b^n_first and B = b^L from one chain of squarings of b
+    V sq = f.from_u64(bm), gv = f.one(), Bv = f.one();
+    for (u64 e1 = e.n_first, e2 = e.jcount > 1 ? e.L : 0; e1 | e2;) {
+        if (e1 & 1) gv = f.mul(gv, sq);
+        if (e2 & 1) Bv = f.mul(Bv, sq);
+        e1 >>= 1;
+        e2 >>= 1;
+        if (e1 | e2) sq = f.mul(sq, sq);
+    }
+    e.G0 = f.residue(gv);
+    if (e.G0 == e.t) {                                 // j = 0
+        emit_relation(e.p, e.n_first, 0, e.item, a.rel, a.rel_cap, ctr);
+        return false;
+    }
+    if (e.jcount <= 1) return false;
+    e.B = f.residue(Bv);
+    if (small) return true;
+    u32 m = (u32)isqrt_ceil_dev(e.jcount);
+    if (it.baby_scale != 256) m = max(1u, (u32)(((u64)m * it.baby_scale + 255) >> 8));
+    // a whole number of baby iterations (lanes x chains per prime): the last
+    // iteration's lanes then all insert, and the extra baby steps save giant steps
+    if (a.m_round > 1) m = (m + a.m_round - 1) / a.m_round * a.m_round;
+    if (m > it.max_baby) m = it.max_baby;
+    if (m > a.m_cap) m = a.m_cap;                      // never more than the launch's tables hold
+    e.m = m;
+    e.Bm = f.residue(f.pow(Bv, m));
+    return true;
+}
+
+template <class F>
+__device__ __forceinline__ u32 lane_solve_entry(const Entry& e) {
+    F f;
+    f.init(e.p);
+    return lane_solve(f, f.from_u64(e.t), f.from_u64(e.G0), f.from_u64(e.B), e.jcount);
+}
+
+__device__ __noinline__ u32 lane_solve_entry_m(const Entry& e) { return lane_solve_entry<FieldM>(e); }
+
+// Entries with at most kLaneMax candidates are solved here, one lane each:
+// 1.6 lane instructions a candidate against about 490 warp instructions of
+// per-prime set-up in k_bsgs.  A warp's lanes walk together, so the entries
+// wait in queues by size (a factor of two each) until one holds 32.
+constexpr u32 kLaneQueues = 6, kLaneMax = 2048, kLaneMin = 64;   // J <= 64, 128, .. 2048
+constexpr u32 kLaneFew = 1u << 16, kLaneMaxFew = 256;            // (2^19 integers at 10^9: 248 us with 2048, 231 with 256)
+
+__global__ void __launch_bounds__(256, 3) k_setup(PrepArgs a, Counters* ctr) {
+    __shared__ u32 queues[8][kLaneQueues][64];
+    u32(&Q)[kLaneQueues][64] = queues[threadIdx.x >> 5];
+    const u32 lane = threadIdx.x & 31, below = (1u << lane) - 1;
+    const u64 n_ent = min((u64)*(volatile unsigned long long*)&ctr->entries, a.ent_cap);
+    // few entries: a lane's walk is then what the launch waits for
+    const u32 lane_max = n_ent < kLaneFew ? kLaneMaxFew : kLaneMax;
+    u32 n[kLaneQueues] = {};                           // queue lengths (warp-uniform)
+    bool inputs = true;
+    u64 steps = 0;
+    for (;;) {
+        // a queue that holds 32 is drained; once the inputs are used up, the
+        // last 32 entries of all the queues together, the longest first
+        u32 q = kLaneQueues, idx = ~0u;
+#pragma unroll
+        for (u32 k = 0; k < kLaneQueues; ++k)
+            if (n[k] >= 32) q = k;
+        if (q < kLaneQueues) {
+#pragma unroll
+            for (u32 k = 0; k < kLaneQueues; ++k)
+                if (k == q) idx = Q[k][n[k] -= 32, n[k] + lane];
+        } else if (!inputs) {
+            u32 taken = 0;
+#pragma unroll
+            for (u32 k = kLaneQueues; k-- > 0;) {
+                const u32 cnt = min(n[k], 32 - taken);
+                if (lane >= taken && lane - taken < cnt) idx = Q[k][n[k] - cnt + lane - taken];
+                n[k] -= cnt;
+                taken += cnt;
+            }
+            if (taken == 0) break;
+        }
+        if (q < kLaneQueues || !inputs) {
+            if (idx != ~0u) {
+                const Entry& e = a.ent[idx];
+                const u32 j = e.p < kFp64Limit ? lane_solve_entry<FieldF>(e) : lane_solve_entry_m(e);
+                if (j != ~0u) emit_relation(e.p, e.n_first + (u64)j * e.L, 0, e.item, a.rel, a.rel_cap, ctr);
+                steps += kLaneBaby + (min(j, e.jcount) + kLaneBaby - 1) / kLaneBaby;
+            }
+            __syncwarp();
+            continue;
+        }
+        u64 first = 0;
+        if (lane == 0) first = atomicAdd(&ctr->setup_next, 32ull);
+        first = __shfl_sync(FULL, first, 0);
+        if (first >= n_ent) {
+            inputs = false;
+            continue;
+        }
+        idx = (u32)first + lane;
+        u32 cls = kLaneQueues + 1;                     // kLaneQueues: for k_bsgs
+        if (first + lane < n_ent) {
+            Entry e = a.ent[idx];
+            const DevItem& it = a.items[e.item];
+            if (apply_events(e, a.tables)) {
+                const bool small = e.jcount <= lane_max;
+                if (e.p < kFp64Limit ? setup_entry<FieldF>(e, it, a, ctr, small)
+                                     : setup_entry<FieldM>(e, it, a, ctr, small)) {
+                    Entry& d = a.ent[idx];
+                    d.t = e.t; d.G0 = e.G0; d.B = e.B; d.Bm = e.Bm; d.jcount = e.jcount; d.m = e.m;
+                    d.n_first = e.n_first; d.L = e.L;
+                    cls = kLaneQueues;
+                    if (small) {
+                        cls = 0;
+                        while (e.jcount > (kLaneMin << cls)) ++cls;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (u32 k = 0; k < kLaneQueues; ++k) {
+            const u32 bal = __ballot_sync(FULL, cls == k);
+            if (cls == k) Q[k][n[k] + __popc(bal & below)] = idx;
+            n[k] += __popc(bal);
+        }
+        const u32 bal = __ballot_sync(FULL, cls == kLaneQueues);
+        if (bal) {
+            u64 base = 0;
+            if (lane == 0) base = atomicAdd(&ctr->big, (unsigned long long)__popc(bal));
+            base = __shfl_sync(FULL, base, 0);
+            if (cls == kLaneQueues) a.big[base + __popc(bal & below)] = idx;
+        }
+        __syncwarp();
+    }
+    steps = __reduce_add_sync(FULL, (u32)steps);
+    if (lane == 0 && steps) atomicAdd(&ctr->steps, (unsigned long long)steps);
 }
 
 // --------------------------------------------------------------- the BSGS --
@@ -800,7 +1219,7 @@ __device__ __forceinline__ u64 pack_steps(u64 baby, u64 giant) { return (giant <
 // indices i = l + 64k and l + 32 + 64k, giant steps g = 1 + l + 64k and
 // 33 + l + 64k.
 template <class F>
-__device__ u64 solve_entry(const Entry& e, unsigned short* tab, u32 tbits, u64* steps_out) {
+__device__ u64 solve_entry(const Solve& e, unsigned short* tab, u32 tbits, u64* steps_out) {
     typedef typename F::V V;
     const u32 lane = threadIdx.x & 31;
     F f;
@@ -953,7 +1372,7 @@ __device__ __noinline__ int ffind_baby(const Fp64& f, double tbl, double B32, u3
 // CH interleaved chains per lane: baby index i = lane + 32c + 32*CH*k,
 // giant step g = 1 + lane + 32c + 32*CH*k.
 template <int CH>
-__device__ u64 solve_fp64(const Entry& e, u32* tab, u32 tbits, u64* steps_out) {
+__device__ u64 solve_fp64(const Solve& e, u32* tab, u32 tbits, u64* steps_out) {
     const u32 lane = threadIdx.x & 31;
     Fp64 f;
     f.init(e.p);
@@ -1227,7 +1646,7 @@ __device__ __forceinline__ u32 fq_probe(const uint2* t2, u32 h, u32 shift, u32 t
 // after the words) instead of one compare-and-swap each (table kind 0); the
 // words and the probes are the same.
 template <int CH, bool WI>
-__device__ u64 solve_fp64q(const Entry& e, unsigned long long* tab, u32 tbits, u32 fill, u64* steps_out) {
+__device__ u64 solve_fp64q(const Solve& e, unsigned long long* tab, u32 tbits, u32 fill, u64* steps_out) {
     const u32 lane = threadIdx.x & 31;
     Fp64 f;
     f.init(e.p);
@@ -1430,7 +1849,7 @@ __device__ __forceinline__ bool h_contains(const unsigned short* tab, u32 mask, 
 }
 
 template <int CH>
-__device__ u64 solve_fp64h(const Entry& e, unsigned short* tab, u32 tbits, u32 load_shift, u64* steps_out) {
+__device__ u64 solve_fp64h(const Solve& e, unsigned short* tab, u32 tbits, u32 load_shift, u64* steps_out) {
     const u32 lane = threadIdx.x & 31;
     Fp64 f;
     f.init(e.p);
@@ -1550,7 +1969,7 @@ __device__ u64 solve_fp64h(const Entry& e, unsigned short* tab, u32 tbits, u32 l
 }
 
 template <int CH, int QT>
-__device__ __forceinline__ u64 solve_any(const Entry& e, void* tab, u32 tbits, u32 load_shift, u32 fill, u64* steps) {
+__device__ __forceinline__ u64 solve_any(const Solve& e, void* tab, u32 tbits, u32 load_shift, u32 fill, u64* steps) {
     if (CH == 0 || e.p >= kFp64Limit) return solve_entry<FieldM>(e, (unsigned short*)tab, tbits + 1, steps);
     if (QT == 0) return solve_fp64q<CH ? CH : 1, false>(e, (unsigned long long*)tab, tbits, fill, steps);
     if (QT == 2) return solve_fp64h<CH ? CH : 1>(e, (unsigned short*)tab, tbits, load_shift, steps);
@@ -1561,11 +1980,18 @@ __device__ __forceinline__ u64 solve_any(const Entry& e, void* tab, u32 tbits, u
 // Whether a prime's baby steps fit the table its solve will use (at most half
 // of its keys' room), so that every insertion finds a free slot.
 template <int CH, int QT>
-__device__ __forceinline__ bool fits_table(const Entry& e, u32 tbits) {
+__device__ __forceinline__ bool fits_table(const Solve& e, u32 tbits) {
     if (CH == 0 || e.p >= kFp64Limit) return e.m <= (1u << tbits);          // 2^(tbits+1) 16-bit slots
     if (QT == 0 || QT == 3) return e.m <= (1u << tbits);                    // 2^(tbits-1) words of four
     if (QT == 2) return e.m <= (1u << tbits);                               // 2^(tbits+1) 16-bit slots
     return e.m < (1u << tbits);                                            // 2^tbits 32-bit slots
+}
+
+__device__ __forceinline__ Solve solve_of(const Entry& g) {
+    Solve e;
+    e.p = g.p; e.t = g.t; e.G0 = g.G0; e.B = g.B; e.Bm = g.Bm;
+    e.jcount = g.jcount; e.m = g.m;
+    return e;
 }
 
 // CH > 0: every entry has p < 2^49 (FP64 solve with CH chains per lane);
@@ -1576,35 +2002,35 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counter
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // per warp 4 << tbits bytes of table (kind 3: and one count byte per eight)
     u32* tab = smem32 + (size_t)warp * ((1u << a.tbits) + (QT == 3 ? (1u << a.tbits) / 8 : 0u));
-    const u64 n_ent = min((u64)*(volatile unsigned long long*)&ctr->entries, a.ent_cap);
+    const u64 n_ent = *(volatile unsigned long long*)&ctr->big;
     u64 my_steps = 0, my_baby = 0;
     if (a.persistent) {
-        // A warp claims the entry after the one it solves, and lanes 0..8 load
-        // that entry's nine words while the current one is solved, so neither
-        // the claim nor the load is waited for between entries.
-        static_assert(sizeof(Entry) == 72, "entry staging assumes nine 64-bit words");
+        // A warp claims the entry after the one it solves, and lanes 0..5 load
+        // that entry's words while the current one is solved, so neither the
+        // claim nor the load is waited for between entries.
+        static_assert(offsetof(Entry, jcount) == 40 && offsetof(Entry, m) == 44, "entry staging assumes p, t, G0, B, Bm, then jcount and m in one word");
         u64 cur = 0;
         if (lane == 0) cur = atomicAdd(&ctr->work_next, 1ull);
         cur = __shfl_sync(FULL, cur, 0);
         u64 claim = 0;                                          // lane 0: the entry after cur
         if (lane == 0 && cur < n_ent) claim = atomicAdd(&ctr->work_next, 1ull);
-        u64 stage = cur < n_ent && lane < 9 ? reinterpret_cast<const u64*>(a.ent + cur)[lane] : 0;
+        u32 idx = cur < n_ent ? a.big[cur] : 0u;
+        u64 stage = cur < n_ent && lane < 6 ? reinterpret_cast<const u64*>(a.ent + idx)[lane] : 0;
         while (cur < n_ent) {
             // the solve's fields; n_first, L and item are read again for a relation
-            Entry e;
+            Solve e;
             e.p = __shfl_sync(FULL, stage, 0);
             e.t = __shfl_sync(FULL, stage, 1);
             e.G0 = __shfl_sync(FULL, stage, 2);
             e.B = __shfl_sync(FULL, stage, 3);
             e.Bm = __shfl_sync(FULL, stage, 4);
-            e.n_first = 0;
-            e.L = 0;
-            e.jcount = __shfl_sync(FULL, stage, 7);
-            e.m = (u32)__shfl_sync(FULL, stage, 8);             // little-endian: m, then item
-            e.item = 0;
-            const u64 idx = cur;
+            const u64 jm = __shfl_sync(FULL, stage, 5);         // little-endian: jcount, then m
+            e.jcount = (u32)jm;
+            e.m = (u32)(jm >> 32);
+            const u32 this_idx = idx;
             const u64 next = __shfl_sync(FULL, claim, 0);
-            stage = next < n_ent && lane < 9 ? reinterpret_cast<const u64*>(a.ent + next)[lane] : 0;
+            idx = next < n_ent ? a.big[next] : 0u;
+            stage = next < n_ent && lane < 6 ? reinterpret_cast<const u64*>(a.ent + idx)[lane] : 0;
             if (lane == 0 && next < n_ent) claim = atomicAdd(&ctr->work_next, 1ull);
             cur = next;
             if (!fits_table<CH, QT>(e, a.tbits)) {              // host sizing error: never overfill a table
@@ -1615,7 +2041,7 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counter
             const u64 j = solve_any<CH, QT>(e, tab, a.tbits, a.load_shift, a.fill, &steps);
             if (lane == 0) {
                 if (j != ~0ull) {
-                    const Entry& g = a.ent[idx];
+                    const Entry& g = a.ent[this_idx];
                     emit_relation(e.p, g.n_first + j * g.L, 0, g.item, a.rel, a.rel_cap, ctr);
                 }
                 my_steps += (steps & 0xFFFFFFFFull) + (steps >> 32);
@@ -1627,9 +2053,10 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counter
             atomicAdd(&ctr->baby, (unsigned long long)my_baby);
         }
     } else {
-        const u64 idx = (u64)blockIdx.x * a.warps_per_block + warp;
-        if (idx >= n_ent) return;
-        const Entry e = a.ent[idx];
+        const u64 k = (u64)blockIdx.x * a.warps_per_block + warp;
+        if (k >= n_ent) return;
+        const Entry& g = a.ent[a.big[k]];
+        const Solve e = solve_of(g);
         if (!fits_table<CH, QT>(e, a.tbits)) {
             if (lane == 0) atomicOr(&ctr->status, kStatusBadLaunch);
             return;
@@ -1637,7 +2064,7 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counter
         u64 steps = 0;
         const u64 j = solve_any<CH, QT>(e, tab, a.tbits, a.load_shift, a.fill, &steps);
         if (lane == 0) {
-            if (j != ~0ull) emit_relation(e.p, e.n_first + j * e.L, 0, e.item, a.rel, a.rel_cap, ctr);
+            if (j != ~0ull) emit_relation(e.p, g.n_first + j * g.L, 0, g.item, a.rel, a.rel_cap, ctr);
             atomicAdd(&ctr->steps, (unsigned long long)((steps & 0xFFFFFFFFull) + (steps >> 32)));
             atomicAdd(&ctr->baby, (unsigned long long)(steps & 0xFFFFFFFFull));
         }
@@ -1685,7 +2112,7 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs_groups(BsgsArgs a, 
     unsigned short* tab = reinterpret_cast<unsigned short*>(smem32 + (size_t)warp * (1u << a.tbits)) +
                           (size_t)grp * group_slots;
     const u32 tw_max = a.tbits + 1 - NG_LOG;
-    const u64 n_ent = min((u64)*(volatile unsigned long long*)&ctr->entries, a.ent_cap);
+    const u64 n_ent = *(volatile unsigned long long*)&ctr->big;
     u64 my_steps = 0, my_baby = 0;
     for (;;) {
         u64 first = 0;
@@ -1693,7 +2120,8 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs_groups(BsgsArgs a, 
         first = __shfl_sync(FULL, first, 0);
         if (first >= n_ent) break;
         const u64 idx = first + grp;
-        Entry e = a.ent[idx < n_ent ? idx : n_ent - 1];
+        const Entry& g = a.ent[a.big[idx < n_ent ? idx : n_ent - 1]];
+        const Solve e = solve_of(g);
         bool active = idx < n_ent;
         // the host sends only p < 2^49 and at most half a group table of baby steps here
         if (active && (e.p >= kFp64Limit || e.m > (1u << (tw_max - 1)))) {
@@ -1832,7 +2260,7 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs_groups(BsgsArgs a, 
         }
         __syncwarp();
         if (gl == 0 && active) {
-            if (best < e.jcount) emit_relation(e.p, e.n_first + best * e.L, 0, e.item, a.rel, a.rel_cap, ctr);
+            if (best < e.jcount) emit_relation(e.p, g.n_first + best * g.L, 0, g.item, a.rel, a.rel_cap, ctr);
             my_steps += (u64)baby_done + giant_done;
             my_baby += baby_done;
         }
@@ -2208,9 +2636,8 @@ __global__ void k_bsgs_direct(const u64* cases, u64* j_out, u64 count, u32 tbits
     if (idx >= count) return;
     const u64* c = cases + 5 * idx;
     const u64 p = c[0];
-    Entry e;
+    Solve e;
     e.p = p; e.B = c[1] % p; e.G0 = c[2] % p; e.t = c[3] % p; e.jcount = c[4];
-    e.n_first = 0; e.L = 1; e.item = 0;
     u64 result;
     if (e.jcount == 0) {
         result = ~0ull;
@@ -2269,8 +2696,8 @@ u32 range_seg_words(u32 seg_words, u64 n_odds) {
     return seg_words;
 }
 
-cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, u64* surv, u32* surv_item, u64 surv_cap,
-                         Counters* ctr, cudaStream_t s, u32 seg_words) {
+cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, const SurvOut& o, Counters* ctr, cudaStream_t s,
+                         u32 seg_words) {
     if (!valid_seg_words(seg_words)) return cudaErrorInvalidValue;
     seg_words = range_seg_words(seg_words, a.n_odds);
     const u64 seg_odds = (u64)seg_words * 32;
@@ -2278,7 +2705,7 @@ cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, u64* surv, u3
     if (segs == 0 && !a.include_two) return cudaSuccess;
     const u64 grid = segs == 0 ? 1 : min(segs, (u64)148 * 8);
     auto go = [&](auto kern) {
-        kern<<<(unsigned)grid, kSieveThreads, 0, s>>>(a, t, surv, surv_item, surv_cap, ctr);
+        kern<<<(unsigned)grid, kSieveThreads, 0, s>>>(a, t, o, ctr);
         return cudaGetLastError();
     };
     switch (seg_words) {
@@ -2290,17 +2717,20 @@ cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, u64* surv, u3
     }
 }
 
-cudaError_t launch_sieve_wave(const WaveDesc* w, const SieveTables& t, u64* surv, u32* surv_item, u64 surv_cap,
-                              Counters* ctr, int grid, cudaStream_t s, u32 seg_words) {
+cudaError_t launch_sieve_wave(const WaveDesc* w, const SieveTables& t, const SurvOut& o, Counters* ctr, int grid,
+                              cudaStream_t s, u32 seg_words) {
     if (!valid_seg_words(seg_words)) return cudaErrorInvalidValue;
-    if (seg_words == 1024) k_sieve_wave<1024><<<grid, kSieveThreads, 0, s>>>(w, t, surv, surv_item, surv_cap, ctr);
-    else if (seg_words == 4096) k_sieve_wave<4096><<<grid, kSieveThreads, 0, s>>>(w, t, surv, surv_item, surv_cap, ctr);
-    else k_sieve_wave<2048><<<grid, kSieveThreads, 0, s>>>(w, t, surv, surv_item, surv_cap, ctr);
+    if (seg_words == 1024) k_sieve_wave<1024><<<grid, kSieveThreads, 0, s>>>(w, t, o, ctr);
+    else if (seg_words == 4096) k_sieve_wave<4096><<<grid, kSieveThreads, 0, s>>>(w, t, o, ctr);
+    else k_sieve_wave<2048><<<grid, kSieveThreads, 0, s>>>(w, t, o, ctr);
     return cudaGetLastError();
 }
 
-cudaError_t launch_prep(const PrepArgs& a, Counters* ctr, int grid, cudaStream_t s) {
+cudaError_t launch_prep(const PrepArgs& a, Counters* ctr, int grid, int num_sms, cudaStream_t s) {
     k_prep<<<grid, kPrepThreads, 0, s>>>(a, ctr);
+    if (!a.surv_split) k_split<<<num_sms * 2, 256, 0, s>>>(a, ctr);
+    k_dlog<<<num_sms * 3, 256, 0, s>>>(a, ctr);
+    k_setup<<<num_sms * 3, 256, 0, s>>>(a, ctr);
     return cudaGetLastError();
 }
 

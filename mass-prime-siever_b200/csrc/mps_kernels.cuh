@@ -21,13 +21,24 @@ struct SieveArgs {
     u64 hi;            // exclusive bound
     u32 include_two;
     u32 n_primes;      // sieving primes to use (those with q*q < hi, at most 6541)
+    u32 n_split;       // split primes to look for in p - 1 (at most kSplitPrimes; 0: none)
     u32 item;          // item index stored with the survivors
+};
+
+// Where the survivors go: surv[], their items (or nullptr), and the split
+// primes l | p - 1 of each (nullptr: not looked for): one 16-bit l index + 1
+// per size class, 0 where there is none.
+struct SurvOut {
+    u64* surv;
+    u32* item;
+    u64* split;
+    u64 cap;
 };
 
 // seg_words: segment bitmap words (1024, 2048 or 4096; 32 odd numbers each)
 constexpr u32 kDefaultSegWords = 2048;
-cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, u64* surv, u32* surv_item, u64 surv_cap,
-                         Counters* ctr, cudaStream_t s, u32 seg_words = kDefaultSegWords);
+cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, const SurvOut& o, Counters* ctr, cudaStream_t s,
+                         u32 seg_words = kDefaultSegWords);
 
 // A wave: several runs (odd ranges of possibly different items) sieved by
 // one launch; kept in device memory so that a captured graph is replayable.
@@ -40,7 +51,7 @@ struct SieveRun {
     u32 n_primes;
     u32 include_two;
     u32 item;
-    u32 pad;
+    u32 n_split;
 };
 
 // Device-resident state of one item: every P below p_done is sieved once the
@@ -68,18 +79,26 @@ cudaError_t launch_commit(const WaveDesc* w, const RawRelation* rel, const Count
 // its n relations rel[0..n) appended to the item's state.
 cudaError_t launch_state_add(ItemState* st, u32 item, u64 hi, const RawRelation* rel, u64 n, cudaStream_t s);
 // The wave's runs' seg_begin must count segments of seg_words * 32 odd numbers.
-cudaError_t launch_sieve_wave(const WaveDesc* w, const SieveTables& t, u64* surv, u32* surv_item, u64 surv_cap,
-                              Counters* ctr, int grid, cudaStream_t s, u32 seg_words = kDefaultSegWords);
+cudaError_t launch_sieve_wave(const WaveDesc* w, const SieveTables& t, const SurvOut& o, Counters* ctr, int grid,
+                              cudaStream_t s, u32 seg_words = kDefaultSegWords);
 
-// Prep: filters, primality screen and BSGS set-up for every survivor.
+// Prep: filters, primality screen and class combination for every survivor
+// (k_prep), the split by larger primes l | p - 1 (k_dlog; k_split finds them
+// where the sieve has not), and the BSGS set-up, which also solves the primes
+// with few candidates left (k_setup).
 struct PrepArgs {
     const u64* surv;
     u64 surv_cap;
     const u32* surv_item;      // nullptr: every survivor belongs to `item0`
+    const u64* surv_split;     // the sieve's split primes (SurvOut::split); nullptr: k_split finds them
+    SieveTables tables;
     u32 item0;
     const DevItem* items;
     Entry* ent;
-    u64 ent_cap;
+    u64 ent_cap;               // < 2^32
+    SplitEvent* events;        // kSplitClasses lists of ev_cap events each
+    u64 ev_cap;
+    u32* big;                  // ent_cap indices: the entries k_bsgs solves
     RawRelation* rel;
     u64 rel_cap;
     u32 full_mr;               // 1: 12-base Miller-Rabin on every survivor that passes the filters
@@ -88,12 +107,19 @@ struct PrepArgs {
     u64 prime_below;           // survivors below this are prime (sieved by every prime up to their
                                // square root: 65521^2 for the sieve's survivors, 0 for caller-given numbers)
 };
+// Events a list needs for ent_cap entries: an entry has 0.3 in the fullest
+// class on average; a full list loses splits, never relations.
+constexpr u64 split_event_cap(u64 ent_cap) { return ent_cap / 2; }
+// Split primes to look for in the range of an item with K in-class exponents.
+u32 split_primes_for(u64 K);
 constexpr u64 kSievedPrimeBelow = (u64)kSieveMaxPrime * kSieveMaxPrime;
-cudaError_t launch_prep(const PrepArgs& a, Counters* ctr, int grid, cudaStream_t s);
+constexpr u32 kPrepLaunches = 3;      // kernels of one launch_prep (one more without surv_split)
+cudaError_t launch_prep(const PrepArgs& a, Counters* ctr, int grid, int num_sms, cudaStream_t s);
 
 // Exact BSGS, one warp per entry.
 struct BsgsArgs {
     const Entry* ent;
+    const u32* big;            // indices of the entries to solve (ctr->big of them)
     u64 ent_cap;
     RawRelation* rel;
     u64 rel_cap;

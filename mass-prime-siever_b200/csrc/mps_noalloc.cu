@@ -40,8 +40,9 @@ namespace {
 
 // Largest range one call takes: 2^19 integers (2^18 odd numbers).
 constexpr u64 kNoAllocMaxSpan = 1ull << 19;
-constexpr u64 kNoAllocOdds = kNoAllocMaxSpan / 2 + 2;
-constexpr u64 kNoAllocEntries = 1ull << 16;
+constexpr u64 kNoAllocEntries = 3ull << 14;          // more than the 43,390 primes below 2^19, the most a range holds
+constexpr u64 kNoAllocSurv = kNoAllocEntries;        // (the same bound holds for the sieve's survivors)
+constexpr u64 kNoAllocEvents = kNoAllocEntries / 4;  // per split list (a full list loses splits, not relations)
 constexpr u64 kNoAllocRelations = 1ull << 14;
 constexpr u32 kNoAllocMaxDevices = 64;
 
@@ -52,8 +53,11 @@ constexpr size_t kOffSp = align256(kOffItem + sizeof(DevItem));
 constexpr size_t kOffRcp = align256(kOffSp + kSievePrimes * sizeof(u32));
 constexpr size_t kOffInv = align256(kOffRcp + kSievePrimes * sizeof(u64));
 constexpr size_t kOffSurv = align256(kOffInv + kSievePrimes * sizeof(u64));
-constexpr size_t kOffEnt = align256(kOffSurv + kNoAllocOdds * sizeof(u64));
-constexpr size_t kOffRel = align256(kOffEnt + kNoAllocEntries * sizeof(Entry));
+constexpr size_t kOffSplit = align256(kOffSurv + kNoAllocSurv * sizeof(u64));
+constexpr size_t kOffEnt = align256(kOffSplit + kNoAllocSurv * sizeof(u64));
+constexpr size_t kOffEvents = align256(kOffEnt + kNoAllocEntries * sizeof(Entry));
+constexpr size_t kOffBig = align256(kOffEvents + kSplitClasses * kNoAllocEvents * sizeof(SplitEvent));
+constexpr size_t kOffRel = align256(kOffBig + kNoAllocEntries * sizeof(u32));
 constexpr size_t kNoAllocUsed = align256(kOffRel + kNoAllocRelations * sizeof(RawRelation));
 constexpr size_t kNoAllocBytes = 8u << 20;
 static_assert(kNoAllocUsed <= kNoAllocBytes, "no-alloc scratch layout exceeds its array");
@@ -157,6 +161,7 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     Counters* ctr = (Counters*)(base + kOffCounters);
     DevItem* ditem = (DevItem*)(base + kOffItem);
     u64* surv = (u64*)(base + kOffSurv);
+    u64* split = (u64*)(base + kOffSplit);
     Entry* ent = (Entry*)(base + kOffEnt);
     RawRelation* rel = (RawRelation*)(base + kOffRel);
     const SieveTables tables{(const u32*)(base + kOffSp), (const u64*)(base + kOffRcp), (const u64*)(base + kOffInv)};
@@ -169,16 +174,22 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     sa.hi = hi;
     sa.include_two = (lo <= 2 && hi > 2) ? 1 : 0;
     sa.n_primes = prime_count_below_sqrt(hi);
+    sa.n_split = split_primes_for(d.K);
     sa.item = 0;
     if (sa.n_odds == 0 && !sa.include_two) return MPS_OK;
 
     PrepArgs pa{};
     pa.surv = surv;
-    pa.surv_cap = kNoAllocOdds;
+    pa.surv_cap = kNoAllocSurv;
+    pa.surv_split = split;
+    pa.tables = tables;
     pa.item0 = 0;
     pa.items = ditem;
     pa.ent = ent;
     pa.ent_cap = kNoAllocEntries;
+    pa.events = (SplitEvent*)(base + kOffEvents);
+    pa.ev_cap = kNoAllocEvents;
+    pa.big = (u32*)(base + kOffBig);
     pa.rel = rel;
     pa.rel_cap = kNoAllocRelations;
     pa.m_cap = std::min<u32>(noalloc_holds(tbits), kMaxBaby);
@@ -186,6 +197,7 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     pa.prime_below = kSievedPrimeBelow;                      // survivors of the sieve
     BsgsArgs ba{};
     ba.ent = ent;
+    ba.big = pa.big;
     ba.ent_cap = kNoAllocEntries;
     ba.rel = rel;
     ba.rel_cap = kNoAllocRelations;
@@ -207,8 +219,8 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     const int bgrid = num_sms * std::max(1, std::min((int)(228 * 1024 / (smem + 1024)), 16));
     if (cudaMemsetAsync(ctr, 0, sizeof(Counters), s) != cudaSuccess) return MPS_E_CUDA;
     if (cudaMemcpyAsync(ditem, &d, sizeof(DevItem), cudaMemcpyHostToDevice, s) != cudaSuccess) return MPS_E_CUDA;
-    if (launch_sieve(sa, tables, surv, nullptr, kNoAllocOdds, ctr, s) != cudaSuccess) return MPS_E_CUDA;
-    if (launch_prep(pa, ctr, num_sms * 4, s) != cudaSuccess) return MPS_E_CUDA;
+    if (launch_sieve(sa, tables, SurvOut{surv, nullptr, split, kNoAllocSurv}, ctr, s) != cudaSuccess) return MPS_E_CUDA;
+    if (launch_prep(pa, ctr, num_sms * 4, num_sms, s) != cudaSuccess) return MPS_E_CUDA;
     if (launch_bsgs(ba, ctr, bgrid, s) != cudaSuccess) return MPS_E_CUDA;
     if (launch_order(oa, ctr, num_sms * 2, s) != cudaSuccess) return MPS_E_CUDA;
     Counters h;
