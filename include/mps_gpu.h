@@ -67,8 +67,9 @@ typedef struct mps_tuning {
     uint32_t max_baby;          /* cap on the baby-step count (0: what the table holds)        */
     uint32_t bsgs_warps;        /* warps per BSGS block (0: 4)                                 */
     uint32_t class_modulus;     /* Q of the power-residue split g = gcd(Q, p-1), even, <= 2^28
-                                   (0: lcm(mod, 232792560), else lcm(mod, 720720), else
-                                    lcm(mod, 5040), the first within 2^28, else 5040;
+                                   (0: lcm(mod, 144), else lcm(mod, 24), the first within
+                                    2^28, else 144, and a further split by every prime
+                                    5..4261 that divides p - 1;
                                     1: lcm(mod, 2), the reference's plain-method filter)       */
     uint32_t full_mr;           /* 1: 12-base Miller-Rabin on every filter survivor (eager)    */
     uint32_t plain;             /* 1: plain per-chunk path (host sync between stages)          */

@@ -53,6 +53,8 @@ struct DevItem {
     u32 item_index;
     u32 qf_n;              // prime factors of Q: qf_l[0..qf_n)
     u32 qf_l[9];
+    double b_small, t_small;   // b and -c as signed numbers below 2^20, 0 when they are larger
+    u32 strong;            // 1: a base-2 strong test screens the survivors (|b| <= 1 proves nothing)
     u32 split_more;        // 1: also split by primes l | p - 1 that Q does not hold (k_dlog)
     // Quadratic-character prefilter (both |b| and |c| below 2^32): for x = b
     // and x = -c, x = (-1)^neg 2^k o with o odd; rcp = floor((2^64-1) / o).
@@ -62,17 +64,22 @@ struct DevItem {
 };
 
 // The split by primes l | p - 1 outside the split modulus: the kSplitPrimes
-// sieving primes from 23 (to 4261), in kSplitClasses size classes; class c holds
-// the indices (from 23) below kSplitClassEnd[c] that no earlier class holds.
-constexpr u32 kSplitClasses = 4;
-constexpr u32 kSplitBase = 7;                 // 23's place among the sieving primes
-constexpr u32 kSplitGroups = 18, kSplitPrimes = 32 * kSplitGroups;
-__host__ __device__ constexpr u32 split_class(u32 k) { return k < 10 ? 0u : k < 46 ? 1u : k < 164 ? 2u : 3u; }   // l < 64, 256, 1024
+// sieving primes from 5 (to 4261); k is an l's index among them.  The first
+// kSplitSmall (5 .. 19) have a slot of an entry each; the sieve finds the others,
+// one of each of kSplitClasses size classes, a slot a class.  Events queue in
+// lists by size, the classes' and one for the small l, for each of the two
+// arithmetics (kFp64Limit).
+constexpr u32 kSplitBase = 1;                 // 5's place among the sieving primes
+constexpr u32 kSplitSmall = 6, kSplitGroups = 18, kSplitPrimes = kSplitSmall + 32 * kSplitGroups;
+constexpr u32 kSplitClasses = 4, kSplitSizes = kSplitClasses + 1, kSplitLists = 2 * kSplitSizes, kSplitSlots = kSplitClasses + kSplitSmall;
+__host__ __device__ constexpr u32 split_class(u32 k) {       // k >= kSplitSmall; l < 64, 256, 1024
+    return k < 16 ? 0u : k < 52 ? 1u : k < 170 ? 2u : 3u;
+}
+__host__ __device__ constexpr u32 slot_list(u32 slot) { return slot < kSplitClasses ? slot : kSplitClasses; }
 
 // One prime that reached the discrete-log stages: the candidates left are
 // n = n_first + j*L, j in [0, jcount).  The prep writes p, n_first, L, jcount,
-// item and the primes l | p - 1 to split the candidates by (one of each size
-// class at most); k_dlog resolves those; k_setup applies them and fills t, G0,
+// item and the primes l | p - 1 to split the candidates by; k_dlog resolves those; k_setup applies them and fills t, G0,
 // B, Bm and m for the solve of G0 * B^j == t (mod p).
 struct Entry {
     u64 p;
@@ -85,17 +92,17 @@ struct Entry {
     u64 n_first;          // smallest candidate n
     u64 L;
     u32 item;             // item index (batched runs)
-    u32 ev[kSplitClasses];   // 0: none, else l's index + 1 << 16 | what k_dlog found (kEv*)
+    u32 ev[kSplitSlots];     // 0: none, else l's index + 1 << 16 | what k_dlog found (kEv*)
     u32 pad;
 };
 constexpr u32 kEvUnknown = 0xFFFFu;   // nothing learned: b is an l-th power residue and so is t
 constexpr u32 kEvReject = 0xFFFEu;    // no n solves it: b is an l-th power residue and t is not
-                                      // (anything else: n == this (mod l))
+                                      // (anything else: j == this (mod l))
 
-// A prime l | p - 1 of an entry, queued for k_dlog (in the list of l's class).
+// A prime l | p - 1 of an entry, queued for k_dlog.
 struct SplitEvent {
     u32 entry;            // entry index
-    u32 k;                // l's index
+    u32 which;            // l's index << 16 | slot
 };
 
 // What a solve needs of an entry (plain residues in [0, p)): the smallest j in
@@ -124,7 +131,7 @@ struct Counters {
     unsigned long long steps;      u64 pad6[7];   // baby + giant steps executed by the BSGS
     unsigned long long prep_next;  u64 pad7[7];   // next survivor the prep's warps claim
     unsigned long long baby;       u64 pad8[7];   // the baby steps among `steps`
-    unsigned long long events[kSplitClasses]; u64 pad9[8 - kSplitClasses];   // split events queued, by size class
+    unsigned long long events[kSplitLists]; u64 pad9[16 - kSplitLists];   // split events queued, by list
     unsigned long long setup_next; u64 pad10[7];  // next entry the set-up's warps claim
     unsigned long long big;        u64 pad11[7];  // entries left for a warp each (k_bsgs)
 };

@@ -23,20 +23,21 @@ inline u64 gcd_host(u64 a, u64 b) {
 constexpr u64 kMaxSplit = 1ull << 28;       // largest split modulus (at most 9 distinct primes)
 
 // The split modulus Q of a tuning value: 0 -> lcm(cm, B) for the first B of
-// kSplitBases whose lcm stays within 2^28 (5040 when none does); 1 ->
+// kSplitBases whose lcm stays within 2^28 (144 when none does); 1 ->
 // lcm(cm, 2), the reference's plain-method filter (Gpu.hpp:247-298: the
 // Legendre test and the gcd(mod, p-1)-th power test); anything else as given.
 // Every prime l of Q with l | p - 1 splits a prime's exponents into l classes
-// and keeps one, so a larger Q leaves fewer BSGS steps (about 1/(l-1) of the
-// primes gain a factor l); the prep pays a longer walk for them.
-constexpr u64 kSplitBases[] = {232792560ull, 720720ull, 5040ull};   // 2^4 3^2 5 7 11 13 17 19; to 13; to 7
+// and keeps one.  Beyond the powers of 2 and 3 that leaves to the split by
+// single primes (split_more), which spends its discrete logarithms only on the
+// primes that got through the class conditions.
+constexpr u64 kSplitBases[] = {144ull, 24ull};
 inline u64 split_modulus(u32 class_modulus, u64 cm) {
     if (class_modulus == 0) {
         for (u64 base : kSplitBases) {
             const u64 l = cm / gcd_host(cm, base) * base;
             if (l <= kMaxSplit) return l;
         }
-        return 5040;
+        return 144;
     }
     if (class_modulus == 1) return cm % 2 == 0 ? cm : 2 * cm;
     return class_modulus;
@@ -88,6 +89,9 @@ inline int item_constants(const mps_item* it, u32 class_modulus, u32 index, DevI
     if (x > 1) d->qf_l[d->qf_n++] = (u32)x;
     d->cmQ = (u32)(cm % Q);
     d->nsQ = (u32)(d->n_start % Q);
+    if (babs < (1u << 20)) d->b_small = b < 0 ? -(double)(u64)babs : (double)(u64)babs;
+    if (cabs < (1u << 20)) d->t_small = c > 0 ? -(double)(u64)cabs : (double)(u64)cabs;
+    d->strong = babs <= 1;
     d->split_more = class_modulus == 0;       // an explicit Q is the whole split
     d->item_index = index;
     d->baby_scale = kDefaultBabyScale;

@@ -78,7 +78,7 @@ __device__ __forceinline__ void emit_relation(u64 p, u64 M, u64 q, u32 item, Raw
 constexpr u32 kSegWords = 2048;
 constexpr u32 kSieveThreads = 256;
 constexpr u32 kNumPattern = 10;               // 3..31: whole-word patterns, no atomics
-constexpr u32 kSplitShared = 164;             // split primes below 1024: a warp's lanes share each
+constexpr u32 kSplitShared = 170;             // split primes below 1024: a warp's lanes share each
 constexpr u32 kNumMedium = 171;               // primes below 1024: a warp's lanes share each prime
 
 // Index j >= 0 of the first odd multiple v0 + 2j of q with v0 + 2j >= v0 (v0 odd).
@@ -249,14 +249,14 @@ __device__ void sieve_segment(SieveShared<W>& sh, u64 v0, u32 len, u32 n_primes,
         }
     }
     if (base + rank > o.cap) atomicOr(&ctr->status, kStatusSurvivorOverflow);
-    if (o.split && n_split) {
+    if (o.split && n_split > kSplitSmall) {
         // 5. the split primes l | v - 1: the bitmap walked once more, from the
         // first v == 1 (mod l), a warp's lanes sharing each l below 1024 (the
         // first three classes), one thread each of the others.  A survivor keeps one
         // l of each size class (a second one of a class, 4% of them, overwrites
         // the first).  This costs 1/l visits an odd number, about a tenth of
         // trying the primes on each entry (k_split).
-        for (u32 k = tid; k < n_split; k += kSieveThreads) {
+        for (u32 k = kSplitSmall + tid; k < n_split; k += kSieveThreads) {
             const u32 q = t.sp[kSplitBase + k];
             u32 r = (u32)(v0 - __umul64hi(v0, t.rcp[kSplitBase + k]) * q);
             if (r >= q) r -= q;
@@ -273,7 +273,7 @@ __device__ void sieve_segment(SieveShared<W>& sh, u64 v0, u32 len, u32 n_primes,
             }
         };
         const u32 n_shared = min(n_split, kSplitShared);
-        for (u32 k = warp; k < n_shared; k += kSieveThreads / 32) {
+        for (u32 k = kSplitSmall + warp; k < n_shared; k += kSieveThreads / 32) {
             const u32 q = t.sp[kSplitBase + k], c = split_class(k);
             for (u32 i = sh.split_start[k] + lane * q; i < len; i += 32 * q) visit(i, c, k);
         }
@@ -333,6 +333,27 @@ __global__ void __launch_bounds__(kSieveThreads) k_sieve_wave(const WaveDesc* w,
 // eq(a, c) compares a product (or one()) with a canonical value c without
 // leaving the field's representation.
 
+// a^e two bits at a time (a product for every two squarings, chosen from 1, a,
+// a^2, a^3 without a branch).
+template <class F>
+__device__ __forceinline__ typename F::V pow_window(const F& f, typename F::V a, u64 e) {
+    typedef typename F::V V;
+    const V one = f.one();
+    if (e == 0) return one;
+    const V a2 = f.mul(a, a), a3 = f.mul(a2, a);
+    int k = (63 - __clzll((long long)e)) & ~1;
+    const u32 top = (u32)(e >> k) & 3u;
+    V x = top == 1 ? a : top == 2 ? a2 : a3;
+    for (k -= 2; k >= 0; k -= 2) {
+        const u32 dgt = (u32)(e >> k) & 3u;
+        const V lo = dgt & 1u ? a : one, hi = dgt & 1u ? a3 : a2;
+        x = f.mul(x, x);
+        x = f.mul(x, x);
+        x = f.mul(x, dgt & 2u ? hi : lo);
+    }
+    return x;
+}
+
 struct FieldF {
     typedef double V;
     Fp64 f;
@@ -351,6 +372,45 @@ struct FieldF {
     __device__ __forceinline__ V dbl(V a) const { return __dadd_rn(a, a); }      // (-p, p) -> (-2p, 2p)
     __device__ __forceinline__ V pow(V b, u64 e) const { return f.pow(b, e); }
     __device__ __forceinline__ bool eq(V a, V c) const { return a == c || a == c - f.p; }   // a in (-p, p)
+
+    // Powers of a small base s (|s| p <= 2^50), from the top bit down: x <- x^2 s^bit
+    // as (x s) x, where x s is exact (below 2^53), so a bit costs one product more
+    // than a squaring's six instead of six.  The quotient of (x s) x by p is below
+    // 0.43 * 2^50 and its estimate off by at most 1/2 + 2^-52 of that, so with
+    // |x| <= 0.66 p, |x'| <= p (1/2 + 0.43 * 2^-2) <= 0.61 p: the values stay small
+    // (the first one, s itself, is below p, and its square below 3/4 p, then
+    // 0.65 p).  About 10 issue slots a bit against 16 for square-and-multiply.
+    __device__ __forceinline__ bool small(double s) const { return s != 0.0 && fabs(s) * f.p <= 1125899906842624.0 && fabs(s) < f.p; }
+    __device__ __forceinline__ V pow_small(double s, u64 e) const {
+        if (e == 0) return 1.0;
+        double x = s;
+        for (int k = 62 - __clzll((long long)e); k >= 0; --k) {
+            const double y = (e >> k) & 1 ? __dmul_rn(x, s) : x;
+            x = f.mul(y, x);
+        }
+        return x;
+    }
+    // b^e and t^e (t = -c) for e > 0.
+    __device__ __forceinline__ void powers(const DevItem& it, u64 e, V& w, V& u) const {
+        const double bs = it.b_small, ts = it.t_small;
+        if (small(bs) && small(ts)) {
+            w = bs;
+            u = ts;
+            for (int k = 62 - __clzll((long long)e); k >= 0; --k) {
+                const bool bit = (e >> k) & 1;
+                const double y = bit ? __dmul_rn(w, bs) : w, z = bit ? __dmul_rn(u, ts) : u;
+                w = f.mul(y, w);
+                u = f.mul(z, u);
+            }
+            return;
+        }
+        w = b_power(it, e);
+        u = small(ts) ? pow_small(ts, e) : pow_window(*this, from_u64(f.pi - residue128(it.cabs_hi, it.cabs_lo, it.c_neg, f.pi)), e);
+    }
+    __device__ __forceinline__ V b_power(const DevItem& it, u64 e) const {
+        return small(it.b_small) ? pow_small(it.b_small, e)
+                                 : pow_window(*this, from_u64(residue128(it.babs_hi, it.babs_lo, it.b_neg, f.pi)), e);
+    }
 };
 
 struct FieldM {
@@ -371,6 +431,13 @@ struct FieldM {
     __device__ __forceinline__ V dbl(V a) const { return M.dbl(a); }
     __device__ __forceinline__ V pow(V b, u64 e) const { return M.pow(b, e); }
     __device__ __forceinline__ bool eq(V a, V c) const { return a == c || a == c + M.p; }   // a in [0, 2p)
+    __device__ __forceinline__ void powers(const DevItem& it, u64 e, V& w, V& u) const {
+        w = b_power(it, e);
+        u = pow_window(*this, from_u64(M.p - residue128(it.cabs_hi, it.cabs_lo, it.c_neg, M.p)), e);
+    }
+    __device__ __forceinline__ V b_power(const DevItem& it, u64 e) const {
+        return pow_window(*this, from_u64(residue128(it.babs_hi, it.babs_lo, it.b_neg, M.p)), e);
+    }
 };
 
 // --------------------------------------------------------------- the prep --
@@ -457,50 +524,81 @@ __device__ __forceinline__ u64 exact_quotient(u64 pm1, u32 g) {
     return (pm1 >> tz) * (0 - Mont::neg_inverse((u64)(g >> tz)));
 }
 
+// gcd(Q, p - 1): the power of two by counting zeros, the odd parts by the
+// binary algorithm (no divisions).
 __device__ __forceinline__ u32 gcd_Q(const DevItem& it, u64 pm1) {
     const u64 qh = __umul64hi(pm1, it.Q_rcp);
     u32 rem = (u32)(pm1 - qh * it.Q);
     if (rem >= it.Q) rem -= it.Q;
-    return gcd32(it.Q, rem);
+    if (rem == 0) return it.Q;
+    const int zq = __ffs((int)it.Q) - 1, zr = __ffs((int)rem) - 1;
+    u32 x = it.Q >> zq, y = rem >> zr;
+    while (x != y) {
+        const u32 d = x > y ? x - y : y - x;
+        y = min(x, y);
+        x = d >> (__ffs((int)d) - 1);
+    }
+    return x << min(zq, zr);
 }
 
 // Stage 2: with g = gcd(Q, p - 1) and e = (p - 1) / g, w = b^e and u = t^e
 // are g-th roots of unity and b^n == t forces w^n == u, i.e. n == r (mod d),
 // d = ord(w) -- or there is no solution.  Returns 0 (no solution), 1 (d, r
-// found by a walk of at most `walk` steps) or 2 (longer: deferred, with the
-// residues of w and u in w_out, u_out for stage 2b).
+// found within `walk` steps) or 2 (longer: deferred, with the residues of w
+// and u in w_out, u_out for stage 2b).  This is the primality screen too: a
+// composite p has w^g != 1 but for the rare pseudoprimes to base b, which the
+// order stage drops.
+//
+// The orders and logarithms are found S at a time: with w^(S k) (k = 1,
+// 2, ..) compared with w^i and u w^i, i < S, the largest match i gives the
+// smallest exponent S k - i.  (S = 8 takes as many instructions and 16 more
+// registers, a block less per SM: 2% of the prep.)
+//
+// Against a base-2 strong test of every survivor, the two powers by squaring
+// from the low bit and a walk one step at a time, with 5 .. 19 in Q: k_prep on
+// 2^27 integers at 10^12 0.90 -> 0.55 ms (and k_dlog, which took 5 .. 19 over,
+// 0.21 -> 0.28).
 template <class F>
-__device__ __forceinline__ int power_split(const F& f, u64 p, u64 b_mod, u64 t, const DevItem& it, u32 walk, u32& d,
-                                           u32& r, u64& w_out, u64& u_out) {
+__device__ __forceinline__ int power_split(const F& f, u64 p, const DevItem& it, u32 walk, u32& d, u32& r, u64& w_out,
+                                           u64& u_out) {
     typedef typename F::V V;
+    constexpr u32 S = 4;
     const u64 pm1 = p - 1;
     const u32 g = gcd_Q(it, pm1);
-    const u64 e = exact_quotient(pm1, g);
-    V u = f.one(), w = f.one(), bu = f.from_u64(t), bw = f.from_u64(b_mod);
-    for (u64 x = e; x; x >>= 1) {                      // two exponentiations, interleaved
-        if (x & 1) {
-            u = f.mul(u, bu);
-            w = f.mul(w, bw);
-        }
-        bu = f.mul(bu, bu);
-        bw = f.mul(bw, bw);
-    }
-    const V uc = f.canon(u), one = f.one();
-    V x = one;
-    bool found = false;
-    const u32 lim = min(g, walk);
-    for (u32 k = 0; k < lim; ++k) {                    // discrete log in <w>
-        if (!found && f.eq(x, uc)) {
-            r = k;
-            found = true;
-        }
+    V w, u;
+    f.powers(it, exact_quotient(pm1, g), w, u);
+    V wi[S], ui[S];                                    // w^i, u w^i (canonical)
+    wi[0] = f.canon(f.one());
+    ui[0] = f.canon(u);
+    V x = w, y = f.mul(u, w);
+#pragma unroll
+    for (u32 i = 1; i < S; ++i) {
+        wi[i] = f.canon(x);
+        ui[i] = f.canon(y);
         x = f.mul(x, w);
-        if (f.eq(x, one)) {
-            d = k + 1;
-            return found ? 1 : 0;
-        }
+        y = f.mul(y, w);
     }
-    if (lim == g) return 0;
+    const V step = x;                                  // w^S
+    const u32 lim = min(g, walk);
+    u32 log = ui[0] == wi[0] ? 0 : ~0u, ord = ~0u;
+    for (u32 k = S; k < lim + S && ord == ~0u; k += S) {
+        const V c = f.canon(x);
+        x = f.mul(x, step);
+        u32 mu = 0, mw = 0;                            // the largest i + 1 that matches
+#pragma unroll
+        for (u32 i = 0; i < S; ++i) {
+            if (ui[i] == c) mu = i + 1;
+            if (wi[i] == c) mw = i + 1;
+        }
+        if (mu && log == ~0u) log = k + 1 - mu;
+        if (mw) ord = k + 1 - mw;
+    }
+    if (ord <= lim) {
+        d = ord;
+        r = log;
+        return log < ord ? 1 : 0;
+    }
+    if (lim == g) return 0;                            // w^g != 1: p is not prime
     w_out = f.residue(w);
     u_out = f.residue(u);
     return 2;
@@ -526,7 +624,7 @@ __device__ bool power_split_pp(const F& f, u64 p, u64 w_res, u64 u_res, const De
         const V wl = f.pow(w, k), uc = f.canon(f.pow(u, k)), one = f.one();
         V x = one;
         bool found = false;
-        u32 xr = 0, dl = lc;
+        u32 xr = 0, dl = 0;
         for (u32 y = 0; y < lc; ++y) {
             if (!found && f.eq(x, uc)) {
                 xr = y;
@@ -538,7 +636,7 @@ __device__ bool power_split_pp(const F& f, u64 p, u64 w_res, u64 u_res, const De
                 break;
             }
         }
-        if (!found) return false;
+        if (!found || dl == 0) return false;               // (dl == 0: p is not prime)
         // r' == r (mod d), r' == xr (mod dl); d, dl coprime
         u32 step = 0;                                      // d * dl <= g <= Q <= 2^28
         while ((r + d * step) % dl != xr) ++step;
@@ -586,48 +684,50 @@ __device__ __forceinline__ bool combine_class(u64 p, const DevItem& it, u32 d, u
 
 // How many primes of the table an entry with J candidates is split by.
 __host__ __device__ constexpr u32 split_limit(u32 J) {
-    return J < 512 ? 0u : J < 1024 ? 64u : J < 4096 ? 164u : kSplitPrimes;
+    return J < 512 ? 0u : J < 1024 ? 64u : J < 4096 ? 170u : kSplitPrimes;
 }
 u32 split_primes_for(u64 K) { return split_limit((u32)min(K, (u64)~0u)); }
 
-// Queues the split events of the warp's entries (idx, lanes with ok): k[c] is
-// the index + 1 of the entry's l of class c, 0 for none.  One atomic per class
-// and warp; a full list drops the event.
-__device__ __forceinline__ void queue_events(bool ok, u64 idx, const u32 (&k)[kSplitClasses], const PrepArgs& a,
+// Queues the split events of the warp's entries (idx, lanes with ok) in slots
+// S0 .. S1 - 1: k[slot] is the index + 1 of the entry's l, 0 for none.  One
+// atomic per list and warp; a full list drops the event.
+template <u32 S0, u32 S1>
+__device__ __forceinline__ void queue_events(bool ok, u64 idx, u64 p, const u32 (&k)[kSplitSlots], const PrepArgs& a,
                                              Counters* ctr) {
     const u32 lane = threadIdx.x & 31, below = (1u << lane) - 1;
-    u32 bal[kSplitClasses], mine = 0;                  // mine: lane c < kSplitClasses, events of class c
+    const u32 field = a.two_fields && p >= kFp64Limit ? kSplitSizes : 0u;
+    const u32 second = __ballot_sync(FULL, field != 0), mine_field = field ? second : ~second;
+    u32 pos[kSplitSlots], n[kSplitLists] = {}, mine = 0;
 #pragma unroll
-    for (u32 c = 0; c < kSplitClasses; ++c) {
-        bal[c] = __ballot_sync(FULL, ok && k[c] != 0);
-        if (lane == c) mine = __popc(bal[c]);
+    for (u32 s = S0; s < S1; ++s) {
+        const u32 bal = __ballot_sync(FULL, ok && k[s] != 0), c = slot_list(s);
+        pos[s] = (field ? n[c + kSplitSizes] : n[c]) + __popc(bal & mine_field & below);
+        n[c] += __popc(bal & ~second);
+        n[c + kSplitSizes] += __popc(bal & second);
     }
+#pragma unroll
+    for (u32 c = 0; c < kSplitLists; ++c)
+        if (lane == c) mine = n[c];
     u64 at0 = 0;
     if (mine) at0 = atomicAdd(&ctr->events[lane], (unsigned long long)mine);
 #pragma unroll
-    for (u32 c = 0; c < kSplitClasses; ++c) {
-        const u64 at = __shfl_sync(FULL, at0, c) + __popc(bal[c] & below);
+    for (u32 s = S0; s < S1; ++s) {
+        const u32 c = slot_list(s) + field;
+        const u64 at = __shfl_sync(FULL, at0, c) + pos[s];
         if (!ok) continue;
-        const bool in = k[c] != 0 && at < a.ev_cap;
-        if (in) a.events[c * a.ev_cap + at] = SplitEvent{(u32)idx, k[c] - 1};
-        a.ent[idx].ev[c] = in ? k[c] << 16 | kEvUnknown : 0u;
+        const bool in = k[s] != 0 && at < a.ev_cap;
+        if (in) a.events[c * a.ev_cap + at] = SplitEvent{(u32)idx, (k[s] - 1) << 16 | s};
+        a.ent[idx].ev[s] = in ? k[s] << 16 | kEvUnknown : 0u;
     }
 }
 
-// Two powers with one exponent, interleaved: a^x and b^x.
-template <class F>
-__device__ __forceinline__ void pow_pair(const F& f, typename F::V a, typename F::V b, u64 x, typename F::V& ra,
-                                         typename F::V& rb) {
-    ra = f.one();
-    rb = f.one();
-    for (; x; x >>= 1) {
-        if (x & 1) {
-            ra = f.mul(ra, a);
-            rb = f.mul(rb, b);
-        }
-        a = f.mul(a, a);
-        b = f.mul(b, b);
-    }
+// Whether l divides x, l^-1 mod 2^64 and floor((2^64 - 1) / l) folded at compile time.
+template <u32 L>
+__device__ __forceinline__ bool divides(u64 x) {
+    constexpr u64 i0 = (3ull * L) ^ 2, i1 = i0 * (2 - L * i0), i2 = i1 * (2 - L * i1), i3 = i2 * (2 - L * i2),
+                  inv = i3 * (2 - L * i3);
+    static_assert(inv * L == 1, "inverse");
+    return x * inv <= ~0ull / L;
 }
 
 // The smallest j in [1, J) with G0 * B^j == t, by one lane (~0: none): kLaneBaby
@@ -670,12 +770,16 @@ __device__ u32 lane_solve(const F& f, typename F::V t, typename F::V G0, typenam
     return ~0u;
 }
 
+// What stage 1 tests of primality itself: a base-2 strong test where the powers
+// of b prove nothing (|b| <= 1), all 12 bases when the caller asks for them.
 template <class F>
-__device__ __forceinline__ bool stage1(u64 p, const PrepArgs& a) {
+__device__ __forceinline__ bool stage1(u64 p, const DevItem& it, const PrepArgs& a) {
     if (p < a.prime_below) return true;                // the sieve removed every composite below this
-    F f;
-    f.init(p);
-    if (!sprp2_f(f, p)) return false;
+    if (it.strong) {
+        F f;
+        f.init(p);
+        if (!sprp2_f(f, p)) return false;
+    }
     return !a.full_mr || is_prime64(p);
 }
 
@@ -727,9 +831,7 @@ template <class F>
 __device__ __forceinline__ int split_in(const DevItem& it, u64 p, u32& d, u32& r, u64& w, u64& u) {
     F f;
     f.init(p);
-    const u64 bm = residue128(it.babs_hi, it.babs_lo, it.b_neg, p);
-    const u64 t = p - residue128(it.cabs_hi, it.cabs_lo, it.c_neg, p);
-    return power_split(f, p, bm, t, it, kWalk, d, r, w, u);
+    return power_split(f, p, it, kWalk, d, r, w, u);
 }
 
 template <class F>
@@ -739,7 +841,7 @@ __device__ __forceinline__ bool split_pp_in(const DevItem& it, u64 p, u64 w, u64
     return power_split_pp(f, p, w, u, it, d, r);
 }
 
-__global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr) {
+__global__ void __launch_bounds__(kPrepThreads, 4) k_prep(PrepArgs a, Counters* ctr) {
     __shared__ PrepQueues qs[kPrepWarps];
     PrepQueues& Q = qs[threadIdx.x >> 5];
     const u32 lane = threadIdx.x & 31;
@@ -775,17 +877,30 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr
                     Entry& d = a.ent[slot];
                     d.p = e.p; d.n_first = e.n_first; d.L = e.L; d.jcount = e.jcount; d.item = e.item;
                 }
-                if (a.surv_split) {
-                    const u64 found = ok ? a.surv_split[sv] : 0;
-                    const u32 limit = ok && a.items[e.item].split_more ? split_limit(e.jcount) : 0u;
-                    u32 k[kSplitClasses];
+                // the primes l | p - 1 to split by: 5 .. 19 here, the others from the sieve
+                u32 k[kSplitSlots] = {};
+                if (ok && a.items[e.item].split_more) {
+                    const u32 limit = split_limit(e.jcount), Q = a.items[e.item].Q;
+                    const u64 found = a.surv_split ? a.surv_split[sv] : 0;
 #pragma unroll
                     for (u32 c = 0; c < kSplitClasses; ++c) {
                         k[c] = (u32)(found >> (16 * c)) & 0xFFFFu;
                         if (k[c] > limit) k[c] = 0;
                     }
-                    queue_events(ok, slot, k, a, ctr);
+                    if (limit) {
+                        const u64 pm1 = e.p - 1;
+                        if (divides<5>(pm1)) k[kSplitClasses] = 1;
+                        if (divides<7>(pm1)) k[kSplitClasses + 1] = 2;
+                        if (divides<11>(pm1)) k[kSplitClasses + 2] = 3;
+                        if (divides<13>(pm1)) k[kSplitClasses + 3] = 4;
+                        if (divides<17>(pm1)) k[kSplitClasses + 4] = 5;
+                        if (divides<19>(pm1)) k[kSplitClasses + 5] = 6;
+                    }
+#pragma unroll
+                    for (u32 s = 0; s < kSplitSlots; ++s)
+                        if (k[s] && Q % a.tables.sp[kSplitBase + k[s] - 1] == 0) k[s] = 0;   // Q splits by it
                 }
+                queue_events<0, kSplitSlots>(ok, slot, ok ? e.p : 0, k, a, ctr);
             }
             continue;
         }
@@ -854,8 +969,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr
             continue;
         }
         if (!inputs) break;
-        // stage 1: claim 32 survivors; special cases, the quadratic-character
-        // prefilter, then the base-2 strong test
+        // stage 1: claim 32 survivors; special cases and the quadratic-character prefilter
         u64 first = 0;
         if (lane == 0) first = atomicAdd(&ctr->prep_next, 32ull);
         first = __shfl_sync(FULL, first, 0);
@@ -872,7 +986,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(PrepArgs a, Counters* ctr
             if (a.surv_item) item = a.surv_item[k];
             u64 bm, t;
             if (prep_special(p, a.items[item], a, ctr, bm, t) && !qr_reject(p, a.items[item]))
-                keep = p < kFp64Limit ? stage1<FieldF>(p, a) : stage1<FieldM>(p, a);
+                keep = p < kFp64Limit ? stage1<FieldF>(p, a.items[item], a) : stage1<FieldM>(p, a.items[item], a);
         }
         u32 s1;
         qpush(keep, n1, &s1);
@@ -897,10 +1011,10 @@ __global__ void __launch_bounds__(256, 2) k_split(PrepArgs a, Counters* ctr) {
     u32 inv_lo[kSplitGroups], inv_hi[kSplitGroups], lim[kSplitGroups];
 #pragma unroll
     for (u32 g = 0; g < kSplitGroups; ++g) {
-        const u64 inv = a.tables.inv[kSplitBase + 32 * g + lane];
+        const u64 inv = a.tables.inv[kSplitBase + kSplitSmall + 32 * g + lane];
         inv_lo[g] = (u32)inv;
         inv_hi[g] = (u32)(inv >> 32);
-        lim[g] = (u32)(a.tables.rcp[kSplitBase + 32 * g + lane] >> 32);
+        lim[g] = (u32)(a.tables.rcp[kSplitBase + kSplitSmall + 32 * g + lane] >> 32);
     }
     // few entries: fewer than 32 a warp, so that every warp has some
     const u32 per = (u32)min((u64)32, max((u64)1, n_ent / warps));
@@ -915,14 +1029,14 @@ __global__ void __launch_bounds__(256, 2) k_split(PrepArgs a, Counters* ctr) {
             hi = (u32)(pm1 >> 32);
             limit = a.items[e.item].split_more ? split_limit(e.jcount) : 0u;
         }
-        u32 found[kSplitClasses] = {};
+        u32 found[kSplitSlots] = {};
         for (u32 i = 0; i < per; ++i) {
             const u32 n = __shfl_sync(FULL, limit, i);
             const u32 xl = __shfl_sync(FULL, lo, i), xh = __shfl_sync(FULL, hi, i);
             u32 div = 0;
 #pragma unroll
             for (u32 g = 0; g < kSplitGroups; ++g) {
-                if (32 * g >= n) break;
+                if (kSplitSmall + 32 * g >= n) break;
                 // l | x iff x l^-1 mod 2^64 <= floor((2^64 - 1) / l); the high words
                 // alone let through 2^-32 of the others (k_dlog compares in full)
                 if (__umulhi(xl, inv_lo[g]) + xl * inv_hi[g] + xh * inv_lo[g] <= lim[g]) div |= 1u << g;
@@ -931,19 +1045,19 @@ __global__ void __launch_bounds__(256, 2) k_split(PrepArgs a, Counters* ctr) {
             while (bal) {                                      // one prime of each lane
                 const u32 src = (u32)__ffs((int)bal) - 1;
                 bal &= bal - 1;
-                const u32 k = 32 * ((u32)__ffs((int)__shfl_sync(FULL, div, src)) - 1) + src;
+                const u32 k = kSplitSmall + 32 * ((u32)__ffs((int)__shfl_sync(FULL, div, src)) - 1) + src;
 #pragma unroll
                 for (u32 c = 0; c < kSplitClasses; ++c)
                     if (lane == i && split_class(k) == c) found[c] = k + 1;
             }
         }
-        queue_events(ok, idx, found, a, ctr);
+        queue_events<0, kSplitClasses>(ok, idx, ok ? a.ent[idx].p : 0, found, a, ctr);
     }
 }
 
 // ---- k_dlog: the split events ----
 
-// n mod l for the entry's p: dlog of u = t^((p-1)/l) to w = b^((p-1)/l), or kEvUnknown / kEvReject.
+// n mod l for an entry's p: dlog of u = t^((p-1)/l) to w = b^((p-1)/l), or kEvUnknown / kEvReject.
 template <class F>
 __device__ __forceinline__ u32 split_solve(u64 p, const DevItem& it, u32 l, u64 l_inv) {
     typedef typename F::V V;
@@ -951,10 +1065,8 @@ __device__ __forceinline__ u32 split_solve(u64 p, const DevItem& it, u32 l, u64 
     f.init(p);
     const u64 e = (p - 1) * l_inv;                     // (p - 1) / l
     if (__umul64hi(e, l) != 0) return kEvUnknown;      // l does not divide p - 1 after all
-    const u64 bm = residue128(it.babs_hi, it.babs_lo, it.b_neg, p);
-    const u64 t = p - residue128(it.cabs_hi, it.cabs_lo, it.c_neg, p);
     V w, u;
-    pow_pair(f, f.from_u64(bm), f.from_u64(t), e, w, u);
+    f.powers(it, e, w, u);
     const V one = f.one();
     const bool u1 = f.eq(u, one);
     if (f.eq(w, one)) return u1 ? kEvUnknown : kEvReject;
@@ -964,60 +1076,88 @@ __device__ __forceinline__ u32 split_solve(u64 p, const DevItem& it, u32 l, u64 
 }
 
 __device__ __noinline__ u32 split_solve_m(u64 p, const DevItem& it, u32 l, u64 l_inv) {
-    return split_solve<FieldM>(p, it, l, l_inv);              // out of line: the FP64 path sets the registers
+    return split_solve<FieldM>(p, it, l, l_inv);       // out of line: the FP64 path sets the registers
 }
 
-// One lane per event, the classes of larger l first (longest walks first).
+// One lane per event, a list after the other, the longest walks first.
 __global__ void __launch_bounds__(256, 3) k_dlog(PrepArgs a, Counters* ctr) {
     const u32 lane = threadIdx.x & 31;
     const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
-    u64 units[kSplitClasses], total = 0;
+    constexpr u32 order[kSplitLists] = {8, 3, 7, 2, 6, 1, 5, 0, 9, 4};
+    static_assert(kSplitSizes == 5, "the lists' order");
+    u64 count[kSplitLists], total = 0;
 #pragma unroll
-    for (u32 c = 0; c < kSplitClasses; ++c) {
-        units[c] = (min((u64)*(volatile unsigned long long*)&ctr->events[c], a.ev_cap) + 31) / 32;
-        total += units[c];
+    for (u32 i = 0; i < kSplitLists; ++i) {
+        count[i] = min((u64)*(volatile unsigned long long*)&ctr->events[order[i]], a.ev_cap);
+        total += (count[i] + 31) / 32;
     }
-    for (u64 u = (u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < total; u += warps) {
-        u64 k = u;
-        u32 c = kSplitClasses - 1;
+    for (u64 unit = (u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; unit < total; unit += warps) {
+        u64 k = unit, idx = 0;
+        bool placed = false, live = false;
 #pragma unroll
-        for (u32 i = kSplitClasses - 1; i > 0; --i)
-            if (c == i && k >= units[i]) {
-                k -= units[i];
-                --c;
+        for (u32 i = 0; i < kSplitLists; ++i) {
+            const u64 units = (count[i] + 31) / 32;
+            if (!placed && k < units) {
+                idx = order[i] * a.ev_cap + k * 32 + lane;
+                live = k * 32 + lane < count[i];
+                placed = true;
             }
-        const u64 idx = k * 32 + lane;
-        if (idx >= min((u64)ctr->events[c], a.ev_cap)) continue;
-        const SplitEvent s = a.events[(u64)c * a.ev_cap + idx];
+            k -= units;
+        }
+        if (!live) continue;
+        const SplitEvent s = a.events[idx];
         Entry& e = a.ent[s.entry];
         const u64 p = e.p;
         const DevItem& it = a.items[e.item];
-        const u32 l = a.tables.sp[kSplitBase + s.k];
-        const u64 l_inv = a.tables.inv[kSplitBase + s.k];
-        const u32 x = p < kFp64Limit ? split_solve<FieldF>(p, it, l, l_inv) : split_solve_m(p, it, l, l_inv);
-        e.ev[c] = (s.k + 1) << 16 | x;
+        const u32 li = s.which >> 16, l = a.tables.sp[kSplitBase + li];
+        const u64 l_inv = a.tables.inv[kSplitBase + li], rcp = a.tables.rcp[kSplitBase + li];
+        u32 x = p < kFp64Limit ? split_solve<FieldF>(p, it, l, l_inv) : split_solve_m(p, it, l, l_inv);
+        if (x < kEvReject) {
+            // n_first + j L == x (mod l) for j; L is prime to l unless the class modulus holds l
+            const u32 Lm = mod_small(e.L, l, rcp), nm = mod_small(e.n_first, l, rcp);
+            if (Lm != 0) x = (x >= nm ? x - nm : x + l - nm) * inv_mod32(Lm, l) % l;
+            else x = x == nm ? kEvUnknown : kEvReject;
+        }
+        e.ev[s.which & 0xFFFFu] = (li + 1) << 16 | x;
     }
 }
 
 // ---- k_setup: the solve's set-up, and the solve of primes with few candidates ----
 
-// Applies what k_dlog found to the entry's candidates; false when none is left.
-__device__ __forceinline__ bool apply_events(Entry& e, const SieveTables& t) {
+// Applies what k_dlog found to the entry's candidates; false when none is
+// left.  ev: the entry's slots in memory, each lane taking its own next one (an
+// entry has 1.7 on average, so a loop over the slots would mostly idle).
+__device__ __forceinline__ bool apply_events(Entry& e, const u32* ev, const SieveTables& t) {
+    u32 mask = 0;
 #pragma unroll
-    for (u32 i = 0; i < kSplitClasses; ++i) {
-        const u32 x = e.ev[i] & 0xFFFFu;
-        if (e.ev[i] == 0 || x == kEvUnknown) continue;
+    for (u32 i = 0; i < kSplitSlots; ++i)
+        if (e.ev[i] != 0 && (e.ev[i] & 0xFFFFu) != kEvUnknown) mask |= 1u << i;
+    u64 j = 0, M = 1;                                  // the j left: == j (mod M)
+    while (mask) {
+        const u32 v = ev[__ffs((int)mask) - 1], x = v & 0xFFFFu;
+        mask &= mask - 1;
         if (x == kEvReject) return false;
-        // the j in [0, l) with n_first + j L == x (mod l); L is prime to l unless the class modulus holds l
-        const u32 l = t.sp[kSplitBase + (e.ev[i] >> 16) - 1];
-        const u32 Lm = (u32)(e.L % l), nm = (u32)(e.n_first % l);
-        if (Lm == 0) continue;
-        const u32 j0 = (x >= nm ? x - nm : x + l - nm) * inv_mod32(Lm, l) % l;
-        if (j0 >= e.jcount) return false;
-        e.n_first += (u64)j0 * e.L;
-        e.jcount = (e.jcount - j0 + l - 1) / l;
-        if (e.jcount > 1) e.L *= l;                    // L < N1 - N0 while two candidates are left
+        const u32 k = kSplitBase + (v >> 16) - 1, l = t.sp[k];
+        if (M == 1) {
+            j = x;
+            M = l;
+        } else {
+            const u64 rcp = t.rcp[k];
+            const u32 jm = mod_small(j, l, rcp);
+            const u32 diff = x >= jm ? x - jm : x + l - jm;
+            if (M >= e.jcount) {                       // one candidate at most: check it
+                if (diff) return false;
+            } else {
+                j += M * (diff * inv_mod32(mod_small(M, l, rcp), l) % l);
+                M *= l;
+            }
+        }
+        if (j >= e.jcount) return false;
     }
+    e.n_first += j * e.L;
+    const u32 left = e.jcount - (u32)j;                // >= 1
+    e.jcount = M >= left ? 1 : (left + (u32)M - 1) / (u32)M;
+    if (e.jcount > 1) e.L *= M;
     return true;
 }
 
@@ -1028,23 +1168,15 @@ __device__ __forceinline__ bool setup_entry(Entry& e, const DevItem& it, const P
     typedef typename F::V V;
     F f;
     f.init(e.p);
-    const u64 bm = residue128(it.babs_hi, it.babs_lo, it.b_neg, e.p);
     e.t = e.p - residue128(it.cabs_hi, it.cabs_lo, it.c_neg, e.p);
-    // G0 = b^n_first and B = b^L from one chain of squarings of b
-    V sq = f.from_u64(bm), gv = f.one(), Bv = f.one();
-    for (u64 e1 = e.n_first, e2 = e.jcount > 1 ? e.L : 0; e1 | e2;) {
-        if (e1 & 1) gv = f.mul(gv, sq);
-        if (e2 & 1) Bv = f.mul(Bv, sq);
-        e1 >>= 1;
-        e2 >>= 1;
-        if (e1 | e2) sq = f.mul(sq, sq);
-    }
+    const V gv = f.b_power(it, e.n_first);
     e.G0 = f.residue(gv);
     if (e.G0 == e.t) {                                 // j = 0
         emit_relation(e.p, e.n_first, 0, e.item, a.rel, a.rel_cap, ctr);
         return false;
     }
     if (e.jcount <= 1) return false;
+    const V Bv = f.b_power(it, e.L);
     e.B = f.residue(Bv);
     if (small) return true;
     u32 m = (u32)isqrt_ceil_dev(e.jcount);
@@ -1071,8 +1203,8 @@ __device__ __noinline__ u32 lane_solve_entry_m(const Entry& e) { return lane_sol
 // Entries with at most kLaneMax candidates are solved here, one lane each:
 // 1.6 lane instructions a candidate against about 490 warp instructions of
 // per-prime set-up in k_bsgs.  A warp's lanes walk together, so the entries
-// wait in queues by size (a factor of two each) until one holds 32.
-constexpr u32 kLaneQueues = 6, kLaneMax = 2048, kLaneMin = 64;   // J <= 64, 128, .. 2048
+// wait in queues by size (a factor of two each) and arithmetic until one holds 32.
+constexpr u32 kLaneSizes = 6, kLaneQueues = 2 * kLaneSizes, kLaneMax = 2048, kLaneMin = 64;   // J <= 64, 128, .. 2048
 constexpr u32 kLaneFew = 1u << 16, kLaneMaxFew = 256;            // (2^19 integers at 10^9: 248 us with 2048, 231 with 256)
 
 __global__ void __launch_bounds__(256, 3) k_setup(PrepArgs a, Counters* ctr) {
@@ -1129,7 +1261,7 @@ __global__ void __launch_bounds__(256, 3) k_setup(PrepArgs a, Counters* ctr) {
         if (first + lane < n_ent) {
             Entry e = a.ent[idx];
             const DevItem& it = a.items[e.item];
-            if (apply_events(e, a.tables)) {
+            if (apply_events(e, a.ent[idx].ev, a.tables)) {
                 const bool small = e.jcount <= lane_max;
                 if (e.p < kFp64Limit ? setup_entry<FieldF>(e, it, a, ctr, small)
                                      : setup_entry<FieldM>(e, it, a, ctr, small)) {
@@ -1140,6 +1272,7 @@ __global__ void __launch_bounds__(256, 3) k_setup(PrepArgs a, Counters* ctr) {
                     if (small) {
                         cls = 0;
                         while (e.jcount > (kLaneMin << cls)) ++cls;
+                        if (e.p >= kFp64Limit) cls += kLaneSizes;
                     }
                 }
             }

@@ -96,8 +96,9 @@ struct PrepArgs {
     const DevItem* items;
     Entry* ent;
     u64 ent_cap;               // < 2^32
-    SplitEvent* events;        // kSplitClasses lists of ev_cap events each
+    SplitEvent* events;        // kSplitLists lists of ev_cap events each
     u64 ev_cap;
+    u32 two_fields;            // 0: kSplitSizes lists only, shared by both arithmetics
     u32* big;                  // ent_cap indices: the entries k_bsgs solves
     RawRelation* rel;
     u64 rel_cap;
@@ -107,9 +108,10 @@ struct PrepArgs {
     u64 prime_below;           // survivors below this are prime (sieved by every prime up to their
                                // square root: 65521^2 for the sieve's survivors, 0 for caller-given numbers)
 };
-// Events a list needs for ent_cap entries: an entry has 0.3 in the fullest
-// class on average; a full list loses splits, never relations.
-constexpr u64 split_event_cap(u64 ent_cap) { return ent_cap / 2; }
+// Events a list needs for ent_cap entries (an entry has 0.7 small l on average,
+// and a chunk above 10^6 fills its entries to a third at most); a full list
+// loses splits, never relations.
+constexpr u64 split_event_cap(u64 ent_cap) { return ent_cap / 4; }
 // Split primes to look for in the range of an item with K in-class exponents.
 u32 split_primes_for(u64 K);
 constexpr u64 kSievedPrimeBelow = (u64)kSieveMaxPrime * kSieveMaxPrime;

@@ -42,7 +42,7 @@ namespace {
 constexpr u64 kNoAllocMaxSpan = 1ull << 19;
 constexpr u64 kNoAllocEntries = 3ull << 14;          // more than the 43,390 primes below 2^19, the most a range holds
 constexpr u64 kNoAllocSurv = kNoAllocEntries;        // (the same bound holds for the sieve's survivors)
-constexpr u64 kNoAllocEvents = kNoAllocEntries / 4;  // per split list (a full list loses splits, not relations)
+constexpr u64 kNoAllocEvents = 5ull << 12;           // per split list (a full list loses splits, not relations)
 constexpr u64 kNoAllocRelations = 1ull << 14;
 constexpr u32 kNoAllocMaxDevices = 64;
 
@@ -56,7 +56,7 @@ constexpr size_t kOffSurv = align256(kOffInv + kSievePrimes * sizeof(u64));
 constexpr size_t kOffSplit = align256(kOffSurv + kNoAllocSurv * sizeof(u64));
 constexpr size_t kOffEnt = align256(kOffSplit + kNoAllocSurv * sizeof(u64));
 constexpr size_t kOffEvents = align256(kOffEnt + kNoAllocEntries * sizeof(Entry));
-constexpr size_t kOffBig = align256(kOffEvents + kSplitClasses * kNoAllocEvents * sizeof(SplitEvent));
+constexpr size_t kOffBig = align256(kOffEvents + kSplitSizes * kNoAllocEvents * sizeof(SplitEvent));
 constexpr size_t kOffRel = align256(kOffBig + kNoAllocEntries * sizeof(u32));
 constexpr size_t kNoAllocUsed = align256(kOffRel + kNoAllocRelations * sizeof(RawRelation));
 constexpr size_t kNoAllocBytes = 8u << 20;
