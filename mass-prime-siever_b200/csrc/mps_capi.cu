@@ -433,6 +433,8 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     pa.full_mr = c->tun.full_mr;
     pa.m_cap = launch_m_cap(c, g, tbits);
     pa.m_round = g.lanes * g.chains;
+    pa.tbits = tbits;
+    pa.fill = g.fill;
     pa.prime_below = kSievedPrimeBelow;             // survivors of the sieve
 
     BsgsArgs ba{};
@@ -603,6 +605,8 @@ int slot_enqueue(mps_ctx* c, WaveSlot& w, u32 tbits, const LaunchCfg& g, bool ca
     pa.full_mr = c->tun.full_mr;
     pa.m_cap = launch_m_cap(c, g, tbits);
     pa.m_round = g.lanes * g.chains;
+    pa.tbits = tbits;
+    pa.fill = g.fill;
     pa.prime_below = kSievedPrimeBelow;             // survivors of the sieve
     BsgsArgs ba{};
     ba.ent = w.d_ent; ba.big = w.d_big; ba.ent_cap = w.ent_cap; ba.rel = w.d_rel; ba.rel_cap = w.rel_cap; ba.tbits = tbits;
@@ -1383,6 +1387,8 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
         pa.events = c->d_events; pa.ev_cap = split_event_cap(c->ent_cap); pa.two_fields = 1; pa.big = c->d_big;
         pa.m_cap = launch_m_cap(c, g, tbits);
         pa.m_round = g.lanes * g.chains;
+        pa.tbits = tbits;
+        pa.fill = g.fill;
         BsgsArgs ba{};
         ba.ent = c->d_ent; ba.big = c->d_big; ba.ent_cap = c->ent_cap; ba.rel = c->d_rel; ba.rel_cap = c->rel_cap;
         ba.tbits = tbits; ba.warps_per_block = warps; ba.persistent = 1; ba.chains = g.chains; ba.table_kind = g.kind;

@@ -87,8 +87,11 @@ struct Entry {
     u64 G0;               // b^n_first
     u64 B;                // b^L
     u64 Bm;               // B^m
+    double pinv;          // 1/p (p < 2^49)
     u32 jcount;           // <= 10^7 (the width of the N range)
     u32 m;                // baby steps (<= kMaxBaby)
+    u32 G;                // giant steps: ceil((jcount - 1) / m)
+    u32 tw;               // log2 of the fingerprint table's words
     u64 n_first;          // smallest candidate n
     u64 L;
     u32 item;             // item index (batched runs)

@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <cuda_fp16.h>
 #include <mutex>
 
 namespace mps {
@@ -369,6 +370,7 @@ struct FieldF {
     __device__ __forceinline__ u64 residue(V a) const { return f.residue(a); }   // any lazy value
     __device__ __forceinline__ V from_u64(u64 x) const { return (double)x; }
     __device__ __forceinline__ V one() const { return 1.0; }
+    __device__ __forceinline__ double reciprocal() const { return f.pinv; }
     __device__ __forceinline__ V dbl(V a) const { return __dadd_rn(a, a); }      // (-p, p) -> (-2p, 2p)
     __device__ __forceinline__ V pow(V b, u64 e) const { return f.pow(b, e); }
     __device__ __forceinline__ bool eq(V a, V c) const { return a == c || a == c - f.p; }   // a in (-p, p)
@@ -428,6 +430,7 @@ struct FieldM {
     __device__ __forceinline__ u64 residue(V a) const { return M.from_mont(a); }
     __device__ __forceinline__ V from_u64(u64 x) const { return M.to_mont(x, rr); }
     __device__ __forceinline__ V one() const { return M.one; }
+    __device__ __forceinline__ double reciprocal() const { return 0.0; }
     __device__ __forceinline__ V dbl(V a) const { return M.dbl(a); }
     __device__ __forceinline__ V pow(V b, u64 e) const { return M.pow(b, e); }
     __device__ __forceinline__ bool eq(V a, V c) const { return a == c || a == c + M.p; }   // a in [0, 2p)
@@ -441,6 +444,17 @@ struct FieldM {
 };
 
 // --------------------------------------------------------------- the prep --
+
+// log2 of the fingerprint-table words (the BSGS) a prime with m baby steps gets: at least m * 256 / fill
+// words (fill 1..256; 0 counts as 256) and at least 32, at most 2^(tbits-1).
+__device__ __forceinline__ u32 fq_words_log(u32 m, u32 fill, u32 tbits) {
+    const u32 f = fill - 1u < 256u ? fill : 256u;
+    const u32 keys = max(m, 2u) * 256u;                // m <= 4096: fits 32 bits
+    u32 t = 32u - __clz(max(m, 2u) - 1);               // 2^t >= m; 2^t f >= 256 m needs at most 8 more
+    while ((f << t) < keys) ++t;                       // no division: f << t <= 2^28
+    return min(tbits - 1, max(5u, t));
+}
+
 
 // p < 1000: the reference's direct BSGS over n in [0, m*m), m = ceil(sqrt(min(p, N1)))
 // (Math.hpp:488-542), which yields the smallest such n; a walk gives the same n.
@@ -682,9 +696,12 @@ __device__ __forceinline__ bool combine_class(u64 p, const DevItem& it, u32 d, u
 // k_setup (which took the set-up over from k_prep and solves the smallest
 // entries); BSGS steps 2.10e9 -> 0.90e9.
 
-// How many primes of the table an entry with J candidates is split by.
+// How many primes of the table an entry with J candidates is split by.  (The
+// optimum is flat: splitting from 512 candidates on, by all primes from 4096,
+// costs an item of K = 10^4 4% and one of K = 10^6 nothing; stopping at half as
+// many primes for each size loses as much.)
 __host__ __device__ constexpr u32 split_limit(u32 J) {
-    return J < 512 ? 0u : J < 1024 ? 64u : J < 4096 ? 170u : kSplitPrimes;
+    return J < 1536 ? 0u : J < 4096 ? 32u : J < 16384 ? 100u : J < 65536 ? 300u : kSplitPrimes;
 }
 u32 split_primes_for(u64 K) { return split_limit((u32)min(K, (u64)~0u)); }
 
@@ -1187,6 +1204,9 @@ __device__ __forceinline__ bool setup_entry(Entry& e, const DevItem& it, const P
     if (m > it.max_baby) m = it.max_baby;
     if (m > a.m_cap) m = a.m_cap;                      // never more than the launch's tables hold
     e.m = m;
+    e.G = (e.jcount - 1 + m - 1) / m;                  // g = 1..G covers j in [1, G*m]
+    e.tw = fq_words_log(m, a.fill, a.tbits);
+    e.pinv = f.reciprocal();
     e.Bm = f.residue(f.pow(Bv, m));
     return true;
 }
@@ -1267,6 +1287,7 @@ __global__ void __launch_bounds__(256, 3) k_setup(PrepArgs a, Counters* ctr) {
                                      : setup_entry<FieldM>(e, it, a, ctr, small)) {
                     Entry& d = a.ent[idx];
                     d.t = e.t; d.G0 = e.G0; d.B = e.B; d.Bm = e.Bm; d.jcount = e.jcount; d.m = e.m;
+                    d.pinv = e.pinv; d.G = e.G; d.tw = e.tw;
                     d.n_first = e.n_first; d.L = e.L;
                     cls = kLaneQueues;
                     if (small) {
@@ -1638,34 +1659,48 @@ __device__ u64 solve_fp64(const Solve& e, u32* tab, u32 tbits, u64* steps_out) {
 // filled in order (half k = bits 16k..16k+15): bit 15 of a half marks it
 // used, bits 0..13 hold a 14-bit fingerprint of the key; bit 14 of half 0 is
 // the word's overflow bit, set when a key homed at this word found it full
-// and moved on (linear probing over words).  The home word is the top tw bits
-// of the key's multiplicative hash h, the fingerprint the next 14 bits.  For
-// m baby steps tw = ceil(log2(m * 256 / fill)), so a word holds at most
-// fill/256 keys on average (fill 160: 0.6, and about 0.1% of the words
-// overflow).  A probe reads one word and tests the four halves at once
-// (fq_probe); a home with its overflow bit set also counts as a candidate.
-// The next giant value is multiplied before the probe of the current one, so
-// the multiply's latency overlaps the shared-memory load.  Candidates leave the
-// hot loop: the lane walks the overflow chain, and a fingerprint found is
-// resolved exactly by recomputation (ffind_baby).  Compared with one 32-bit
-// key per slot this stores 2.5x as many baby steps in the same shared memory
-// and never walks inside the hot loop.
+// and moved on (linear probing over words).  For m baby steps tw =
+// ceil(log2(m * 256 / fill)), so a word holds at most fill/256 keys on average
+// (fill 160: 0.6, and about 0.1% of the words overflow).
+//
+// The step is bound by instruction issue and the ALU pipe, with the FP64 pipe
+// a third busy, so its work sits where there is room.  The hash is one FP64
+// multiply-add of the canonical residue c (fq_hash): the low mantissa word of
+// c K + 2^51, 32 mixed bits of the fixed-point product.  Its bits 3 .. tw + 2
+// are the home word's byte offset as they stand and its bits 16 .. 29 the
+// fingerprint.  The four halves of a word are compared with the fingerprint as
+// half-precision numbers, two instructions of the FMA pipe: a used half is a
+// negative finite number (bit 14 clear), so equality is that of the bits, but
+// for fingerprint 0, -0, which an empty half also equals (one probe in 16,384).
+// A home with its overflow bit set also counts as a candidate.  The next giant
+// value is multiplied before the probe of the current one, so the multiply's
+// latency overlaps the shared-memory load.  Candidates leave the hot loop: the
+// lane walks the overflow chain, and a fingerprint found is resolved exactly by
+// recomputation (ffind_last).
+//
+// Measured on 2^27 integers of b = 10, c = 111 at 10^12: 1.61 -> 1.32 ms (the
+// hash, the half-precision compare and the cycle check left out: 1,358 -> 1,162 M
+// warp instructions; the set-up from k_setup and the half-warp scan: 1,100 M).
+// Per 32 steps a giant step is 27 instructions (9 FP64, 12 ALU), a baby step 36,
+// and a prime costs 290 besides.
+//
+// A cycle B^d == 1 with d < m needs no care: the baby steps then repeat, the
+// table holds some keys several times, and the largest i of the smallest g
+// still gives the smallest j = g m - i.
 
 constexpr u64 kQValid = 0x8000800080008000ull;
-
-// log2 of the words a prime with m baby steps gets: at least m * 256 / fill
-// words (fill 1..256; 0 counts as 256) and at least 32, at most 2^(tbits-1).
-__device__ __forceinline__ u32 fq_words_log(u32 m, u32 fill, u32 tbits, u32 extra_shift) {
-    const u32 f = fill - 1u < 256u ? fill : 256u;
-    const u32 keys = max(m, 2u) * 256u;                // m <= 4096: fits 32 bits
-    u32 t = 32u - __clz(max(m, 2u) - 1);               // 2^t >= m; 2^t f >= 256 m needs at most 8 more
-    while ((f << t) < keys) ++t;                       // no division: f << t <= 2^28
-    return min(tbits - 1, max(5u, t + extra_shift));
-}
 constexpr u32 kQOvf = 0x4000u;
 
-__device__ __forceinline__ u32 fq_pattern(u32 h, u32 tw) {
-    return ((h >> (18 - tw)) & 0x3FFFu) | 0x8000u;
+// c in [0, p), p < 2^49: c K < 2^50, so the sum lies in [2^51, 2^52), its unit
+// 1/2, whatever c: multiples of a power of two do not share their bits.
+__device__ __forceinline__ u32 fq_hash(double c) {
+    return (u32)__double2loint(__fma_rn(c, 1.6180339887498949, 2251799813685248.0));
+}
+__device__ __forceinline__ u32 fq_fingerprints(u32 h) {        // in both halves
+    return (__byte_perm(h, h, 0x3232) & 0x3FFF3FFFu) | 0x80008000u;
+}
+__device__ __forceinline__ u32 fq_equal_halves(u32 a, u32 b) {
+    return __heq2_mask(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
 }
 
 __device__ __forceinline__ bool fq_word_has(u64 w, u32 pat) {
@@ -1673,6 +1708,7 @@ __device__ __forceinline__ bool fq_word_has(u64 w, u32 pat) {
     return (lo & 0xFFFFu) == pat || (lo >> 16) == pat || (hi & 0xFFFFu) == pat || (hi >> 16) == pat;
 }
 
+// One compare-and-swap per key (table kind 0).
 __device__ __forceinline__ void fq_insert(unsigned long long* tab, u32 mask, u32 home, u32 pat) {
     volatile unsigned long long* vt = tab;
     u32 s = home;
@@ -1707,42 +1743,45 @@ __device__ __forceinline__ bool fq_contains(const unsigned long long* tab, u32 m
 }
 
 // Table kind 3: the fingerprint words of kind 0 with a count byte per word
-// (after the launch's words: one byte per eight of table).  Every chain's key
-// with want claims the next half of its home word by one shared-memory atomic
-// add on the word's count and writes its fingerprint with a plain 16-bit
-// store (every claimed half is distinct).  A claim that finds the word full
-// (count >= 4) is taken back at once, so a count rests at 4 at most and never
-// passes 4 + 32 * CH in flight (a byte cannot wrap).  The rare keys whose home
-// was full then walk on, word by word, in rounds of the whole warp, as in
-// kind 0's walk; the overflow bits of their homes are set after every store
-// of the call, so a store to half 0 never clears one.
-__device__ __forceinline__ u32 fq_claim(unsigned char* cnt, u32 s) {
-    const u32 sh = 8u * (s & 3u);
-    u32* c32 = reinterpret_cast<u32*>(cnt) + (s >> 2);
-    const u32 k = (atomicAdd(c32, 1u << sh) >> sh) & 0xFFu;
-    if (k >= 4u) atomicSub(c32, 1u << sh);          // full: take the claim back
-    return k;
+// (after the launch's words: one byte per eight of table).  A key claims the
+// next half of its home word by one shared-memory atomic add on the word's count
+// and writes its fingerprint with a plain 16-bit store (every claimed half is
+// distinct).  A claim that finds the word full (count >= 4) is taken back at
+// once, so a count rests at 4 at most and never passes 4 + 32 * CH in flight (a
+// byte cannot wrap).  The rare keys whose home was full then walk on, word by
+// word, in rounds of the whole warp, as in kind 0's walk; the overflow bits of
+// their homes are set after every store of the call, so a store to half 0
+// never clears one.  off: the word's byte offset.
+__device__ __forceinline__ u32 fq_claim(unsigned char* cnt, u32 off) {
+    const u32 sh = off & 24u;                          // 8 x (word mod 4)
+    u32* c32 = reinterpret_cast<u32*>(cnt) + (off >> 5);
+    return (atomicAdd(c32, 1u << sh) >> sh) & 0xFFu;
+}
+__device__ __forceinline__ void fq_unclaim(unsigned char* cnt, u32 off) {
+    atomicSub(reinterpret_cast<u32*>(cnt) + (off >> 5), 1u << (off & 24u));
 }
 
 template <int CH>
-__device__ __forceinline__ void fq_insert_count(unsigned long long* tab, unsigned char* cnt, u32 mask, u32 want,
-                                                const u32 (&home)[CH], const u32 (&pat)[CH]) {
-    unsigned short* t16 = reinterpret_cast<unsigned short*>(tab);
-    u32 k[CH];
+__device__ __forceinline__ void fq_insert_count(unsigned char* tab, unsigned char* cnt, u32 mask8, u32 want,
+                                                const u32 (&h)[CH]) {
+    u32 k[CH], pend = 0;                               // bit c: chain c found its home full
 #pragma unroll
-    for (int c = 0; c < CH; ++c) k[c] = (want >> c) & 1u ? fq_claim(cnt, home[c]) : 0u;
-    u32 pend = 0;                                      // bit c: chain c found its home full
+    for (int c = 0; c < CH; ++c) k[c] = (want >> c) & 1u ? fq_claim(cnt, h[c] & mask8) : 0u;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
         if (!((want >> c) & 1u)) continue;
-        if (k[c] < 4u) t16[4 * home[c] + k[c]] = (unsigned short)pat[c];
+        if (k[c] < 4u) *reinterpret_cast<unsigned short*>(tab + (h[c] & mask8) + 2 * k[c]) = (unsigned short)fq_fingerprints(h[c]);
         else pend |= 1u << c;
     }
     if (!__any_sync(FULL, pend)) return;
     const u32 ovf = pend;
     u32 s[CH];
 #pragma unroll
-    for (int c = 0; c < CH; ++c) s[c] = (home[c] + 1) & mask;
+    for (int c = 0; c < CH; ++c) {
+        s[c] = h[c] & mask8;
+        if ((pend >> c) & 1u) fq_unclaim(cnt, s[c]);
+        s[c] = (s[c] + 8) & mask8;
+    }
     while (__any_sync(FULL, pend)) {
 #pragma unroll
         for (int c = 0; c < CH; ++c) k[c] = (pend >> c) & 1u ? fq_claim(cnt, s[c]) : 4u;
@@ -1750,75 +1789,96 @@ __device__ __forceinline__ void fq_insert_count(unsigned long long* tab, unsigne
         for (int c = 0; c < CH; ++c) {
             if (!((pend >> c) & 1u)) continue;
             if (k[c] < 4u) {
-                t16[4 * s[c] + k[c]] = (unsigned short)pat[c];
+                *reinterpret_cast<unsigned short*>(tab + s[c] + 2 * k[c]) = (unsigned short)fq_fingerprints(h[c]);
                 pend &= ~(1u << c);
             } else {
-                s[c] = (s[c] + 1) & mask;
+                fq_unclaim(cnt, s[c]);
+                s[c] = (s[c] + 8) & mask8;
             }
         }
     }
     __syncwarp();
 #pragma unroll
     for (int c = 0; c < CH; ++c)
-        if ((ovf >> c) & 1u) atomicOr(reinterpret_cast<u32*>(tab) + 2 * home[c], kQOvf);
+        if ((ovf >> c) & 1u) atomicOr(reinterpret_cast<u32*>(tab + (h[c] & mask8)), kQOvf);
 }
 
-// The probe of a giant value: nonzero when a used half of the home word
-// equals the fingerprint, or the word overflowed.  With x = word ^ pattern
-// (both halves of the pattern), a 16-bit half of x is zero exactly when that
-// half matches, and (x - 0x00010001) & ~x & 0x80008000 is then nonzero.  The
-// caller ORs the probes of its chains and votes once per iteration.
-__device__ __forceinline__ u32 fq_probe(const uint2* t2, u32 h, u32 shift, u32 tw) {
-    const uint2 w = t2[h >> shift];
-    const u32 rep = fq_pattern(h, tw) * 0x10001u;
-    const u32 x0 = (w.x & ~kQOvf) ^ rep, x1 = w.y ^ rep;
-    return (((x0 - 0x10001u) & ~x0) & 0x80008000u) | (((x1 - 0x10001u) & ~x1) & 0x80008000u) | (w.x & kQOvf);
+// The largest i in [0, m) with t * B^i == v (canonical doubles compared
+// exactly); -1 when there is none.  Warp-cooperative: tbl = t * B^lane.
+__device__ __noinline__ int ffind_last(const Fp64& f, double tbl, double B32, u32 m, double v) {
+    const u32 lane = threadIdx.x & 31;
+    double x = tbl;
+    int last = -1;
+    for (u32 base = 0; base < m; base += 32) {
+        const u32 bal = __ballot_sync(FULL, base + lane < m && f.canon(x) == v);
+        if (bal) last = (int)(base + 31 - __clz((int)bal));
+        x = f.mul(x, B32);
+    }
+    return last;
+}
+
+// What the fingerprint-table solve needs of an entry, as k_setup left it.
+struct SolveF {
+    Fp64 f;                                            // p and 1/p
+    double t, G0, B, Bm;
+    u32 jcount, m, G, tw;
+};
+__device__ __forceinline__ SolveF solve_f(const Solve& e, u32 tbits, u32 fill) {
+    SolveF s;
+    s.f.init(e.p);
+    s.t = (double)e.t; s.G0 = (double)e.G0; s.B = (double)e.B; s.Bm = (double)e.Bm;
+    s.jcount = (u32)e.jcount;                          // <= 10^7
+    s.m = e.m;
+    s.G = (s.jcount - 1 + e.m - 1) / e.m;
+    s.tw = fq_words_log(e.m, fill, tbits);
+    return s;
 }
 
 // WI: baby steps inserted by fq_insert_count (table kind 3, count bytes
 // after the words) instead of one compare-and-swap each (table kind 0); the
-// words and the probes are the same.
+// words and the probes are the same.  The words are 2^tw of the launch's
+// 2^(tbits-1).
 template <int CH, bool WI>
-__device__ u64 solve_fp64q(const Solve& e, unsigned long long* tab, u32 tbits, u32 fill, u64* steps_out) {
-    const u32 lane = threadIdx.x & 31;
-    Fp64 f;
-    f.init(e.p);
-    const u32 m = e.m;
-    const u32 jc = (u32)e.jcount;                      // jcount <= 10^7
-    // 2^tw words for m keys (at most fill/256 per word), within the launch's 2^(tbits-1) words
-    const u32 tw = fq_words_log(m, fill, tbits, 0);
-    const u32 mask = (1u << tw) - 1, shift = 32 - tw;
-    const double B = (double)e.B, Bm = (double)e.Bm, tv = (double)e.t, G0 = (double)e.G0;
+__device__ u64 solve_fp64q(const SolveF& e, unsigned long long* tab, u32 tbits, u64* steps_out) {
+    const u32 lane = threadIdx.x & 31, lo = lane & 15;
+    const Fp64& f = e.f;
+    const u32 m = e.m, G = e.G;
+    const u32 mask = (1u << e.tw) - 1, mask8 = mask << 3;
 
-    double xb = B, xg = Bm;                            // B^(l+1), Bm^(l+1)
+    // the lanes' powers: lanes 0..15 scan to B^(lo+1), lanes 16..31 to Bm^(lo+1)
+    // in four steps; B^lane and Bm^(lane+1) are then one product away at most
+    double y = lane < 16 ? e.B : e.Bm;
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const double yb = __shfl_up_sync(FULL, xb, off), yg = __shfl_up_sync(FULL, xg, off);
-        if (lane >= (u32)off) {
-            xb = f.mul(xb, yb);
-            xg = f.mul(xg, yg);
-        }
+    for (int off = 1; off < 16; off <<= 1) {
+        const double z = __shfl_up_sync(FULL, y, off, 16);
+        if (lo >= (u32)off) y = f.mul(y, z);
     }
-    const double B32 = __shfl_sync(FULL, xb, 31), Bm32 = __shfl_sync(FULL, xg, 31);
-    double bl = __shfl_up_sync(FULL, xb, 1);
-    if (lane == 0) bl = 1.0;
+    const double B16 = __shfl_sync(FULL, y, 15), Bm16 = __shfl_sync(FULL, y, 31);
+    double bl = __shfl_sync(FULL, y, (int)((lo - 1) & 15)), gl = __shfl_sync(FULL, y, (int)(16 + lo));
+    if (lo == 0) bl = 1.0;
+    if (lane >= 16) {
+        bl = f.mul(bl, B16);
+        gl = f.mul(gl, Bm16);
+    }
+    const double B32 = f.mul(B16, B16), Bm32 = f.mul(Bm16, Bm16);
     double Bstep = B32, Gstep = Bm32;                  // B^(32 CH), Bm^(32 CH)
 #pragma unroll
     for (int c = 1; c < CH; c <<= 1) {
         Bstep = f.mul(Bstep, Bstep);
         Gstep = f.mul(Gstep, Gstep);
     }
-    const double tbl = f.mul(tv, bl);
+    const double tbl = f.mul(e.t, bl);
     double bx[CH], gx[CH];
     bx[0] = tbl;
-    gx[0] = f.mul(G0, xg);
+    gx[0] = f.mul(e.G0, gl);
 #pragma unroll
     for (int c = 1; c < CH; ++c) {
         bx[c] = f.mul(bx[c - 1], B32);
         gx[c] = f.mul(gx[c - 1], Bm32);
     }
 
-    unsigned char* cnt = reinterpret_cast<unsigned char*>(tab) + (4u << tbits);   // kind 3 only
+    unsigned char* bytes = reinterpret_cast<unsigned char*>(tab);
+    unsigned char* cnt = bytes + (4u << tbits);        // kind 3 only
     uint4* t4 = reinterpret_cast<uint4*>(tab);
 #pragma unroll 4
     for (u32 k = lane; k <= mask / 2; k += 32) t4[k] = make_uint4(0, 0, 0, 0);
@@ -1826,84 +1886,53 @@ __device__ u64 solve_fp64q(const Solve& e, unsigned long long* tab, u32 tbits, u
         for (u32 k = lane; k <= mask / 16; k += 32) reinterpret_cast<uint4*>(cnt)[k] = make_uint4(0, 0, 0, 0);
     __syncwarp();
 
-    // baby steps, stopping at a cycle B^d == 1 (d < m): t B^i == t for an
-    // i in [1, m) is looked for with one vote per iteration, and located
-    // exactly only when one is found
-    u32 cyc = 0, baby_done = m;
     for (u32 base = 0; base < m; base += 32 * CH) {
-        double cv[CH], nb[CH];
-        bool hit = false;
+        u32 h[CH], want = 0;
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
-            cv[c] = f.canon(bx[c]);
-            nb[c] = f.mul(bx[c], Bstep);                   // the next value, independent of the insert
-            hit |= base + 32 * c + lane - 1u < m - 1u && cv[c] == tv;
+            h[c] = fq_hash(f.canon(bx[c]));
+            bx[c] = f.mul(bx[c], Bstep);               // the next value, independent of the insert
+            if (base + 32 * c + lane < m) want |= 1u << c;
         }
-        u32 cb = 0;
-        if (__any_sync(FULL, hit)) {
-#pragma unroll
-            for (int c = 0; c < CH; ++c) {
-                const u32 bc = __ballot_sync(FULL, base + 32 * c + lane - 1u < m - 1u && cv[c] == tv);
-                if (bc && !cb) cb = base + 32 * c + __ffs(bc) - 1;
-            }
-        }
-        const u32 lim = cb ? cb : m;
         if (WI) {
-            u32 home[CH], pat[CH], want = 0;
-#pragma unroll
-            for (int c = 0; c < CH; ++c) {
-                const u32 h = fhash(cv[c]);
-                home[c] = h >> shift;
-                pat[c] = fq_pattern(h, tw);
-                if (base + 32 * c + lane < lim) want |= 1u << c;
-            }
-            fq_insert_count<CH>(tab, cnt, mask, want, home, pat);
+            // (whole iterations but for the last one: want is then a constant)
+            if (base + 32 * CH <= m) fq_insert_count<CH>(bytes, cnt, mask8, (1u << CH) - 1, h);
+            else fq_insert_count<CH>(bytes, cnt, mask8, want, h);
         } else {
 #pragma unroll
-            for (int c = 0; c < CH; ++c) {
-                const u32 h = fhash(cv[c]);
-                if (base + 32 * c + lane < lim) fq_insert(tab, mask, h >> shift, fq_pattern(h, tw));
-            }
+            for (int c = 0; c < CH; ++c)
+                if ((want >> c) & 1u) fq_insert(tab, mask, (h[c] & mask8) >> 3, fq_fingerprints(h[c]) & 0xFFFFu);
         }
-        if (cb) {
-            cyc = cb;
-            baby_done = cb;
-            break;
-        }
-#pragma unroll
-        for (int c = 0; c < CH; ++c) bx[c] = nb[c];
     }
     __syncwarp();
 
     u64 best = ~0ull;
-    u32 giant_done = 0;
-    if (cyc) {
-        const int i = ffind_baby(f, tbl, B32, 1, cyc, G0);
-        if (i > 0) best = cyc - (u32)i;
-    } else {
-        const u32 G = (jc - 1 + m - 1) / m;            // g = 1..G covers j in [1, G*m]
-        giant_done = G;
-        const uint2* t2 = reinterpret_cast<const uint2*>(tab);
-        for (u32 base = 0; base < G; base += 32 * CH) {
-            double cv[CH], nx[CH];
-            u32 hs[CH];
-            u32 z = 0;
+    u32 giant_done = G;                                // g = 1..G covers j in [1, G*m]
+    for (u32 base = 0; base < G; base += 32 * CH) {
+        double cv[CH], nx[CH];
+        u32 hs[CH];
+        u32 z = 0;
 #pragma unroll
-            for (int c = 0; c < CH; ++c) {
-                cv[c] = f.canon(gx[c]);
-                hs[c] = fhash(cv[c]);
-                nx[c] = f.mul(gx[c], Gstep);              // the next value, independent of the probe
-                z |= fq_probe(t2, hs[c], shift, tw);
-            }
-            if (__any_sync(FULL, z)) {
-                // the rare path: walk overflowed homes, then resolve exact matches in increasing g
-                u32 real = 0;
+        for (int c = 0; c < CH; ++c) {
+            cv[c] = f.canon(gx[c]);
+            hs[c] = fq_hash(cv[c]);
+            nx[c] = f.mul(gx[c], Gstep);                  // the next value, independent of the probe
+            const uint2 w = *reinterpret_cast<const uint2*>(bytes + (hs[c] & mask8));
+            const u32 rep = fq_fingerprints(hs[c]);
+            z |= fq_equal_halves(w.x, rep) | fq_equal_halves(w.y, rep) | (w.x & kQOvf);
+        }
+        if (__any_sync(FULL, z)) {
+            // the rare path: walk overflowed homes, then resolve exact matches in increasing g
+            u32 real = 0;
+            if (z) {
 #pragma unroll
                 for (int c = 0; c < CH; ++c)
-                    if (base + 32 * c + lane + 1 <= G && fq_probe(t2, hs[c], shift, tw) &&
-                        fq_contains(tab, mask, hs[c] >> shift, fq_pattern(hs[c], tw)))
+                    if (base + 32 * c + lane + 1 <= G &&
+                        fq_contains(tab, mask, (hs[c] & mask8) >> 3, fq_fingerprints(hs[c]) & 0xFFFFu))
                         real |= 1u << c;
-                u64 jb = ~0ull;
+            }
+            u64 jb = ~0ull;
+            if (__any_sync(FULL, real)) {
 #pragma unroll
                 for (int c = 0; c < CH; ++c) {
                     u32 bb = __ballot_sync(FULL, (real >> c) & 1u);
@@ -1912,22 +1941,22 @@ __device__ u64 solve_fp64q(const Solve& e, unsigned long long* tab, u32 tbits, u
                         bb &= bb - 1;
                         const double v = __shfl_sync(FULL, cv[c], src);
                         const u64 g = base + 32 * c + (u32)src + 1;
-                        const int i = ffind_baby(f, tbl, B32, 0, m, v);
+                        const int i = ffind_last(f, tbl, B32, m, v);
                         if (i >= 0) jb = g * m - (u64)i;
                     }
                 }
-                if (jb != ~0ull) {
-                    best = jb;
-                    giant_done = min(G, base + 32 * CH);
-                    break;
-                }
             }
-#pragma unroll
-            for (int c = 0; c < CH; ++c) gx[c] = nx[c];
+            if (jb != ~0ull) {
+                best = jb;
+                giant_done = min(G, base + 32 * CH);
+                break;
+            }
         }
+#pragma unroll
+        for (int c = 0; c < CH; ++c) gx[c] = nx[c];
     }
     __syncwarp();
-    if (steps_out) *steps_out = pack_steps(baby_done, giant_done);
+    if (steps_out) *steps_out = pack_steps(m, giant_done);
     return best < e.jcount ? best : ~0ull;
 }
 
@@ -2104,20 +2133,20 @@ __device__ u64 solve_fp64h(const Solve& e, unsigned short* tab, u32 tbits, u32 l
 template <int CH, int QT>
 __device__ __forceinline__ u64 solve_any(const Solve& e, void* tab, u32 tbits, u32 load_shift, u32 fill, u64* steps) {
     if (CH == 0 || e.p >= kFp64Limit) return solve_entry<FieldM>(e, (unsigned short*)tab, tbits + 1, steps);
-    if (QT == 0) return solve_fp64q<CH ? CH : 1, false>(e, (unsigned long long*)tab, tbits, fill, steps);
+    if (QT == 0) return solve_fp64q<CH ? CH : 1, false>(solve_f(e, tbits, fill), (unsigned long long*)tab, tbits, steps);
     if (QT == 2) return solve_fp64h<CH ? CH : 1>(e, (unsigned short*)tab, tbits, load_shift, steps);
-    if (QT == 3) return solve_fp64q<CH ? CH : 1, true>(e, (unsigned long long*)tab, tbits, fill, steps);
+    if (QT == 3) return solve_fp64q<CH ? CH : 1, true>(solve_f(e, tbits, fill), (unsigned long long*)tab, tbits, steps);
     return solve_fp64<CH ? CH : 1>(e, (u32*)tab, tbits, steps);
 }
 
 // Whether a prime's baby steps fit the table its solve will use (at most half
 // of its keys' room), so that every insertion finds a free slot.
 template <int CH, int QT>
-__device__ __forceinline__ bool fits_table(const Solve& e, u32 tbits) {
-    if (CH == 0 || e.p >= kFp64Limit) return e.m <= (1u << tbits);          // 2^(tbits+1) 16-bit slots
-    if (QT == 0 || QT == 3) return e.m <= (1u << tbits);                    // 2^(tbits-1) words of four
-    if (QT == 2) return e.m <= (1u << tbits);                               // 2^(tbits+1) 16-bit slots
-    return e.m < (1u << tbits);                                            // 2^tbits 32-bit slots
+__device__ __forceinline__ bool fits_table(u64 p, u32 m, u32 tbits) {
+    if (CH == 0 || p >= kFp64Limit) return m <= (1u << tbits);              // 2^(tbits+1) 16-bit slots
+    if (QT == 0 || QT == 3) return m <= (1u << tbits);                      // 2^(tbits-1) words of four
+    if (QT == 2) return m <= (1u << tbits);                                 // 2^(tbits+1) 16-bit slots
+    return m < (1u << tbits);                                              // 2^tbits 32-bit slots
 }
 
 __device__ __forceinline__ Solve solve_of(const Entry& g) {
@@ -2138,44 +2167,65 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counter
     const u64 n_ent = *(volatile unsigned long long*)&ctr->big;
     u64 my_steps = 0, my_baby = 0;
     if (a.persistent) {
-        // A warp claims the entry after the one it solves, and lanes 0..5 load
+        // A warp claims the entry after the one it solves, and lanes 0..7 load
         // that entry's words while the current one is solved, so neither the
-        // claim nor the load is waited for between entries.
-        static_assert(offsetof(Entry, jcount) == 40 && offsetof(Entry, m) == 44, "entry staging assumes p, t, G0, B, Bm, then jcount and m in one word");
+        // claim nor the load is waited for between entries.  What is the same
+        // for every lane of a solve (1/p, G, the table's width) comes from
+        // k_setup, a lane's work there instead of a warp's here, and the five
+        // residues are converted where they are staged, one lane each.
+        static_assert(offsetof(Entry, pinv) == 40 && offsetof(Entry, jcount) == 48 && offsetof(Entry, G) == 56,
+                      "entry staging assumes p, t, G0, B, Bm, 1/p, (jcount, m), (G, tw)");
         u64 cur = 0;
         if (lane == 0) cur = atomicAdd(&ctr->work_next, 1ull);
         cur = __shfl_sync(FULL, cur, 0);
         u64 claim = 0;                                          // lane 0: the entry after cur
         if (lane == 0 && cur < n_ent) claim = atomicAdd(&ctr->work_next, 1ull);
         u32 idx = cur < n_ent ? a.big[cur] : 0u;
-        u64 stage = cur < n_ent && lane < 6 ? reinterpret_cast<const u64*>(a.ent + idx)[lane] : 0;
+        u64 stage = cur < n_ent && lane < 8 ? reinterpret_cast<const u64*>(a.ent + idx)[lane] : 0;
         while (cur < n_ent) {
-            // the solve's fields; n_first, L and item are read again for a relation
-            Solve e;
-            e.p = __shfl_sync(FULL, stage, 0);
-            e.t = __shfl_sync(FULL, stage, 1);
-            e.G0 = __shfl_sync(FULL, stage, 2);
-            e.B = __shfl_sync(FULL, stage, 3);
-            e.Bm = __shfl_sync(FULL, stage, 4);
-            const u64 jm = __shfl_sync(FULL, stage, 5);         // little-endian: jcount, then m
-            e.jcount = (u32)jm;
-            e.m = (u32)(jm >> 32);
-            const u32 this_idx = idx;
+            const u64 mine = stage, p = __shfl_sync(FULL, mine, 0);
+            const u64 jm = __shfl_sync(FULL, mine, 6), gt = __shfl_sync(FULL, mine, 7);   // little-endian pairs
+            const u32 this_idx = idx, m = (u32)(jm >> 32);
             const u64 next = __shfl_sync(FULL, claim, 0);
             idx = next < n_ent ? a.big[next] : 0u;
-            stage = next < n_ent && lane < 6 ? reinterpret_cast<const u64*>(a.ent + idx)[lane] : 0;
+            stage = next < n_ent && lane < 8 ? reinterpret_cast<const u64*>(a.ent + idx)[lane] : 0;
             if (lane == 0 && next < n_ent) claim = atomicAdd(&ctr->work_next, 1ull);
             cur = next;
-            if (!fits_table<CH, QT>(e, a.tbits)) {              // host sizing error: never overfill a table
+            if (!fits_table<CH, QT>(p, m, a.tbits)) {           // host sizing error: never overfill a table
                 if (lane == 0) atomicOr(&ctr->status, kStatusBadLaunch);
                 continue;
             }
-            u64 steps = 0;
-            const u64 j = solve_any<CH, QT>(e, tab, a.tbits, a.load_shift, a.fill, &steps);
+            u64 steps = 0, j;
+            if (CH > 0 && (QT == 0 || QT == 3) && p < kFp64Limit) {
+                const double v = lane < 5 ? (double)mine : __longlong_as_double((long long)mine);
+                SolveF e;
+                e.f.p = __shfl_sync(FULL, v, 0);
+                e.t = __shfl_sync(FULL, v, 1);
+                e.G0 = __shfl_sync(FULL, v, 2);
+                e.B = __shfl_sync(FULL, v, 3);
+                e.Bm = __shfl_sync(FULL, v, 4);
+                e.f.pinv = __shfl_sync(FULL, v, 5);
+                e.f.pi = p;
+                e.jcount = (u32)jm;
+                e.m = m;
+                e.G = (u32)gt;
+                e.tw = min((u32)(gt >> 32), a.tbits - 1);
+                j = solve_fp64q<CH ? CH : 1, QT == 3>(e, (unsigned long long*)tab, a.tbits, &steps);
+            } else {
+                Solve e;
+                e.p = p;
+                e.t = __shfl_sync(FULL, mine, 1);
+                e.G0 = __shfl_sync(FULL, mine, 2);
+                e.B = __shfl_sync(FULL, mine, 3);
+                e.Bm = __shfl_sync(FULL, mine, 4);
+                e.jcount = (u32)jm;
+                e.m = m;
+                j = solve_any<CH, QT>(e, tab, a.tbits, a.load_shift, a.fill, &steps);
+            }
             if (lane == 0) {
                 if (j != ~0ull) {
                     const Entry& g = a.ent[this_idx];
-                    emit_relation(e.p, g.n_first + j * g.L, 0, g.item, a.rel, a.rel_cap, ctr);
+                    emit_relation(g.p, g.n_first + j * g.L, 0, g.item, a.rel, a.rel_cap, ctr);
                 }
                 my_steps += (steps & 0xFFFFFFFFull) + (steps >> 32);
                 my_baby += steps & 0xFFFFFFFFull;
@@ -2190,7 +2240,7 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counter
         if (k >= n_ent) return;
         const Entry& g = a.ent[a.big[k]];
         const Solve e = solve_of(g);
-        if (!fits_table<CH, QT>(e, a.tbits)) {
+        if (!fits_table<CH, QT>(e.p, e.m, a.tbits)) {
             if (lane == 0) atomicOr(&ctr->status, kStatusBadLaunch);
             return;
         }

@@ -40,7 +40,7 @@ namespace {
 
 // Largest range one call takes: 2^19 integers (2^18 odd numbers).
 constexpr u64 kNoAllocMaxSpan = 1ull << 19;
-constexpr u64 kNoAllocEntries = 3ull << 14;          // more than the 43,390 primes below 2^19, the most a range holds
+constexpr u64 kNoAllocEntries = 11ull << 12;         // more than the 43,390 primes below 2^19, the most a range holds
 constexpr u64 kNoAllocSurv = kNoAllocEntries;        // (the same bound holds for the sieve's survivors)
 constexpr u64 kNoAllocEvents = 5ull << 12;           // per split list (a full list loses splits, not relations)
 constexpr u64 kNoAllocRelations = 1ull << 14;
@@ -194,6 +194,8 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     pa.rel_cap = kNoAllocRelations;
     pa.m_cap = std::min<u32>(noalloc_holds(tbits), kMaxBaby);
     pa.m_round = 64;                                         // one warp, two chains
+    pa.tbits = tbits;
+    pa.fill = kDefaultFill;
     pa.prime_below = kSievedPrimeBelow;                      // survivors of the sieve
     BsgsArgs ba{};
     ba.ent = ent;
