@@ -95,12 +95,16 @@ struct Entry {
     u64 n_first;          // smallest candidate n
     u64 L;
     u32 item;             // item index (batched runs)
-    u32 ev[kSplitSlots];     // 0: none, else l's index + 1 << 16 | what k_dlog found (kEv*)
     u32 pad;
+    unsigned short k[kSplitClasses];   // the index of the l in each class's slot (a small l's is its slot - kSplitClasses)
+    u32 ev[kSplitSlots];  // 0: no l in this slot, else what is known of j mod l (kEv*)
 };
-constexpr u32 kEvUnknown = 0xFFFFu;   // nothing learned: b is an l-th power residue and so is t
-constexpr u32 kEvReject = 0xFFFEu;    // no n solves it: b is an l-th power residue and t is not
-                                      // (anything else: j == this (mod l))
+constexpr u32 kEvQueued = 1u << 31;   // an l is in the slot
+constexpr u32 kEvValue = 0x1FFFu;     // j mod l, or one of
+constexpr u32 kEvUnknown = 0x1FFFu;   //   nothing learned: b is an l-th power residue and so is t
+constexpr u32 kEvReject = 0x1FFEu;    //   no n solves it: b is an l-th power residue and t is not
+constexpr u32 kEvInvShift = 13;       // above it: the inverse mod l of the product of the earlier slots' primes
+__host__ __device__ constexpr u32 slot_small(u32 slot) { return slot - kSplitClasses; }
 
 // A prime l | p - 1 of an entry, queued for k_dlog.
 struct SplitEvent {
@@ -136,6 +140,7 @@ struct Counters {
     unsigned long long baby;       u64 pad8[7];   // the baby steps among `steps`
     unsigned long long events[kSplitLists]; u64 pad9[16 - kSplitLists];   // split events queued, by list
     unsigned long long setup_next; u64 pad10[7];  // next entry the set-up's warps claim
+    unsigned long long dlog_next;  u64 pad12[7];  // next unit of 32 events k_dlog's warps claim
     unsigned long long big;        u64 pad11[7];  // entries left for a warp each (k_bsgs)
 };
 

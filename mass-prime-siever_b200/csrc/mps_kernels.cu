@@ -285,6 +285,7 @@ __device__ void sieve_segment(SieveShared<W>& sh, u64 v0, u32 len, u32 n_primes,
     }
     __syncthreads();
 }
+static_assert(offsetof(Entry, k) % 8 == 0, "k_dlog reads the classes' indices as one word");
 static_assert(kSplitClasses == 4 && split_class(kSplitShared - 1) == 2 && split_class(kSplitShared) == 3, "a survivor's split primes fill one 64-bit word");
 
 template <u32 W>
@@ -383,12 +384,17 @@ struct FieldF {
     // (the first one, s itself, is below p, and its square below 3/4 p, then
     // 0.65 p).  About 10 issue slots a bit against 16 for square-and-multiply.
     __device__ __forceinline__ bool small(double s) const { return s != 0.0 && fabs(s) * f.p <= 1125899906842624.0 && fabs(s) < f.p; }
+    // (A small s has no bits in its low word: the factor s^bit is one select.)
+    __device__ __forceinline__ static double factor(bool bit, int s_hi) { return __hiloint2double(bit ? s_hi : 0x3FF00000, 0); }
     __device__ __forceinline__ V pow_small(double s, u64 e) const {
         if (e == 0) return 1.0;
+        const int lead = __clzll((long long)e), hi = __double2hiint(s);
         double x = s;
-        for (int k = 62 - __clzll((long long)e); k >= 0; --k) {
-            const double y = (e >> k) & 1 ? __dmul_rn(x, s) : x;
-            x = f.mul(y, x);
+        e <<= lead;
+        for (int k = 63 - lead; k > 0; --k) {
+            e <<= 1;
+            const bool bit = (long long)e < 0;
+            x = f.mul(__dmul_rn(x, factor(bit, hi)), x);
         }
         return x;
     }
@@ -396,13 +402,15 @@ struct FieldF {
     __device__ __forceinline__ void powers(const DevItem& it, u64 e, V& w, V& u) const {
         const double bs = it.b_small, ts = it.t_small;
         if (small(bs) && small(ts)) {
+            const int lead = __clzll((long long)e), bh = __double2hiint(bs), th = __double2hiint(ts);
             w = bs;
             u = ts;
-            for (int k = 62 - __clzll((long long)e); k >= 0; --k) {
-                const bool bit = (e >> k) & 1;
-                const double y = bit ? __dmul_rn(w, bs) : w, z = bit ? __dmul_rn(u, ts) : u;
-                w = f.mul(y, w);
-                u = f.mul(z, u);
+            e <<= lead;
+            for (int k = 63 - lead; k > 0; --k) {
+                e <<= 1;
+                const bool bit = (long long)e < 0;
+                w = f.mul(__dmul_rn(w, factor(bit, bh)), w);
+                u = f.mul(__dmul_rn(u, factor(bit, th)), u);
             }
             return;
         }
@@ -458,7 +466,7 @@ __device__ __forceinline__ u32 fq_words_log(u32 m, u32 fill, u32 tbits) {
 
 // p < 1000: the reference's direct BSGS over n in [0, m*m), m = ceil(sqrt(min(p, N1)))
 // (Math.hpp:488-542), which yields the smallest such n; a walk gives the same n.
-__device__ void small_prime(u64 p, u64 b_mod, u64 t, const DevItem& it, const PrepArgs& a, Counters* ctr) {
+__device__ __noinline__ void small_prime(u64 p, u64 b_mod, u64 t, const DevItem& it, const PrepArgs& a, Counters* ctr) {
     const i64 lim = ((i64)p > it.N1_raw) ? it.N1_raw : (i64)p;
     if (lim <= 0) return;
     const u64 m = isqrt_ceil_dev((u64)lim);
@@ -525,8 +533,12 @@ __device__ __forceinline__ bool prep_special(u64 p, const DevItem& it, const Pre
 // symbols of 32-bit numbers, before any modular exponentiation.
 __device__ __forceinline__ bool qr_reject(u64 p, const DevItem& it) {
     if (!it.qr_on) return false;
-    const int jb = jacobi_small(p, it.qr_neg[0], it.qr_k[0], it.qr_o[0], it.qr_rcp[0]);
-    const int jt = jacobi_small(p, it.qr_neg[1], it.qr_k[1], it.qr_o[1], it.qr_rcp[1]);
+    int jb = 0, jt = 0;
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) {                      // (one copy of the code)
+        jb = jt;
+        jt = jacobi_small(p, it.qr_neg[i], it.qr_k[i], it.qr_o[i], it.qr_rcp[i]);
+    }
     if (jb == 0 || jt == 0) return false;              // p shares a factor with b or c: the exact path decides
     if ((it.cm & 1) == 0) return (it.n_start & 1) ? jb != jt : jt != 1;
     return jb == 1 && jt != 1;
@@ -734,7 +746,8 @@ __device__ __forceinline__ void queue_events(bool ok, u64 idx, u64 p, const u32 
         if (!ok) continue;
         const bool in = k[s] != 0 && at < a.ev_cap;
         if (in) a.events[c * a.ev_cap + at] = SplitEvent{(u32)idx, (k[s] - 1) << 16 | s};
-        a.ent[idx].ev[s] = in ? k[s] << 16 | kEvUnknown : 0u;
+        a.ent[idx].ev[s] = in ? kEvQueued | kEvUnknown : 0u;
+        if (s < kSplitClasses) a.ent[idx].k[s] = (unsigned short)(k[s] - 1);
     }
 }
 
@@ -747,51 +760,177 @@ __device__ __forceinline__ bool divides(u64 x) {
     return x * inv <= ~0ull / L;
 }
 
-// The smallest j in [1, J) with G0 * B^j == t, by one lane (~0: none): kLaneBaby
-// baby steps t * B^i whose low words stay in registers, giant steps G0 *
-// B^(kLaneBaby g) compared with all of them (a compare is one instruction, a
-// product six on the FP64 pipe), a low word that matches resolved exactly.  t canonical.
-constexpr u32 kLaneBaby = 16;
+// Two 16-bit halves of a compared with those of b as half-precision numbers
+// (two FMA-pipe compares in one instruction): 0xFFFF where equal.
+__device__ __forceinline__ u32 equal_halves(u32 a, u32 b) {
+    return __heq2_mask(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+}
+
+// The largest i < M with t * B^i == g as base + M - i, ~0 when there is none.
+template <u32 M, class F>
+__device__ __forceinline__ u32 lane_match(const F& f, typename F::V t, typename F::V B, typename F::V g, u32 base) {
+    const typename F::V c = f.canon(g);
+    typename F::V x = t;
+    u32 best = ~0u;
+#pragma unroll 4
+    for (u32 i = 0; i < M; ++i) {
+        if (f.canon(x) == c) best = base + M - i;
+        x = f.mul(x, B);
+    }
+    return best;
+}
+
+// The smallest j in [1, J) with G0 * B^j == t, by one lane (~0: none): M baby
+// steps t * B^i, giant steps G0 * B^(M g) each compared with all of them, a
+// match resolved exactly after the loop.  t canonical.  The lanes leave the loop
+// at different times and are brought together by __syncwarp before the
+// resolution; without it each group that leaves runs the resolution on its own
+// (k_dlog: 0.58 ms instead of 0.29 on 2^27 integers at 10^12).
+//   16 baby steps (small J): their low words in registers, a compare each; the
+//     walk ends at the first match (a wrong one, 2^-28, goes on from there).
+//   32 baby steps: the low 14 bits and bit 15 of their low words, two to a
+//     register, as finite half-precision numbers, so that a giant step costs 16
+//     FMA-pipe compares and 8 ORs where 32 integer compares would take twice the
+//     ALU's time.  One giant step in 1,000 matches by chance: the walk goes on,
+//     keeping the last two matches (a third one has the first resolved at once).
 template <class F>
-__device__ u32 lane_solve(const F& f, typename F::V t, typename F::V G0, typename F::V B, u32 J) {
+__device__ __noinline__ u32 lane_rest(F f, typename F::V t, typename F::V B, typename F::V S, typename F::V g,
+                                      u32 base, u32 M, u32 J) {
+    for (; base + 1 < J; base += M) {                  // every giant step resolved in full
+        const typename F::V c = f.canon(g);
+        typename F::V x = t;
+        u32 best = ~0u;
+        for (u32 i = 0; i < M; ++i) {
+            if (f.canon(x) == c) best = base + M - i;
+            x = f.mul(x, B);
+        }
+        if (best != ~0u) return best < J ? best : ~0u;
+        g = f.mul(g, S);
+    }
+    return ~0u;
+}
+
+template <class F>
+__device__ __forceinline__ u32 lane_match32(F f, typename F::V t, typename F::V B, typename F::V g, u32 base) {
+    return lane_match<32>(f, t, B, g, base);
+}
+
+template <class F>
+__device__ __forceinline__ u32 lane_solve16(const F& f, typename F::V t, typename F::V G0, typename F::V B, u32 J) {
     typedef typename F::V V;
-    u32 key[kLaneBaby];
+    constexpr u32 M = 16;
+    const u32 together = __activemask();
+    u32 key[M];
     V x = t;
 #pragma unroll
-    for (u32 i = 0; i < kLaneBaby; ++i) {
+    for (u32 i = 0; i < M; ++i) {
         key[i] = f.key32(x);
         x = f.mul(x, B);
     }
     V S = f.mul(B, B);
 #pragma unroll
-    for (u32 i = 2; i < kLaneBaby; i <<= 1) S = f.mul(S, S);
+    for (u32 i = 2; i < M; i <<= 1) S = f.mul(S, S);
     V g = f.mul(G0, S);
-    for (u32 base = 0; base + 1 < J; base += kLaneBaby) {   // g = G0 B^(base + kLaneBaby): j in (base, base + kLaneBaby]
+    u32 base = 0;
+    bool hit = false;
+    for (; base + 1 < J; base += M) {                  // g = G0 B^(base + M): j in (base, base + M]
         const u32 k = f.key32(g);
         const V next = f.mul(g, S);
-        bool hit = false;
 #pragma unroll
-        for (u32 i = 0; i < kLaneBaby; ++i) hit |= key[i] == k;
-        if (hit) {
-            const V c = f.canon(g);
-            u32 best = ~0u;
-            x = t;
-            for (u32 i = 0; i < kLaneBaby; ++i) {           // the last i is the smallest j
-                if (f.canon(x) == c) best = base + kLaneBaby - i;
-                x = f.mul(x, B);
+        for (u32 i = 0; i < M; ++i) hit |= key[i] == k;
+        if (hit) break;
+        g = next;
+    }
+    __syncwarp(together);
+    u32 best = ~0u;
+    if (hit) {
+        best = lane_match<M>(f, t, B, g, base);
+        if (best == ~0u) best = lane_rest(f, t, B, S, f.mul(g, S), base + M, M, J);
+    }
+    return best < J ? best : ~0u;
+}
+
+template <class F>
+__device__ __forceinline__ u32 lane_solve32(const F& f, typename F::V t, typename F::V G0, typename F::V B, u32 J) {
+    typedef typename F::V V;
+    constexpr u32 M = 32;
+    const u32 together = __activemask();
+    u32 key[M / 2];
+    V x = t;
+#pragma unroll
+    for (u32 i = 0; i < M; i += 2) {
+        const u32 k0 = f.key32(x);
+        x = f.mul(x, B);
+        const u32 k1 = f.key32(x);
+        x = f.mul(x, B);
+        key[i / 2] = __byte_perm(k0, k1, 0x5410) & 0xBFFFBFFFu;
+    }
+    V S = f.mul(B, B);
+#pragma unroll
+    for (u32 i = 2; i < M; i <<= 1) S = f.mul(S, S);
+    V g = f.mul(G0, S), g0 = g, g1 = g;
+    u32 n = 0, b0 = 0, b1 = 0, best = ~0u;
+    for (u32 base = 0; base + 1 < J; base += M) {      // g = G0 B^(base + M): j in (base, base + M]
+        const u32 k = f.key32(g), rep = __byte_perm(k, k, 0x1010) & 0xBFFFBFFFu;
+        const V next = f.mul(g, S);
+        u32 z = 0;
+#pragma unroll
+        for (u32 i = 0; i < M / 2; ++i) z |= equal_halves(key[i], rep);
+        if (z) {
+            if (n == 2) {
+                best = lane_match32(f, t, B, g0, b0);
+                if (best != ~0u) break;
+                g0 = g1;
+                b0 = b1;
+                n = 1;
             }
-            if (best != ~0u) return best < J ? best : ~0u;
+            if (n == 0) {
+                g0 = g;
+                b0 = base;
+            } else {
+                g1 = g;
+                b1 = base;
+            }
+            ++n;
         }
         g = next;
     }
-    return ~0u;
+    __syncwarp(together);
+    if (best == ~0u && n > 0) best = lane_match32(f, t, B, g0, b0);
+    if (best == ~0u && n > 1) best = lane_match32(f, t, B, g1, b1);
+    return best < J ? best : ~0u;
 }
+
+// a^-1 mod m for gcd(a, m) = 1, 0 < a < m < 2^13: extended Euclid with the
+// quotients by single-precision division, off by one at most and set right.  (At
+// most 18 steps: the remainders fall as fast as Fibonacci numbers.)
+__device__ __forceinline__ u32 inv_mod_small(u32 a, u32 m) {
+    int r0 = (int)m, r1 = (int)a, s0 = 0, s1 = 1;
+    for (int step = 0; step < 20 && r1 > 0; ++step) {
+        int q = (int)__fdividef((float)r0, (float)r1);
+        int r2 = r0 - q * r1;
+        if (r2 < 0) {
+            --q;
+            r2 += r1;
+        } else if (r2 >= r1) {
+            ++q;
+            r2 -= r1;
+        }
+        const int s2 = s0 - q * s1;
+        r0 = r1;
+        r1 = r2;
+        s0 = s1;
+        s1 = s2;
+    }
+    const int x = s0 % (int)m;
+    return (u32)(x < 0 ? x + (int)m : x);
+}
+
 
 // What stage 1 tests of primality itself: a base-2 strong test where the powers
 // of b prove nothing (|b| <= 1), all 12 bases when the caller asks for them.
 template <class F>
-__device__ __forceinline__ bool stage1(u64 p, const DevItem& it, const PrepArgs& a) {
-    if (p < a.prime_below) return true;                // the sieve removed every composite below this
+__device__ __forceinline__ bool stage1_in(u64 p, const DevItem& it, const PrepArgs& a) {
     if (it.strong) {
         F f;
         f.init(p);
@@ -851,11 +990,24 @@ __device__ __forceinline__ int split_in(const DevItem& it, u64 p, u32& d, u32& r
     return power_split(f, p, it, kWalk, d, r, w, u);
 }
 
-template <class F>
-__device__ __forceinline__ bool split_pp_in(const DevItem& it, u64 p, u64 w, u64 u, u32& d, u32& r) {
-    F f;
+// The rare paths are out of line: with everything inline the kernel's warps, each
+// at another stage, waited for instruction fetches more than for anything else
+// but their own arithmetic (2.25 stalls an issue).
+__device__ __noinline__ int split_in_m(const DevItem& it, u64 p, u32& d, u32& r, u64& w, u64& u) {
+    return split_in<FieldM>(it, p, d, r, w, u);
+}
+__device__ __noinline__ bool split_pp_in(const DevItem& it, u64 p, u64 w, u64 u, u32& d, u32& r) {
+    if (p < kFp64Limit) {
+        FieldF f;
+        f.init(p);
+        return power_split_pp(f, p, w, u, it, d, r);
+    }
+    FieldM f;
     f.init(p);
     return power_split_pp(f, p, w, u, it, d, r);
+}
+__device__ __noinline__ bool stage1(u64 p, const DevItem& it, const PrepArgs& a) {
+    return p < kFp64Limit ? stage1_in<FieldF>(p, it, a) : stage1_in<FieldM>(p, it, a);
 }
 
 __global__ void __launch_bounds__(kPrepThreads, 4) k_prep(PrepArgs a, Counters* ctr) {
@@ -934,7 +1086,7 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep(PrepArgs a, Counters* 
                 sv = Q.sd[k];
                 const DevItem& it = a.items[item];
                 const u64 w = Q.wd[k], u = Q.ud[k];
-                ok = p < kFp64Limit ? split_pp_in<FieldF>(it, p, w, u, d, r) : split_pp_in<FieldM>(it, p, w, u, d, r);
+                ok = split_pp_in(it, p, w, u, d, r);
             }
             nd -= cnt;
             __syncwarp();
@@ -962,7 +1114,7 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep(PrepArgs a, Counters* 
                 item = Q.i1[k];
                 sv = Q.s1[k];
                 const DevItem& it = a.items[item];
-                res = p < kFp64Limit ? split_in<FieldF>(it, p, d, r, w, u) : split_in<FieldM>(it, p, d, r, w, u);
+                res = p < kFp64Limit ? split_in<FieldF>(it, p, d, r, w, u) : split_in_m(it, p, d, r, w, u);
             }
             n1 -= cnt;
             __syncwarp();
@@ -1003,7 +1155,8 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep(PrepArgs a, Counters* 
             if (a.surv_item) item = a.surv_item[k];
             u64 bm, t;
             if (prep_special(p, a.items[item], a, ctr, bm, t) && !qr_reject(p, a.items[item]))
-                keep = p < kFp64Limit ? stage1<FieldF>(p, a.items[item], a) : stage1<FieldM>(p, a.items[item], a);
+                // (below prime_below the sieve removed every composite)
+                keep = p < a.prime_below || !(a.items[item].strong || a.full_mr) || stage1(p, a.items[item], a);
         }
         u32 s1;
         qpush(keep, n1, &s1);
@@ -1074,32 +1227,35 @@ __global__ void __launch_bounds__(256, 2) k_split(PrepArgs a, Counters* ctr) {
 
 // ---- k_dlog: the split events ----
 
-// n mod l for an entry's p: dlog of u = t^((p-1)/l) to w = b^((p-1)/l), or kEvUnknown / kEvReject.
+// n mod l for an entry's p: dlog of u = t^((p-1)/l) to w = b^((p-1)/l), or
+// kEvUnknown / kEvReject.  together: the lanes that call this; they are brought
+// together after the powers, whose lengths differ.
 template <class F>
-__device__ __forceinline__ u32 split_solve(u64 p, const DevItem& it, u32 l, u64 l_inv) {
+__device__ __forceinline__ u32 split_solve(u64 p, const DevItem& it, u32 l, u64 l_inv, bool large, u32 together) {
     typedef typename F::V V;
     F f;
     f.init(p);
-    const u64 e = (p - 1) * l_inv;                     // (p - 1) / l
-    if (__umul64hi(e, l) != 0) return kEvUnknown;      // l does not divide p - 1 after all
+    const u64 e = (p - 1) * l_inv;                     // (p - 1) / l, if l divides p - 1 at all
     V w, u;
     f.powers(it, e, w, u);
+    __syncwarp(together);
     const V one = f.one();
-    const bool u1 = f.eq(u, one);
-    if (f.eq(w, one)) return u1 ? kEvUnknown : kEvReject;
-    if (u1) return 0;
-    const u32 x = lane_solve(f, f.canon(u), one, w, l);
-    return x == ~0u ? kEvUnknown : x;                  // (~0: p is not prime; the order stage drops it)
+    const bool w1 = f.eq(w, one), u1 = f.eq(u, one);
+    u32 x = w1 ? (u1 ? kEvUnknown : kEvReject) : 0u;
+    if (!w1 && !u1) {
+        x = large ? lane_solve32(f, f.canon(u), one, w, l) : lane_solve16(f, f.canon(u), one, w, l);
+        if (x == ~0u) x = kEvUnknown;                  // p is not prime; the order stage drops it
+    }
+    return __umul64hi(e, l) == 0 ? x : kEvUnknown;
 }
 
-__device__ __noinline__ u32 split_solve_m(u64 p, const DevItem& it, u32 l, u64 l_inv) {
-    return split_solve<FieldM>(p, it, l, l_inv);       // out of line: the FP64 path sets the registers
+__device__ __noinline__ u32 split_solve_m(u64 p, const DevItem& it, u32 l, u64 l_inv, bool large, u32 together) {
+    return split_solve<FieldM>(p, it, l, l_inv, large, together);   // out of line: the FP64 path sets the registers
 }
 
 // One lane per event, a list after the other, the longest walks first.
-__global__ void __launch_bounds__(256, 3) k_dlog(PrepArgs a, Counters* ctr) {
+__global__ void __launch_bounds__(256, 4) k_dlog(PrepArgs a, Counters* ctr) {
     const u32 lane = threadIdx.x & 31;
-    const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
     constexpr u32 order[kSplitLists] = {8, 3, 7, 2, 6, 1, 5, 0, 9, 4};
     static_assert(kSplitSizes == 5, "the lists' order");
     u64 count[kSplitLists], total = 0;
@@ -1108,34 +1264,66 @@ __global__ void __launch_bounds__(256, 3) k_dlog(PrepArgs a, Counters* ctr) {
         count[i] = min((u64)*(volatile unsigned long long*)&ctr->events[order[i]], a.ev_cap);
         total += (count[i] + 31) / 32;
     }
-    for (u64 unit = (u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; unit < total; unit += warps) {
+    // the first unit of a warp is fixed, block by block, so that the longest walks
+    // start on all SMs (claimed like the others, they went to the SMs whose blocks
+    // started first: 2^20 integers at 10^9, 64 us instead of 27)
+    const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
+    for (u64 unit = (u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; unit < total;) {
         u64 k = unit, idx = 0;
-        bool placed = false, live = false;
+        if (lane == 0) unit = warps + atomicAdd(&ctr->dlog_next, 1ull);
+        unit = __shfl_sync(FULL, unit, 0);
+        bool placed = false, live = false, large = false;
 #pragma unroll
         for (u32 i = 0; i < kSplitLists; ++i) {
             const u64 units = (count[i] + 31) / 32;
             if (!placed && k < units) {
                 idx = order[i] * a.ev_cap + k * 32 + lane;
                 live = k * 32 + lane < count[i];
+                large = i < 4;                         // l > 256
                 placed = true;
             }
             k -= units;
         }
-        if (!live) continue;
-        const SplitEvent s = a.events[idx];
-        Entry& e = a.ent[s.entry];
-        const u64 p = e.p;
-        const DevItem& it = a.items[e.item];
-        const u32 li = s.which >> 16, l = a.tables.sp[kSplitBase + li];
-        const u64 l_inv = a.tables.inv[kSplitBase + li], rcp = a.tables.rcp[kSplitBase + li];
-        u32 x = p < kFp64Limit ? split_solve<FieldF>(p, it, l, l_inv) : split_solve_m(p, it, l, l_inv);
-        if (x < kEvReject) {
-            // n_first + j L == x (mod l) for j; L is prime to l unless the class modulus holds l
+        const u32 together = __ballot_sync(FULL, live);
+        if (live) {
+            const SplitEvent s = a.events[idx];
+            Entry& e = a.ent[s.entry];
+            const u64 p = e.p;
+            u32 slots = 0;                             // the slots with an l (their loads go together)
+#pragma unroll
+            for (u32 i = 0; i < kSplitSlots; ++i)
+                if (e.ev[i] != 0) slots |= 1u << i;
+            const u64 classes = *reinterpret_cast<const u64*>(e.k);
+            const u32 together_f = __ballot_sync(together, p < kFp64Limit);
+            const DevItem& it = a.items[e.item];
+            const u32 li = s.which >> 16, l = a.tables.sp[kSplitBase + li];
+            const u64 l_inv = a.tables.inv[kSplitBase + li], rcp = a.tables.rcp[kSplitBase + li];
+            u32 x = p < kFp64Limit ? split_solve<FieldF>(p, it, l, l_inv, large, together_f)
+                                   : split_solve_m(p, it, l, l_inv, large, together & ~together_f);
+            __syncwarp(together);
+            // n_first + j L == x (mod l) for j, and the inverse that k_setup combines
+            // it with, that of the earlier slots' primes' product M: from one
+            // inverse, of L M.  L is prime to l unless the class modulus holds l
+            const u32 slot = s.which & 0xFFFFu;
             const u32 Lm = mod_small(e.L, l, rcp), nm = mod_small(e.n_first, l, rcp);
-            if (Lm != 0) x = (x >= nm ? x - nm : x + l - nm) * inv_mod32(Lm, l) % l;
-            else x = x == nm ? kEvUnknown : kEvReject;
+            u32 Mm = 1, inv = 0;
+            for (u32 before = slots & ((1u << slot) - 1); before; before &= before - 1) {
+                const u32 i = (u32)__ffs((int)before) - 1;
+                const u32 k = i < kSplitClasses ? (u32)(classes >> (16 * i)) & 0xFFFFu : slot_small(i);
+                Mm = Mm * a.tables.sp[kSplitBase + k] % l;
+            }
+            if (x < kEvReject) {
+                if (Lm != 0) {
+                    const u32 lm = inv_mod_small(Lm * Mm % l, l);
+                    x = (x >= nm ? x - nm : x + l - nm) * (lm * Mm % l) % l;
+                    inv = lm * Lm % l;
+                } else {
+                    x = x == nm ? kEvUnknown : kEvReject;
+                }
+            }
+            e.ev[slot] = kEvQueued | inv << kEvInvShift | x;
         }
-        e.ev[s.which & 0xFFFFu] = (li + 1) << 16 | x;
+        __syncwarp();
     }
 }
 
@@ -1143,31 +1331,36 @@ __global__ void __launch_bounds__(256, 3) k_dlog(PrepArgs a, Counters* ctr) {
 
 // Applies what k_dlog found to the entry's candidates; false when none is
 // left.  ev: the entry's slots in memory, each lane taking its own next one (an
-// entry has 1.7 on average, so a loop over the slots would mostly idle).
-__device__ __forceinline__ bool apply_events(Entry& e, const u32* ev, const SieveTables& t) {
+// entry has 1.7 on average, so a loop over the slots would mostly idle).  The
+// residues are combined one after the other with the inverses that k_dlog left;
+// these are those of all earlier slots' primes, so after a slot that taught
+// nothing (1 in l^2) they are computed here.
+__device__ __forceinline__ bool apply_events(Entry& e, const Entry& mem, const SieveTables& t) {
     u32 mask = 0;
 #pragma unroll
     for (u32 i = 0; i < kSplitSlots; ++i)
-        if (e.ev[i] != 0 && (e.ev[i] & 0xFFFFu) != kEvUnknown) mask |= 1u << i;
+        if (e.ev[i] != 0) mask |= 1u << i;
     u64 j = 0, M = 1;                                  // the j left: == j (mod M)
+    bool whole = true;                                 // M is the product of all earlier slots' primes
     while (mask) {
-        const u32 v = ev[__ffs((int)mask) - 1], x = v & 0xFFFFu;
+        const u32 slot = (u32)__ffs((int)mask) - 1, v = mem.ev[slot], x = v & kEvValue;
         mask &= mask - 1;
         if (x == kEvReject) return false;
-        const u32 k = kSplitBase + (v >> 16) - 1, l = t.sp[k];
-        if (M == 1) {
-            j = x;
-            M = l;
+        if (x == kEvUnknown) {
+            whole = false;
+            continue;
+        }
+        const u32 k = kSplitBase + (slot < kSplitClasses ? mem.k[slot] : slot_small(slot)), l = t.sp[k];
+        const u64 rcp = t.rcp[k];
+        const u32 jm = mod_small(j, l, rcp);
+        const u32 diff = x >= jm ? x - jm : x + l - jm;
+        if (M >= e.jcount) {                           // one candidate at most: check it
+            if (diff) return false;
+            whole = false;
         } else {
-            const u64 rcp = t.rcp[k];
-            const u32 jm = mod_small(j, l, rcp);
-            const u32 diff = x >= jm ? x - jm : x + l - jm;
-            if (M >= e.jcount) {                       // one candidate at most: check it
-                if (diff) return false;
-            } else {
-                j += M * (diff * inv_mod32(mod_small(M, l, rcp), l) % l);
-                M *= l;
-            }
+            const u32 inv = whole ? v >> kEvInvShift & kEvValue : inv_mod_small(mod_small(M, l, rcp), l);
+            j += M * mod_small((u64)diff * inv, l, rcp);
+            M *= l;
         }
         if (j >= e.jcount) return false;
     }
@@ -1212,13 +1405,14 @@ __device__ __forceinline__ bool setup_entry(Entry& e, const DevItem& it, const P
 }
 
 template <class F>
-__device__ __forceinline__ u32 lane_solve_entry(const Entry& e) {
+__device__ __forceinline__ u32 lane_solve_entry(const Entry& e, bool large) {
     F f;
     f.init(e.p);
-    return lane_solve(f, f.from_u64(e.t), f.from_u64(e.G0), f.from_u64(e.B), e.jcount);
+    return large ? lane_solve32(f, f.from_u64(e.t), f.from_u64(e.G0), f.from_u64(e.B), e.jcount)
+                 : lane_solve16(f, f.from_u64(e.t), f.from_u64(e.G0), f.from_u64(e.B), e.jcount);
 }
 
-__device__ __noinline__ u32 lane_solve_entry_m(const Entry& e) { return lane_solve_entry<FieldM>(e); }
+__device__ __noinline__ u32 lane_solve_entry_m(const Entry& e, bool large) { return lane_solve_entry<FieldM>(e, large); }
 
 // Entries with at most kLaneMax candidates are solved here, one lane each:
 // 1.6 lane instructions a candidate against about 490 warp instructions of
@@ -1227,8 +1421,9 @@ __device__ __noinline__ u32 lane_solve_entry_m(const Entry& e) { return lane_sol
 constexpr u32 kLaneSizes = 6, kLaneQueues = 2 * kLaneSizes, kLaneMax = 2048, kLaneMin = 64;   // J <= 64, 128, .. 2048
 constexpr u32 kLaneFew = 1u << 16, kLaneMaxFew = 256;            // (2^19 integers at 10^9: 248 us with 2048, 231 with 256)
 
-__global__ void __launch_bounds__(256, 3) k_setup(PrepArgs a, Counters* ctr) {
-    __shared__ u32 queues[8][kLaneQueues][64];
+constexpr u32 kSetupWarps = 4;
+__global__ void __launch_bounds__(kSetupWarps * 32, 7) k_setup(PrepArgs a, Counters* ctr) {
+    __shared__ u32 queues[kSetupWarps][kLaneQueues][64];
     u32(&Q)[kLaneQueues][64] = queues[threadIdx.x >> 5];
     const u32 lane = threadIdx.x & 31, below = (1u << lane) - 1;
     const u64 n_ent = min((u64)*(volatile unsigned long long*)&ctr->entries, a.ent_cap);
@@ -1260,11 +1455,13 @@ __global__ void __launch_bounds__(256, 3) k_setup(PrepArgs a, Counters* ctr) {
             if (taken == 0) break;
         }
         if (q < kLaneQueues || !inputs) {
+            // the two smallest sizes with 16 baby steps
+            const bool large = q < kLaneQueues ? q % kLaneSizes >= 2 : lane_max > kLaneMaxFew;
             if (idx != ~0u) {
                 const Entry& e = a.ent[idx];
-                const u32 j = e.p < kFp64Limit ? lane_solve_entry<FieldF>(e) : lane_solve_entry_m(e);
+                const u32 j = e.p < kFp64Limit ? lane_solve_entry<FieldF>(e, large) : lane_solve_entry_m(e, large);
                 if (j != ~0u) emit_relation(e.p, e.n_first + (u64)j * e.L, 0, e.item, a.rel, a.rel_cap, ctr);
-                steps += kLaneBaby + (min(j, e.jcount) + kLaneBaby - 1) / kLaneBaby;
+                steps += large ? 32 + (min(j, e.jcount) + 31) / 32 : 16 + (min(j, e.jcount) + 15) / 16;
             }
             __syncwarp();
             continue;
@@ -1278,26 +1475,32 @@ __global__ void __launch_bounds__(256, 3) k_setup(PrepArgs a, Counters* ctr) {
         }
         idx = (u32)first + lane;
         u32 cls = kLaneQueues + 1;                     // kLaneQueues: for k_bsgs
+        // (the lanes leave apply_events at different times: together again for the powers)
+        Entry e;
+        bool ok = false;
         if (first + lane < n_ent) {
-            Entry e = a.ent[idx];
+            e = a.ent[idx];
+            ok = apply_events(e, a.ent[idx], a.tables);
+        }
+        __syncwarp();
+        if (ok) {
             const DevItem& it = a.items[e.item];
-            if (apply_events(e, a.ent[idx].ev, a.tables)) {
-                const bool small = e.jcount <= lane_max;
-                if (e.p < kFp64Limit ? setup_entry<FieldF>(e, it, a, ctr, small)
-                                     : setup_entry<FieldM>(e, it, a, ctr, small)) {
-                    Entry& d = a.ent[idx];
-                    d.t = e.t; d.G0 = e.G0; d.B = e.B; d.Bm = e.Bm; d.jcount = e.jcount; d.m = e.m;
-                    d.pinv = e.pinv; d.G = e.G; d.tw = e.tw;
-                    d.n_first = e.n_first; d.L = e.L;
-                    cls = kLaneQueues;
-                    if (small) {
-                        cls = 0;
-                        while (e.jcount > (kLaneMin << cls)) ++cls;
-                        if (e.p >= kFp64Limit) cls += kLaneSizes;
-                    }
+            const bool small = e.jcount <= lane_max;
+            if (e.p < kFp64Limit ? setup_entry<FieldF>(e, it, a, ctr, small)
+                                 : setup_entry<FieldM>(e, it, a, ctr, small)) {
+                Entry& d = a.ent[idx];
+                d.t = e.t; d.G0 = e.G0; d.B = e.B; d.Bm = e.Bm; d.jcount = e.jcount; d.m = e.m;
+                d.pinv = e.pinv; d.G = e.G; d.tw = e.tw;
+                d.n_first = e.n_first; d.L = e.L;
+                cls = kLaneQueues;
+                if (small) {
+                    cls = 0;
+                    while (e.jcount > (kLaneMin << cls)) ++cls;
+                    if (e.p >= kFp64Limit) cls += kLaneSizes;
                 }
             }
         }
+        __syncwarp();
 #pragma unroll
         for (u32 k = 0; k < kLaneQueues; ++k) {
             const u32 bal = __ballot_sync(FULL, cls == k);
@@ -1351,7 +1554,7 @@ __device__ __forceinline__ bool table_maybe(const unsigned short* tab, u32 mask,
 // Smallest i in [lo, limit) with key(t * B^i) == key, or -1 (warp-cooperative;
 // tbl = t * B^lane, B32 = B^32).
 template <class F>
-__device__ __noinline__ int find_baby_index(const F& f, typename F::V tbl, typename F::V B32, u32 lo, u32 limit, u64 key) {
+__device__ __noinline__ int find_baby_index(F f, typename F::V tbl, typename F::V B32, u32 lo, u32 limit, u64 key) {
     const u32 lane = threadIdx.x & 31;
     typename F::V v = tbl;
     for (u32 base = 0; base < limit; base += 32) {
@@ -1510,7 +1713,7 @@ __device__ __forceinline__ bool ftable_walk(const u32* tab, u32 mask, u32 s, u32
 
 // Smallest i in [lo, limit) with t * B^i == v (canonical doubles compared
 // exactly); -1 when there is none.  Warp-cooperative: tbl = t * B^lane.
-__device__ __noinline__ int ffind_baby(const Fp64& f, double tbl, double B32, u32 lo, u32 limit, double v) {
+__device__ __noinline__ int ffind_baby(Fp64 f, double tbl, double B32, u32 lo, u32 limit, double v) {
     const u32 lane = threadIdx.x & 31;
     double x = tbl;
     for (u32 base = 0; base < limit; base += 32) {
@@ -1699,9 +1902,6 @@ __device__ __forceinline__ u32 fq_hash(double c) {
 __device__ __forceinline__ u32 fq_fingerprints(u32 h) {        // in both halves
     return (__byte_perm(h, h, 0x3232) & 0x3FFF3FFFu) | 0x80008000u;
 }
-__device__ __forceinline__ u32 fq_equal_halves(u32 a, u32 b) {
-    return __heq2_mask(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
-}
 
 __device__ __forceinline__ bool fq_word_has(u64 w, u32 pat) {
     const u32 lo = (u32)w & ~kQOvf, hi = (u32)(w >> 32);
@@ -1805,7 +2005,7 @@ __device__ __forceinline__ void fq_insert_count(unsigned char* tab, unsigned cha
 
 // The largest i in [0, m) with t * B^i == v (canonical doubles compared
 // exactly); -1 when there is none.  Warp-cooperative: tbl = t * B^lane.
-__device__ __noinline__ int ffind_last(const Fp64& f, double tbl, double B32, u32 m, double v) {
+__device__ __noinline__ int ffind_last(Fp64 f, double tbl, double B32, u32 m, double v) {
     const u32 lane = threadIdx.x & 31;
     double x = tbl;
     int last = -1;
@@ -1841,7 +2041,7 @@ __device__ __forceinline__ SolveF solve_f(const Solve& e, u32 tbits, u32 fill) {
 template <int CH, bool WI>
 __device__ u64 solve_fp64q(const SolveF& e, unsigned long long* tab, u32 tbits, u64* steps_out) {
     const u32 lane = threadIdx.x & 31, lo = lane & 15;
-    const Fp64& f = e.f;
+    const Fp64 f = e.f;
     const u32 m = e.m, G = e.G;
     const u32 mask = (1u << e.tw) - 1, mask8 = mask << 3;
 
@@ -1919,7 +2119,7 @@ __device__ u64 solve_fp64q(const SolveF& e, unsigned long long* tab, u32 tbits, 
             nx[c] = f.mul(gx[c], Gstep);                  // the next value, independent of the probe
             const uint2 w = *reinterpret_cast<const uint2*>(bytes + (hs[c] & mask8));
             const u32 rep = fq_fingerprints(hs[c]);
-            z |= fq_equal_halves(w.x, rep) | fq_equal_halves(w.y, rep) | (w.x & kQOvf);
+            z |= equal_halves(w.x, rep) | equal_halves(w.y, rep) | (w.x & kQOvf);
         }
         if (__any_sync(FULL, z)) {
             // the rare path: walk overflowed homes, then resolve exact matches in increasing g
@@ -2912,8 +3112,8 @@ cudaError_t launch_sieve_wave(const WaveDesc* w, const SieveTables& t, const Sur
 cudaError_t launch_prep(const PrepArgs& a, Counters* ctr, int grid, int num_sms, cudaStream_t s) {
     k_prep<<<grid, kPrepThreads, 0, s>>>(a, ctr);
     if (!a.surv_split) k_split<<<num_sms * 2, 256, 0, s>>>(a, ctr);
-    k_dlog<<<num_sms * 3, 256, 0, s>>>(a, ctr);
-    k_setup<<<num_sms * 3, 256, 0, s>>>(a, ctr);
+    k_dlog<<<num_sms * 4, 256, 0, s>>>(a, ctr);
+    k_setup<<<num_sms * 7, kSetupWarps * 32, 0, s>>>(a, ctr);
     return cudaGetLastError();
 }
 

@@ -42,7 +42,7 @@ namespace {
 constexpr u64 kNoAllocMaxSpan = 1ull << 19;
 constexpr u64 kNoAllocEntries = 11ull << 12;         // more than the 43,390 primes below 2^19, the most a range holds
 constexpr u64 kNoAllocSurv = kNoAllocEntries;        // (the same bound holds for the sieve's survivors)
-constexpr u64 kNoAllocEvents = 5ull << 12;           // per split list (a full list loses splits, not relations)
+constexpr u64 kNoAllocEvents = 1ull << 14;           // per split list (a full list loses splits, not relations)
 constexpr u64 kNoAllocRelations = 1ull << 14;
 constexpr u32 kNoAllocMaxDevices = 64;
 
