@@ -49,7 +49,8 @@ constexpr u32 kNoAllocMaxDevices = 64;
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kOffCounters = 0;
 constexpr size_t kOffItem = align256(kOffCounters + sizeof(Counters));
-constexpr size_t kOffSp = align256(kOffItem + sizeof(DevItem));
+constexpr size_t kOffRel = align256(kOffItem + sizeof(DevItem));     // read back with the counters in one copy
+constexpr size_t kOffSp = align256(kOffRel + kNoAllocRelations * sizeof(RawRelation));
 constexpr size_t kOffRcp = align256(kOffSp + kSievePrimes * sizeof(u32));
 constexpr size_t kOffInv = align256(kOffRcp + kSievePrimes * sizeof(u64));
 constexpr size_t kOffSurv = align256(kOffInv + kSievePrimes * sizeof(u64));
@@ -57,8 +58,7 @@ constexpr size_t kOffSplit = align256(kOffSurv + kNoAllocSurv * sizeof(u64));
 constexpr size_t kOffEnt = align256(kOffSplit + kNoAllocSurv * sizeof(u64));
 constexpr size_t kOffEvents = align256(kOffEnt + kNoAllocEntries * sizeof(Entry));
 constexpr size_t kOffBig = align256(kOffEvents + kSplitSizes * kNoAllocEvents * sizeof(SplitEvent));
-constexpr size_t kOffRel = align256(kOffBig + kNoAllocEntries * sizeof(u32));
-constexpr size_t kNoAllocUsed = align256(kOffRel + kNoAllocRelations * sizeof(RawRelation));
+constexpr size_t kNoAllocUsed = align256(kOffBig + kNoAllocEntries * sizeof(u32));
 constexpr size_t kNoAllocBytes = 8u << 20;
 static_assert(kNoAllocUsed <= kNoAllocBytes, "no-alloc scratch layout exceeds its array");
 
@@ -219,15 +219,20 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
 
     const size_t smem = bsgs_smem_bytes(tbits, 4, 0);
     const int bgrid = num_sms * std::max(1, std::min((int)(228 * 1024 / (smem + 1024)), 16));
-    if (cudaMemsetAsync(ctr, 0, sizeof(Counters), s) != cudaSuccess) return MPS_E_CUDA;
-    if (cudaMemcpyAsync(ditem, &d, sizeof(DevItem), cudaMemcpyHostToDevice, s) != cudaSuccess) return MPS_E_CUDA;
+    // the cleared counters and the item go up in one copy, and come back with the
+    // first relations in one
+    alignas(256) unsigned char head[kOffRel + kReadBatch * sizeof(RawRelation)];
+    std::memset(head, 0, kOffRel);
+    std::memcpy(head + kOffItem, &d, sizeof(DevItem));
+    if (cudaMemcpyAsync(base, head, kOffRel, cudaMemcpyHostToDevice, s) != cudaSuccess) return MPS_E_CUDA;
     if (launch_sieve(sa, tables, SurvOut{surv, nullptr, split, kNoAllocSurv}, ctr, s) != cudaSuccess) return MPS_E_CUDA;
     if (launch_prep(pa, ctr, num_sms * 4, num_sms, s) != cudaSuccess) return MPS_E_CUDA;
     if (launch_bsgs(ba, ctr, bgrid, s) != cudaSuccess) return MPS_E_CUDA;
     if (launch_order(oa, ctr, num_sms * 2, s) != cudaSuccess) return MPS_E_CUDA;
-    Counters h;
-    if (cudaMemcpyAsync(&h, ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MPS_E_CUDA;
+    if (cudaMemcpyAsync(head, base, sizeof(head), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MPS_E_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return MPS_E_CUDA;
+    Counters h;
+    std::memcpy(&h, head + kOffCounters, sizeof(Counters));
     if (h.status & (kStatusOrderFailed | kStatusBadLaunch)) return MPS_E_CUDA;
     if (h.status & (kStatusSurvivorOverflow | kStatusEntryOverflow | kStatusRelationOverflow)) {
         // denser than the scratch holds: split the range (no allocation)
@@ -240,8 +245,10 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     RawRelation buf[kReadBatch];
     for (u64 i0 = 0; i0 < nr; i0 += kReadBatch) {
         const u64 k = std::min<u64>(kReadBatch, nr - i0);
-        if (cudaMemcpyAsync(buf, rel + i0, k * sizeof(RawRelation), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
+        if (i0 == 0)
+            std::memcpy(buf, head + kOffRel, k * sizeof(RawRelation));
+        else if (cudaMemcpyAsync(buf, rel + i0, k * sizeof(RawRelation), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+                 cudaStreamSynchronize(s) != cudaSuccess)
             return MPS_E_CUDA;
         for (u64 i = 0; i < k; ++i) {
             if (buf[i].q == ~0ull) continue;      // a composite survivor
