@@ -73,7 +73,8 @@ typedef struct mps_tuning {
                                     1: lcm(mod, 2), the reference's plain-method filter)       */
     uint32_t full_mr;           /* 1: 12-base Miller-Rabin on every filter survivor (eager)    */
     uint32_t plain;             /* 1: plain per-chunk path (host sync between stages)          */
-    uint32_t chains;            /* BSGS chains per lane, 1, 2 or 4 (0: 2)                      */
+    uint32_t chains;            /* BSGS chains per lane, 1, 2 or 4 (0: 2, or 4 for an item of at
+                                   least 2^20 in-class exponents)                               */
     uint32_t graphs_off;        /* 1: launch waves directly instead of replaying CUDA graphs   */
     uint32_t table_kind;        /* BSGS table: 0 = four 16-bit fingerprints per 64-bit word,
                                    inserted by compare-and-swap, 1 = one 32-bit key per slot,
