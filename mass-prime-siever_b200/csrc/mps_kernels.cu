@@ -265,21 +265,24 @@ __device__ void sieve_segment(SieveShared<W>& sh, u64 v0, u32 len, u32 n_primes,
             sh.split_start[k] = (unsigned short)((d & 1u) ? (d + q) >> 1 : d >> 1);
         }
         __syncthreads();
-        unsigned short* out = reinterpret_cast<unsigned short*>(o.split);
+        unsigned short* out = reinterpret_cast<unsigned short*>(o.split + base);
+        const u32 room = base < o.cap ? (u32)min(o.cap - base, (u64)~0u) : 0u;
         auto visit = [&](u32 i, u32 c, u32 k) {
             const u32 w = ~sh.bits[i >> 5] << (31 - (i & 31));     // bit i on top
             if ((int)w < 0) {
-                const u64 pos = base + sh.before[i >> 5] + __popc(w) - 1;
-                if (pos < o.cap) out[4 * pos + c] = (unsigned short)(k + 1);
+                const u32 r = sh.before[i >> 5] + __popc(w) - 1;
+                if (r < room) out[4 * r + c] = (unsigned short)(k + 1);
             }
         };
         const u32 n_shared = min(n_split, kSplitShared);
         for (u32 k = kSplitSmall + warp; k < n_shared; k += kSieveThreads / 32) {
             const u32 q = t.sp[kSplitBase + k], c = split_class(k);
+#pragma unroll 4
             for (u32 i = sh.split_start[k] + lane * q; i < len; i += 32 * q) visit(i, c, k);
         }
         for (u32 k = kSplitShared + tid; k < n_split; k += kSieveThreads) {
             const u32 q = t.sp[kSplitBase + k];
+#pragma unroll 4
             for (u32 i = sh.split_start[k]; i < len; i += q) visit(i, kSplitClasses - 1, k);
         }
     }
