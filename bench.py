@@ -297,8 +297,8 @@ def kernel_rooflines(siever, pieces, peaks, fp64_path: bool) -> dict:
             "baby_steps_per_launch": tot["baby"] / n, "entries_per_launch": tot["entries"] / n,
             "traffic": traffic * tot["steps"] / n if traffic is not None else None,
             "traffic_unit": "DRAM bytes per launch", "traffic_source": traffic_src,
-            "hbm_side": {"algorithmic_bytes_per_launch": 72.0 * tot["entries"] / n,
-                         "frac_of_measured_hbm": (72.0 * tot["entries"] / (tot["bsgs_ms"] / 1e3)) / (hbm * 1e9)
+            "hbm_side": {"algorithmic_bytes_per_launch": 68.0 * tot["entries"] / n,   # at most: 64 B and an index each
+                         "frac_of_measured_hbm": (68.0 * tot["entries"] / (tot["bsgs_ms"] / 1e3)) / (hbm * 1e9)
                          if tot["bsgs_ms"] > 0 and hbm else None},
             "peaks_measured": {k: v / 1e9 for k, v in peaks.items()}}
     smem_peak = peaks.get("smem_atomic_per_s")

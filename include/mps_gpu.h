@@ -95,16 +95,16 @@ typedef struct mps_tuning {
 typedef struct mps_stats {
     uint64_t odds;              /* odd integers sieved                          */
     uint64_t survivors;         /* survivors of the sieve by the primes <= 65521 */
-    uint64_t entries;           /* primes that reached the BSGS                 */
+    uint64_t entries;           /* primes that reached the discrete-log stages  */
     uint64_t relations;         /* relations returned                           */
     uint64_t chunks;            /* device chunks run                            */
     double   device_ms;         /* device time of the call (CUDA events)        */
     double   bsgs_ms;           /* device time of the BSGS kernel               */
     uint64_t bsgs_launches;
     uint64_t kernel_launches;   /* kernels of this library launched             */
-    uint64_t bsgs_steps;        /* baby + giant steps (Montgomery multiplies) done by the BSGS */
+    uint64_t bsgs_steps;        /* baby + giant steps (modular multiplies) of the BSGS kernel */
     double   sieve_ms;          /* device time of the sieve kernel (CUDA events)  */
-    double   prep_ms;           /* device time of the prep kernel                 */
+    double   prep_ms;           /* device time of the prep kernels (prep, splits, set-up) */
     double   order_ms;          /* device time of the order kernel                */
     uint64_t bsgs_baby_steps;   /* the baby steps among bsgs_steps                */
 } mps_stats;

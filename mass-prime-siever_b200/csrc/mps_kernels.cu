@@ -1434,7 +1434,6 @@ __global__ void __launch_bounds__(kSetupWarps * 32, 7) k_setup(PrepArgs a, Count
     const u32 lane_max = n_ent < kLaneFew ? kLaneMaxFew : kLaneMax;
     u32 n[kLaneQueues] = {};                           // queue lengths (warp-uniform)
     bool inputs = true;
-    u64 steps = 0;
     for (;;) {
         // a queue that holds 32 is drained; once the inputs are used up, the
         // last 32 entries of all the queues together, the longest first
@@ -1464,7 +1463,6 @@ __global__ void __launch_bounds__(kSetupWarps * 32, 7) k_setup(PrepArgs a, Count
                 const Entry& e = a.ent[idx];
                 const u32 j = e.p < kFp64Limit ? lane_solve_entry<FieldF>(e, large) : lane_solve_entry_m(e, large);
                 if (j != ~0u) emit_relation(e.p, e.n_first + (u64)j * e.L, 0, e.item, a.rel, a.rel_cap, ctr);
-                steps += large ? 32 + (min(j, e.jcount) + 31) / 32 : 16 + (min(j, e.jcount) + 15) / 16;
             }
             __syncwarp();
             continue;
@@ -1519,8 +1517,6 @@ __global__ void __launch_bounds__(kSetupWarps * 32, 7) k_setup(PrepArgs a, Count
         }
         __syncwarp();
     }
-    steps = __reduce_add_sync(FULL, (u32)steps);
-    if (lane == 0 && steps) atomicAdd(&ctr->steps, (unsigned long long)steps);
 }
 
 // --------------------------------------------------------------- the BSGS --
