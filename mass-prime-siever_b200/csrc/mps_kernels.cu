@@ -3,10 +3,14 @@
 //   k_sieve  segment sieve of the odd numbers by the odd primes <= 65521,
 //            bitmap in shared memory, survivors compacted to global memory
 //            (what psieve does, Gpu.hpp:385-455, sized for 148 SMs)
-//   k_prep   per survivor: residues of b and -c, base-2 strong test,
+//   k_prep   per survivor: residues of b and -c, quadratic-character filter,
 //            power-residue split over g = gcd(Q, p - 1) (Gpu.hpp:465-589,
-//            Math.hpp:410-433), BSGS set-up; staged through shared-memory
+//            Math.hpp:410-433), class combination; staged through shared-memory
 //            queues so that every stage runs with full warps
+//   k_dlog   per prime and l | p - 1 (5 .. 4261, found by the sieve, or by
+//            k_split for given primes): the candidates' residue mod l
+//   k_setup  applies those, sets the solve up, and solves entries with few
+//            candidates left, one lane each
 //   k_bsgs   exact baby-step giant-step, one warp per prime: baby-step table
 //            of fingerprints + indices in shared memory, giant steps probed by
 //            every lane, the smallest j found with a warp min-reduction
