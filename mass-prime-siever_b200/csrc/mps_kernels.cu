@@ -679,20 +679,86 @@ __device__ bool power_split_pp(const F& f, u64 p, u64 w_res, u64 u_res, const De
     return true;
 }
 
+// a^-1 mod m for gcd(a, m) = 1, 0 < a < m < 2^13: extended Euclid with the
+// quotients by single-precision division, off by one at most and set right.  (At
+// most 18 steps: the remainders fall as fast as Fibonacci numbers.)
+__device__ __forceinline__ u32 inv_mod_small(u32 a, u32 m) {
+    int r0 = (int)m, r1 = (int)a, s0 = 0, s1 = 1;
+    for (int step = 0; step < 20 && r1 > 0; ++step) {
+        int q = (int)__fdividef((float)r0, (float)r1);
+        int r2 = r0 - q * r1;
+        if (r2 < 0) {
+            --q;
+            r2 += r1;
+        } else if (r2 >= r1) {
+            ++q;
+            r2 -= r1;
+        }
+        const int s2 = s0 - q * s1;
+        r0 = r1;
+        r1 = r2;
+        s0 = s1;
+        s1 = s2;
+    }
+    const int x = s0 % (int)m;
+    return (u32)(x < 0 ? x + (int)m : x);
+}
+
+// a / m and a % m for a < 2^24, 0 < m < 2^13 by single-precision division (off by one at most, set right).
+__device__ __forceinline__ u32 div_small(u32 a, u32 m, u32& rem) {
+    int q = (int)__fdividef((float)a, (float)m), r = (int)a - q * (int)m;
+    if (r < 0) {
+        --q;
+        r += (int)m;
+    } else if (r >= (int)m) {
+        ++q;
+        r -= (int)m;
+    }
+    rem = (u32)r;
+    return (u32)q;
+}
+__device__ __forceinline__ u32 mod_small24(u32 a, u32 m) {
+    u32 r;
+    div_small(a, m, r);
+    return r;
+}
+
 // Stage 3: n = n_start + cm*k (in class) with n == r (mod d): the candidates
 // n_first + j*L, j < jcount.  False when there is none.
 __device__ __forceinline__ bool combine_class(u64 p, const DevItem& it, u32 d, u32 r, Entry& e) {
     // the smallest k0 >= 0 with n_start + cm*k0 == r (mod d): k0*cmd == want
     // (mod d) is solvable iff h = gcd(cmd, d) divides want, and then its
     // solutions are k0 + per*i with per = d/h, k0 = (want/h)(cmd/h)^-1 mod per
-    const u32 cmd = it.cmQ % d;                        // d | Q
-    const u32 want = (r + d - it.nsQ % d) % d;
-    const u32 h = gcd32(cmd, d);                       // gcd(0, d) = d
-    if (want % h) return false;
-    const u32 per = d / h;                             // period of k
-    const u32 k0 = (u32)((u64)(want / h) * inv_mod32((cmd / h) % per, per) % per);
-    if (k0 >= it.K) return false;
-    u64 jcount = ((u32)it.K - k0 + per - 1) / per;     // K < 2^32 (N1 - N0 <= 10^7)
+    u32 per, k0;                                       // period of k
+    u64 jcount;
+    if (it.Q <= 4096) {
+        // (every value here is below 2^24, where a quotient by single precision costs
+        // half of an integer division: the prep kernels -0.8%)
+        const u32 cmd = mod_small24(it.cmQ, d);        // d | Q
+        const u32 want = mod_small24(r + d - mod_small24(it.nsQ, d), d);
+        u32 h = d, x = cmd, rem;                       // h = gcd(cmd, d), gcd(0, d) = d
+        for (int step = 0; step < 20 && x != 0; ++step) {
+            const u32 y = mod_small24(h, x);
+            h = x;
+            x = y;
+        }
+        const u32 wh = div_small(want, h, rem);
+        if (rem) return false;
+        per = div_small(d, h, rem);
+        const u32 ch = mod_small24(div_small(cmd, h, rem), per);
+        k0 = per == 1 ? 0u : mod_small24(wh * inv_mod_small(ch, per), per);
+        if (k0 >= it.K) return false;
+        jcount = div_small((u32)it.K - k0 + per - 1, per, rem);   // K <= 10^7
+    } else {
+        const u32 cmd = it.cmQ % d;
+        const u32 want = (r + d - it.nsQ % d) % d;
+        const u32 h = gcd32(cmd, d);
+        if (want % h) return false;
+        per = d / h;
+        k0 = (u32)((u64)(want / h) * inv_mod32((cmd / h) % per, per) % per);
+        if (k0 >= it.K) return false;
+        jcount = ((u32)it.K - k0 + per - 1) / per;
+    }
     if (jcount > p) jcount = p;                        // ord(B) < p (Math.hpp:398-400)
     e.jcount = (u32)jcount;
     e.L = it.cm * per;
@@ -907,32 +973,6 @@ __device__ __forceinline__ u32 lane_solve32(const F& f, typename F::V t, typenam
     if (best == ~0u && n > 1) best = lane_match32(f, t, B, g1, b1);
     return best < J ? best : ~0u;
 }
-
-// a^-1 mod m for gcd(a, m) = 1, 0 < a < m < 2^13: extended Euclid with the
-// quotients by single-precision division, off by one at most and set right.  (At
-// most 18 steps: the remainders fall as fast as Fibonacci numbers.)
-__device__ __forceinline__ u32 inv_mod_small(u32 a, u32 m) {
-    int r0 = (int)m, r1 = (int)a, s0 = 0, s1 = 1;
-    for (int step = 0; step < 20 && r1 > 0; ++step) {
-        int q = (int)__fdividef((float)r0, (float)r1);
-        int r2 = r0 - q * r1;
-        if (r2 < 0) {
-            --q;
-            r2 += r1;
-        } else if (r2 >= r1) {
-            ++q;
-            r2 -= r1;
-        }
-        const int s2 = s0 - q * s1;
-        r0 = r1;
-        r1 = r2;
-        s0 = s1;
-        s1 = s2;
-    }
-    const int x = s0 % (int)m;
-    return (u32)(x < 0 ? x + (int)m : x);
-}
-
 
 // What stage 1 tests of primality itself: a base-2 strong test where the powers
 // of b prove nothing (|b| <= 1), all 12 bases when the caller asks for them.
