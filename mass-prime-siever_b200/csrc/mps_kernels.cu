@@ -772,14 +772,16 @@ __device__ __forceinline__ bool combine_class(u64 p, const DevItem& it, u32 d, u
 // w = b^((p-1)/l) and u = t^((p-1)/l), b^n == t forces w^n == u, so n is known
 // mod l (or, when b is an l-th power residue, t has to be one too).  One
 // discrete logarithm in a group of l elements divides the candidates by l and
-// the baby and giant steps by sqrt(l); a prime has an l of 23 .. 4261 with
-// chance 1/(l-1), about one each.  Finding them costs a second walk of the
-// sieve's bitmap (sieve_segment); a logarithm costs about 720 + 1.6 l lane
-// instructions (k_dlog), so only entries with enough candidates have it.
-// Measured on 2^27 integers of b = 10, c = 111 at 10^12 (1.25 M entries):
-// k_bsgs 3.44 -> 1.62 ms for 0.06 ms of sieve, 0.21 of k_dlog and 0.20 of
-// k_setup (which took the set-up over from k_prep and solves the smallest
-// entries); BSGS steps 2.10e9 -> 0.90e9.
+// the baby and giant steps by sqrt(l); a prime has an l of 5 .. 4261 with
+// chance 1/(l-1), 1.7 in all.  Those of 5 .. 19 are tried on each entry, finding
+// the others costs a second walk of the sieve's bitmap (sieve_segment); a
+// logarithm costs about 700 lane instructions for the powers and 1.2 l for the
+// walk (k_dlog), so only entries with enough candidates have it.
+// On 2^27 integers of b = 10, c = 111 at 10^12 (1.36 M entries), against the split
+// by lcm(mod, 232792560) alone: BSGS steps 2.10e9 -> 0.87e9 and, with the later
+// changes of the step itself, k_bsgs 3.44 -> 1.28 ms, for 0.13 ms of sieve, 0.28 of
+// k_dlog and 0.17 of k_setup (which took the set-up over from k_prep and solves
+// the smallest entries).
 
 // How many primes of the table an entry with J candidates is split by.  (The
 // optimum is flat: splitting from 512 candidates on, by all primes from 4096,
@@ -1462,8 +1464,8 @@ __device__ __forceinline__ u32 lane_solve_entry(const Entry& e, bool large) {
 __device__ __noinline__ u32 lane_solve_entry_m(const Entry& e, bool large) { return lane_solve_entry<FieldM>(e, large); }
 
 // Entries with at most kLaneMax candidates are solved here, one lane each:
-// 1.6 lane instructions a candidate against about 490 warp instructions of
-// per-prime set-up in k_bsgs.  A warp's lanes walk together, so the entries
+// 1.2 lane instructions a candidate against about 290 warp instructions of
+// per-prime set-up in k_bsgs and its partly filled iterations.  A warp's lanes walk together, so the entries
 // wait in queues by size (a factor of two each) and arithmetic until one holds 32.
 constexpr u32 kLaneSizes = 6, kLaneQueues = 2 * kLaneSizes, kLaneMax = 2048, kLaneMin = 64;   // J <= 64, 128, .. 2048
 constexpr u32 kLaneFew = 1u << 16, kLaneMaxFew = 256;            // (2^19 integers at 10^9: 248 us with 2048, 231 with 256)
