@@ -1487,9 +1487,11 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
     // flags by p (host-supplied primes may repeat or be unsorted)
     if (ascending) {
         std::memset(flags, 0, n);
-        for (const RawRelation& r : rel)
-            for (const uint64_t* q = std::lower_bound(primes, primes + n, (uint64_t)r.p); q != primes + n && *q == r.p; ++q)
-                flags[q - primes] = 1;
+        for (const RawRelation& r : rel) {
+            const uint64_t* q = std::lower_bound(primes, primes + n, (uint64_t)r.p);
+            if (flags[q - primes]) continue;             // a repeated prime has a relation for each of its places
+            for (; q != primes + n && *q == r.p; ++q) flags[q - primes] = 1;
+        }
     } else {
         std::vector<u64> ps;
         ps.reserve(rel.size());
