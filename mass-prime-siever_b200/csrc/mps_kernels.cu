@@ -1437,6 +1437,14 @@ __device__ __forceinline__ bool setup_entry(Entry& e, const DevItem& it, const P
     if (e.jcount <= 1) return false;
     const V Bv = f.b_power(it, e.L);
     e.B = f.residue(Bv);
+    // B = 1 or -1: G0 B^j takes G0 and -G0 only.  (Every prime of an item with |b| = 1 is
+    // one; all its baby steps would share one or two words of the table, each walking
+    // past all the earlier ones: 2^20 integers at 10^9 with b = -1, K = 10^7, took 26 ms.)
+    if (e.B == 1 || e.B == e.p - 1) {
+        if (e.B != 1 && e.G0 + e.t == e.p)             // j = 1
+            emit_relation(e.p, e.n_first + e.L, 0, e.item, a.rel, a.rel_cap, ctr);
+        return false;
+    }
     if (small) return true;
     u32 m = (u32)isqrt_ceil_dev(e.jcount);
     if (it.baby_scale != 256) m = max(1u, (u32)(((u64)m * it.baby_scale + 255) >> 8));
@@ -1932,9 +1940,12 @@ __device__ u64 solve_fp64(const Solve& e, u32* tab, u32 tbits, u64* steps_out) {
 // Per 32 steps a giant step is 27 instructions (9 FP64, 12 ALU), a baby step 36,
 // and a prime costs 290 besides.
 //
-// A cycle B^d == 1 with d < m needs no care: the baby steps then repeat, the
-// table holds some keys several times, and the largest i of the smallest g
-// still gives the smallest j = g m - i.
+// A cycle B^d == 1 with d < m needs no care for the result: the baby steps then
+// repeat, the table holds some keys several times, and the largest i of the
+// smallest g still gives the smallest j = g m - i.  It costs a walk of about
+// m / 4d words an insertion, so k_setup decides the entries with d <= 2 itself;
+// larger orders as small as that are left to chance (p divides b^k - 1 for a k
+// of at most d L).
 
 constexpr u64 kQValid = 0x8000800080008000ull;
 constexpr u32 kQOvf = 0x4000u;
