@@ -418,7 +418,7 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     const u64 need_surv = n_odds + 16;
     if (int r = ensure(c, &c->d_surv, &c->surv_cap, std::max<u64>(need_surv, chunk + 16), "survivor buffer")) return r;
     if (int r = ensure(c, &c->d_surv_split, &c->surv_split_cap, c->surv_cap, "split primes")) return r;
-    if (int r = ensure_entries(c, std::max<u64>(chunk / 4, 1 << 16))) return r;
+    if (int r = ensure_entries(c, entry_cap(chunk))) return r;
     if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
 
     u32 tbits, max_baby;
@@ -592,8 +592,8 @@ int slot_alloc(mps_ctx* c, WaveSlot& w) {
         CK(cudaMalloc((void**)&w.d_surv_split, w.surv_cap * sizeof(u64)), "split primes");
         drop_graphs(w);
     }
-    if (w.ent_cap < std::max<u64>(chunk / 4, 1 << 16)) {
-        if (int r = alloc_entries(c, &w.d_ent, &w.d_events, &w.d_big, &w.ent_cap, std::max<u64>(chunk / 4, 1 << 16))) return r;
+    if (w.ent_cap < entry_cap(chunk)) {
+        if (int r = alloc_entries(c, &w.d_ent, &w.d_events, &w.d_big, &w.ent_cap, entry_cap(chunk))) return r;
         drop_graphs(w);
     }
     if (w.rel_cap < (1u << 16)) {

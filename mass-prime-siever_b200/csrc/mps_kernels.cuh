@@ -109,6 +109,11 @@ struct PrepArgs {
     u64 prime_below;           // survivors below this are prime (sieved by every prime up to their
                                // square root: 65521^2 for the sieve's survivors, 0 for caller-given numbers)
 };
+// Entries for a range of that many odd numbers: the primes of any such range (the
+// first one holds the most: pi(2 odds) stays below this, by 2% at 2^24 .. 2^26).
+// 160 B an entry (Entry, events, BSGS list): 20 B an odd number, and 16 B more
+// for the survivors and their split primes.
+constexpr u64 entry_cap(u64 odds) { return odds / 8 + (1u << 17); }
 // Events a list needs for ent_cap entries (an entry has 0.7 small l on average,
 // and a chunk above 10^6 fills its entries to a third at most); a full list
 // loses splits, never relations.

@@ -1,0 +1,29 @@
+"""Device memory of the work buffers."""
+from __future__ import annotations
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_wave_buffers_per_odd_number(mps_lib):
+    """The two wave slots together: at most 90 bytes per odd number of a chunk."""
+    import torch
+
+    torch.cuda.init()
+    before = torch.cuda.mem_get_info()[0]
+    with mps_lib.Siever(0, chunk_odds=1 << 27) as s:
+        s.item_relations(mps_lib.make_item(2, -25, 10**6, 2 * 10**6, 0, 1000, 2, 1))
+        used = before - torch.cuda.mem_get_info()[0]
+    assert used <= 90 << 27
+
+
+@pytest.mark.parametrize("odds", [1 << 20, 1 << 22, 1 << 23])
+def test_every_prime_of_the_densest_chunk_fits(mps_lib, odds):
+    """b = 2, c = -4 is solvable for every prime (n = 2): a chunk of the first odd
+    numbers has as many entries as a chunk can have, and is done in one piece."""
+    with mps_lib.Siever(0, chunk_odds=odds) as s:
+        it = mps_lib.make_item(2, -4, 3, 3 + 2 * odds, 3, 50, 1, 0)
+        s.chunk_relations(3, 3 + 2 * odds, it)
+        st = s.stats()
+        assert st["chunks"] == 1 and st["entries"] > 0.9 * s.count_primes(1000, 3 + 2 * odds)
