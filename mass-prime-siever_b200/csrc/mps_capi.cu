@@ -1482,6 +1482,9 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
                 if (c->h_rel[i].q != ~0ull) rel.push_back(c->h_rel[i]);
         }
         c->stats.kernel_launches += 3 + kPrepLaunches;
+        c->stats.entries += c->h_ctr->entries;
+        c->stats.bsgs_steps += c->h_ctr->steps;
+        c->stats.bsgs_baby_steps += c->h_ctr->baby;
     }
     if (int r = end_call(c)) return r;
     // flags by p (host-supplied primes may repeat or be unsorted)

@@ -1256,9 +1256,9 @@ __global__ void __launch_bounds__(256, 2) k_split(PrepArgs a, Counters* ctr) {
 #pragma unroll
             for (u32 g = 0; g < kSplitGroups; ++g) {
                 if (kSplitSmall + 32 * g >= n) break;
-                // l | x iff x l^-1 mod 2^64 <= floor((2^64 - 1) / l); the high words
-                // alone let through 2^-32 of the others (k_dlog compares in full)
-                if (__umulhi(xl, inv_lo[g]) + xl * inv_hi[g] + xh * inv_lo[g] <= lim[g]) div |= 1u << g;
+                // y = x l^-1 mod 2^64 is x / l when l | x, below 2^62 / l, and at least
+                // 2^64 / l when not (l y = x + i 2^64, i >= 1): the high words decide
+                if (__umulhi(xl, inv_lo[g]) + xl * inv_hi[g] + xh * inv_lo[g] < lim[g]) div |= 1u << g;
             }
             u32 bal = __ballot_sync(FULL, div != 0);
             while (bal) {                                      // one prime of each lane

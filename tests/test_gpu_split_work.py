@@ -1,0 +1,44 @@
+"""The split by primes l | p - 1 does its work: relations alone would not show a
+split that no longer happens, so the baby and giant steps left are compared,
+on every path, with those of the power-residue split alone."""
+from __future__ import annotations
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# b, c, P0, width, N0, N1, mod, res: both arithmetics; widths below and above 148 segments of the sieve
+ITEMS = [(3, 2, 10**9, 1 << 21, 0, 10**7, 1, 0), (10, 111, 10**12, 1 << 25, 0, 10**7, 6, 4),
+         (3, 2, 2**49, 1 << 22, 0, 2_000_000, 1, 0)]
+
+
+@pytest.mark.parametrize("b,c,P0,width,N0,N1,mod,res", ITEMS)
+def test_steps_left_by_the_split(mps_lib, b, c, P0, width, N0, N1, mod, res):
+    it = mps_lib.make_item(b, c, P0, P0 + width, N0, N1, mod, res)
+    steps, entries, relations = {}, {}, {}
+    for name, tuning in (("split", {}), ("unsplit", {"class_modulus": 144})):
+        with mps_lib.Siever(0, chains=2, **tuning) as s:
+            relations[name] = s.chunk_relations(P0, P0 + width, it)
+            steps[name, "chunk"], entries[name] = s.stats()["bsgs_steps"], s.stats()["entries"]
+            assert s.item_relations(it) == relations[name]
+            steps[name, "wave"] = s.stats()["bsgs_steps"]
+    assert relations["split"] == relations["unsplit"] and entries["split"] == entries["unsplit"]
+    for path in ("chunk", "wave"):
+        assert steps["split", path] < 0.55 * steps["unsplit", path]
+    # of two l of one size class the sieve keeps either one
+    assert abs(steps["split", "chunk"] - steps["split", "wave"]) < 0.01 * steps["split", "chunk"]
+
+
+@pytest.mark.parametrize("b,c,P0,width,N0,N1,mod,res", ITEMS)
+def test_given_primes_are_split_as_sieved_ones(mps_lib, oracle, b, c, P0, width, N0, N1, mod, res):
+    width = min(width, 1 << 22)
+    primes = oracle.primes(P0, P0 + width, 1 << 19)
+    it = mps_lib.make_item(b, c, P0, P0 + width, N0, N1, mod, res)
+    with mps_lib.Siever(0) as s:
+        want = s.chunk_relations(P0, P0 + width, it)
+        sieved = s.stats()
+        flags = s.filter(primes, it)
+        given = s.stats()
+    assert [p for p, f in zip(primes, flags) if f] == [r[0] for r in want]
+    assert given["entries"] == sieved["entries"]
+    assert abs(given["bsgs_steps"] - sieved["bsgs_steps"]) < 0.01 * sieved["bsgs_steps"]
