@@ -96,8 +96,8 @@ struct PrepArgs {
     const DevItem* items;
     Entry* ent;
     u64 ent_cap;               // < 2^32
-    SplitEvent* events;        // kSplitLists lists of ev_cap events each
-    u64 ev_cap;
+    SplitEvent* events;        // kSplitLists lists, ev_cap events each, ev_small those of the small l
+    u64 ev_cap, ev_small;
     u32 two_fields;            // 0: kSplitSizes lists only, shared by both arithmetics
     u32* big;                  // ent_cap indices: the entries k_bsgs solves
     RawRelation* rel;
@@ -111,13 +111,16 @@ struct PrepArgs {
 };
 // Entries for a range of that many odd numbers: the primes of any such range (the
 // first one holds the most: pi(2 odds) stays below this, by 2% at 2^24 .. 2^26).
-// 160 B an entry (Entry, events, BSGS list): 20 B an odd number, and 16 B more
+// 168 B an entry (Entry, events, BSGS list): 21 B an odd number, and 16 B more
 // for the survivors and their split primes.
 constexpr u64 entry_cap(u64 odds) { return odds / 8 + (1u << 17); }
-// Events a list needs for ent_cap entries (an entry has 0.7 small l on average,
-// and a chunk above 10^6 fills its entries to a third at most); a full list
-// loses splits, never relations.
+// Events of a size class's list and of a small-l list for ent_cap entries: a prime has
+// an l of a class with chance 1/4 at most (0.25 for 67 .. 251) and 0.72 small l on
+// average, so neither fills up unless the caller's own primes were chosen for it; a
+// full list loses splits, never relations.
 constexpr u64 split_event_cap(u64 ent_cap) { return ent_cap / 4; }
+constexpr u64 split_small_cap(u64 ent_cap) { return ent_cap / 4 * 3; }
+constexpr u64 split_events(u64 ev_cap, u64 ev_small) { return kSplitLists / kSplitSizes * (kSplitClasses * ev_cap + ev_small); }
 // Split primes to look for in the range of an item with K in-class exponents.
 u32 split_primes_for(u64 K);
 constexpr u64 kSievedPrimeBelow = (u64)kSieveMaxPrime * kSieveMaxPrime;

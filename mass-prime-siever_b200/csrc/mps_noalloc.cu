@@ -42,7 +42,9 @@ namespace {
 constexpr u64 kNoAllocMaxSpan = 1ull << 19;
 constexpr u64 kNoAllocEntries = 11ull << 12;         // more than the 43,390 primes below 2^19, the most a range holds
 constexpr u64 kNoAllocSurv = kNoAllocEntries;        // (the same bound holds for the sieve's survivors)
-constexpr u64 kNoAllocEvents = 1ull << 14;           // per split list (a full list loses splits, not relations)
+// Events of a size class's list and of the small-l list: mod 1 leaves 65% of the primes
+// below 2^19 as entries, 0.25 and 0.72 events each (a full list loses splits, not relations).
+constexpr u64 kNoAllocEvents = 5ull << 11, kNoAllocSmallEvents = 1ull << 15;
 constexpr u64 kNoAllocRelations = 1ull << 14;
 constexpr u32 kNoAllocMaxDevices = 64;
 
@@ -57,7 +59,7 @@ constexpr size_t kOffSurv = align256(kOffInv + kSievePrimes * sizeof(u64));
 constexpr size_t kOffSplit = align256(kOffSurv + kNoAllocSurv * sizeof(u64));
 constexpr size_t kOffEnt = align256(kOffSplit + kNoAllocSurv * sizeof(u64));
 constexpr size_t kOffEvents = align256(kOffEnt + kNoAllocEntries * sizeof(Entry));
-constexpr size_t kOffBig = align256(kOffEvents + kSplitSizes * kNoAllocEvents * sizeof(SplitEvent));
+constexpr size_t kOffBig = align256(kOffEvents + (kSplitClasses * kNoAllocEvents + kNoAllocSmallEvents) * sizeof(SplitEvent));
 constexpr size_t kNoAllocUsed = align256(kOffBig + kNoAllocEntries * sizeof(u32));
 constexpr size_t kNoAllocBytes = 8u << 20;
 static_assert(kNoAllocUsed <= kNoAllocBytes, "no-alloc scratch layout exceeds its array");
@@ -189,6 +191,7 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     pa.ent_cap = kNoAllocEntries;
     pa.events = (SplitEvent*)(base + kOffEvents);
     pa.ev_cap = kNoAllocEvents;
+    pa.ev_small = kNoAllocSmallEvents;
     pa.big = (u32*)(base + kOffBig);
     pa.rel = rel;
     pa.rel_cap = kNoAllocRelations;

@@ -42,3 +42,36 @@ def test_given_primes_are_split_as_sieved_ones(mps_lib, oracle, b, c, P0, width,
     assert [p for p, f in zip(primes, flags) if f] == [r[0] for r in want]
     assert given["entries"] == sieved["entries"]
     assert abs(given["bsgs_steps"] - sieved["bsgs_steps"]) < 0.01 * sieved["bsgs_steps"]
+
+
+def test_no_split_of_a_given_prime_is_lost(mps_lib, oracle):
+    """filter in a context whose buffers fit the list, all of whose primes are entries
+    (b = 2, c = -4: n = 2 solves every prime, N0 = 3 leaves it out): as many steps as
+    in a context with larger buffers."""
+    lo = 10**9
+    primes = oracle.primes(lo, lo + (1 << 21), 1 << 18)
+    it = mps_lib.make_item(2, -4, lo, lo + (1 << 21), 3, 5_000_003, 1, 0)
+    with mps_lib.Siever(0) as s:
+        s.filter(primes, it)
+        fitted = s.stats()
+        s.chunk_relations(lo, lo + 1000, it)                  # (a chunk's buffers are larger)
+        s.filter(primes, it)
+        large = s.stats()
+    assert fitted["entries"] == len(primes)
+    assert fitted["bsgs_steps"] == large["bsgs_steps"]
+
+
+def test_full_event_lists_lose_no_relation(mps_lib):
+    """70,000 primes p == 1 (mod 5 7 11 13 17 19): six small l each, eight times what the
+    list holds.  Flags and relations as without the split."""
+    step = 2 * 5 * 7 * 11 * 13 * 17 * 19
+    with mps_lib.Siever(0, class_modulus=144) as s:
+        cand = [1 + step * k for k in range(1000, 900_000)]
+        primes = [p for p, f in zip(cand, s.is_prime(cand)) if f][:70_000]
+        assert len(primes) == 70_000
+        it = mps_lib.make_item(3, 2, primes[0], primes[-1] + 1, 0, 10**7, 1, 0)
+        want = s.filter(primes, it)
+    assert 0 < sum(want) < 70_000
+    with mps_lib.Siever(0) as s:
+        for _ in range(2):
+            assert s.filter(primes, it) == want
