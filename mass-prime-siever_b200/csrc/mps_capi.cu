@@ -1467,8 +1467,10 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
         ba.tbits = tbits; ba.warps_per_block = warps; ba.persistent = 1; ba.chains = g.chains; ba.table_kind = g.kind;
         ba.load_shift = g.load_shift;
         ba.fill = g.fill;
-        ba.lanes = for_range(g, top + 1).lanes;
-        ba.max_p = top;
+        // (the arithmetic goes by this chunk's primes: one beyond 2^49 elsewhere in the list costs it nothing)
+        const u64 chunk_top = top < kFp64Limit || cnt == n ? top : *std::max_element(primes + off, primes + off + cnt);
+        ba.lanes = for_range(g, chunk_top + 1).lanes;
+        ba.max_p = chunk_top;
         OrderArgs oa{};
         oa.rel = c->d_rel; oa.rel_cap = c->rel_cap; oa.items = c->d_items; oa.tables = c->tables();
         CK(launch_prep(pa, c->d_ctr, grid_for(c, 4), c->num_sms, s), "prep launch");

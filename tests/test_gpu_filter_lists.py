@@ -20,3 +20,21 @@ def test_one_prime_many_times(siever, mps_lib, oracle):
     t0 = time.perf_counter()
     assert siever.filter([hit] * 100_000, it) == [1] * 100_000
     assert time.perf_counter() - t0 < 1.0
+
+
+def test_arithmetic_by_chunk(mps_lib, oracle):
+    """A list of two chunks, below and above 2^49: each runs as it does alone (with
+    four chains the two arithmetics' solves end after different step counts)."""
+    low = oracle.primes(10**9, 10**9 + 200_000, 1 << 16)[:4096]
+    high = oracle.primes(2**49, 2**49 + 20_000, 1 << 16)
+    it = mps_lib.make_item(3, 2, 10**9, 2**50, 0, 10**7, 1, 0)
+    with mps_lib.Siever(0, chunk_odds=4096, chains=4) as s:
+        flags, steps = [], 0
+        for part in (low, high):
+            flags += s.filter(part, it)
+            steps += s.stats()["bsgs_steps"]
+        assert s.filter(low + high, it) == flags
+        assert s.stats()["bsgs_steps"] == steps
+        # in one chunk: the same flags
+        mixed = low[:2000] + high + low[2000:3000]
+        assert s.filter(mixed, it) == flags[:2000] + flags[4096:] + flags[2000:3000]
