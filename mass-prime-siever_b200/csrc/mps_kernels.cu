@@ -704,7 +704,9 @@ __device__ __forceinline__ u32 inv_mod_small(u32 a, u32 m) {
     return (u32)(x < 0 ? x + (int)m : x);
 }
 
-// a / m and a % m for a < 2^24, 0 < m < 2^13 by single-precision division (off by one at most, set right).
+// a / m and a % m for a < 2^24, 0 < m < 2^13 and a quotient below 2^23, by single-precision
+// division: its error of 2 units in the last place is 1 at most there, so the quotient is
+// off by one at most, and set right.
 __device__ __forceinline__ u32 div_small(u32 a, u32 m, u32& rem) {
     int q = (int)__fdividef((float)a, (float)m), r = (int)a - q * (int)m;
     if (r < 0) {
@@ -748,7 +750,8 @@ __device__ __forceinline__ bool combine_class(u64 p, const DevItem& it, u32 d, u
         const u32 ch = mod_small24(div_small(cmd, h, rem), per);
         k0 = per == 1 ? 0u : mod_small24(wh * inv_mod_small(ch, per), per);
         if (k0 >= it.K) return false;
-        jcount = div_small((u32)it.K - k0 + per - 1, per, rem);   // K <= 10^7
+        const u32 left = (u32)it.K - k0;               // K <= 10^7: above 2^23 only when undivided
+        jcount = per == 1 ? left : div_small(left + per - 1, per, rem);
     } else {
         const u32 cmd = it.cmQ % d;
         const u32 want = (r + d - it.nsQ % d) % d;
