@@ -11,6 +11,9 @@
 
 #include "mps_common.cuh"
 
+#include <cmath>
+#include <cstring>
+
 namespace mps {
 
 struct Mont {
@@ -242,6 +245,26 @@ struct Fp64 {
         return r;
     }
 };
+
+// The hash of the baby-step tables for residues c < p < 2^49: the low mantissa word of
+// c k + 2^51, with c k < 2^50, so the sum lies in one binade, its unit 1/2, whatever c:
+// multiples of a power of two do not share their bits.  k is the golden ratio, or 2^19
+// times that for a launch whose primes lie below 2^30: with k = kHashK the word's top
+// bits are always 0 below 3 * 10^8 (at 10^6, 50 of the 16,384 fingerprints occurred, one
+// probe in 130 matched a wrong one, and k_bsgs took a third longer: 2^22 integers at
+// 10^7 with 10^7 exponents 0.32 ms, now 0.25).  k is a constant of the kernel: a k for each
+// prime, or one from the launch's arguments, takes registers that the solve with four
+// chains does not have (1% of k_bsgs at 10^12).
+__host__ __device__ __forceinline__ u32 fq_hash(double c, double k) {
+#ifdef __CUDA_ARCH__
+    return (u32)__double2loint(__fma_rn(c, k, 2251799813685248.0));
+#else
+    const double x = std::fma(c, k, 2251799813685248.0);
+    u64 w;
+    std::memcpy(&w, &x, sizeof w);
+    return (u32)w;
+#endif
+}
 
 // Plain modular product for moduli below 2^32 (small-prime paths).
 __device__ __forceinline__ u64 mulmod_small(u64 a, u64 b, u64 p) { return (a * b) % p; }

@@ -65,9 +65,10 @@ struct LaunchCfg {
     u32 lanes = 32;     // lanes per prime (table kind 2: 32, or groups of 16 / 8 for p < 2^49)
     u32 fill = kDefaultFill;           // table kinds 0 and 3: keys per word x 256, at most
     u32 scale = kDefaultBabyScale;     // baby steps: ceil(sqrt(j range)) x scale / 256
+    u32 low = 0;        // 1: the range's primes lie below kHashLow (for_range)
     bool operator==(const LaunchCfg& o) const {
         return kind == o.kind && load_shift == o.load_shift && chains == o.chains && warps == o.warps &&
-               seg_words == o.seg_words && lanes == o.lanes && fill == o.fill && scale == o.scale;
+               seg_words == o.seg_words && lanes == o.lanes && fill == o.fill && scale == o.scale && low == o.low;
     }
     bool operator!=(const LaunchCfg& o) const { return !(*this == o); }
 };
@@ -334,10 +335,11 @@ u32 launch_m_cap(const mps_ctx* c, const LaunchCfg& g, u32 tbits) {
     return std::max<u32>(1, std::min<u32>(std::min<u32>(holds, table_room(g, tbits)), kMaxBaby));
 }
 
-// Groups of lanes per prime run the FP64 solve only: a range that reaches
-// 2^49 runs a whole warp per prime.
+// The configuration for a range's primes.  Groups of lanes per prime run the FP64
+// solve only: a range that reaches 2^49 runs a whole warp per prime.
 LaunchCfg for_range(LaunchCfg g, u64 hi) {
     if (hi > kFp64Limit) g.lanes = 32;
+    g.low = hi <= kHashLow;
     return g;
 }
 
@@ -471,6 +473,7 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     ba.fill = g.fill;
     ba.load_shift = g.load_shift;
     ba.lanes = g.lanes;
+    ba.low = g.low;
     ba.max_p = hi;
 
     OrderArgs oa{};
@@ -638,7 +641,7 @@ int slot_enqueue(mps_ctx* c, WaveSlot& w, u32 tbits, const LaunchCfg& g, bool ca
     BsgsArgs ba{};
     ba.ent = w.d_ent; ba.big = w.d_big; ba.ent_cap = w.ent_cap; ba.rel = w.d_rel; ba.rel_cap = w.rel_cap; ba.tbits = tbits;
     ba.warps_per_block = warps; ba.persistent = 1; ba.chains = g.chains;
-    ba.table_kind = g.kind; ba.load_shift = g.load_shift; ba.lanes = g.lanes; ba.fill = g.fill;
+    ba.table_kind = g.kind; ba.load_shift = g.load_shift; ba.lanes = g.lanes; ba.fill = g.fill; ba.low = g.low;
     ba.max_p = 0;   // per-entry arithmetic
     OrderArgs oa{};
     oa.rel = w.d_rel; oa.rel_cap = w.rel_cap; oa.items = c->d_items; oa.tables = c->tables();
@@ -1470,6 +1473,7 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
         // (the arithmetic goes by this chunk's primes: one beyond 2^49 elsewhere in the list costs it nothing)
         const u64 chunk_top = top < kFp64Limit || cnt == n ? top : *std::max_element(primes + off, primes + off + cnt);
         ba.lanes = for_range(g, chunk_top + 1).lanes;
+        ba.low = chunk_top < kHashLow;
         ba.max_p = chunk_top;
         OrderArgs oa{};
         oa.rel = c->d_rel; oa.rel_cap = c->rel_cap; oa.items = c->d_items; oa.tables = c->tables();

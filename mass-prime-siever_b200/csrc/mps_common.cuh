@@ -23,6 +23,11 @@ constexpr u32 kSieveMaxPrime = 65521;
 // ones 64-bit Montgomery.
 constexpr u64 kFp64Limit = 1ull << 49;
 
+// The multiplier of the baby-step tables' hash (fq_hash), and that of a launch whose
+// primes all lie below kHashLow.
+constexpr double kHashK = 1.6180339887498949, kHashKLow = kHashK * 524288.0;
+constexpr u64 kHashLow = 1ull << 30;
+
 // Largest baby-step count of one prime (a table of 2^13 slots at load 1/2).
 constexpr u32 kMaxBaby = 4096;
 // Measured on the B200 (C2 and C3 slices): a baby step (hash, insert) costs

@@ -1930,7 +1930,7 @@ __device__ u64 solve_fp64(const Solve& e, u32* tab, u32 tbits, u64* steps_out) {
 // The step is bound by instruction issue and the ALU pipe, with the FP64 pipe
 // a third busy, so its work sits where there is room.  The hash is one FP64
 // multiply-add of the canonical residue c (fq_hash): the low mantissa word of
-// c K + 2^51, 32 mixed bits of the fixed-point product.  Its bits 3 .. tw + 2
+// c k + 2^51, 32 mixed bits of the fixed-point product.  Its bits 3 .. tw + 2
 // are the home word's byte offset as they stand and its bits 16 .. 29 the
 // fingerprint.  The four halves of a word are compared with the fingerprint as
 // half-precision numbers, two instructions of the FMA pipe: a used half is a
@@ -1958,11 +1958,6 @@ __device__ u64 solve_fp64(const Solve& e, u32* tab, u32 tbits, u64* steps_out) {
 constexpr u64 kQValid = 0x8000800080008000ull;
 constexpr u32 kQOvf = 0x4000u;
 
-// c in [0, p), p < 2^49: c K < 2^50, so the sum lies in [2^51, 2^52), its unit
-// 1/2, whatever c: multiples of a power of two do not share their bits.
-__device__ __forceinline__ u32 fq_hash(double c) {
-    return (u32)__double2loint(__fma_rn(c, 1.6180339887498949, 2251799813685248.0));
-}
 __device__ __forceinline__ u32 fq_fingerprints(u32 h) {        // in both halves
     return (__byte_perm(h, h, 0x3232) & 0x3FFF3FFFu) | 0x80008000u;
 }
@@ -2102,7 +2097,7 @@ __device__ __forceinline__ SolveF solve_f(const Solve& e, u32 tbits, u32 fill) {
 // after the words) instead of one compare-and-swap each (table kind 0); the
 // words and the probes are the same.  The words are 2^tw of the launch's
 // 2^(tbits-1).
-template <int CH, bool WI>
+template <int CH, bool WI, bool LOW>
 __device__ u64 solve_fp64q(const SolveF& e, unsigned long long* tab, u32 tbits, u64* steps_out) {
     const u32 lane = threadIdx.x & 31, lo = lane & 15;
     const Fp64 f = e.f;
@@ -2154,7 +2149,7 @@ __device__ u64 solve_fp64q(const SolveF& e, unsigned long long* tab, u32 tbits, 
         u32 h[CH], want = 0;
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
-            h[c] = fq_hash(f.canon(bx[c]));
+            h[c] = fq_hash(f.canon(bx[c]), LOW ? kHashKLow : kHashK);
             bx[c] = f.mul(bx[c], Bstep);               // the next value, independent of the insert
             if (base + 32 * c + lane < m) want |= 1u << c;
         }
@@ -2179,7 +2174,7 @@ __device__ u64 solve_fp64q(const SolveF& e, unsigned long long* tab, u32 tbits, 
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             cv[c] = f.canon(gx[c]);
-            hs[c] = fq_hash(cv[c]);
+            hs[c] = fq_hash(cv[c], LOW ? kHashKLow : kHashK);
             nx[c] = f.mul(gx[c], Gstep);                  // the next value, independent of the probe
             const uint2 w = *reinterpret_cast<const uint2*>(bytes + (hs[c] & mask8));
             const u32 rep = fq_fingerprints(hs[c]);
@@ -2394,12 +2389,12 @@ __device__ u64 solve_fp64h(const Solve& e, unsigned short* tab, u32 tbits, u32 l
     return best < e.jcount ? best : ~0ull;
 }
 
-template <int CH, int QT>
+template <int CH, int QT, bool LOW>
 __device__ __forceinline__ u64 solve_any(const Solve& e, void* tab, u32 tbits, u32 load_shift, u32 fill, u64* steps) {
     if (CH == 0 || e.p >= kFp64Limit) return solve_entry<FieldM>(e, (unsigned short*)tab, tbits + 1, steps);
-    if (QT == 0) return solve_fp64q<CH ? CH : 1, false>(solve_f(e, tbits, fill), (unsigned long long*)tab, tbits, steps);
+    if (QT == 0) return solve_fp64q<CH ? CH : 1, false, LOW>(solve_f(e, tbits, fill), (unsigned long long*)tab, tbits, steps);
     if (QT == 2) return solve_fp64h<CH ? CH : 1>(e, (unsigned short*)tab, tbits, load_shift, steps);
-    if (QT == 3) return solve_fp64q<CH ? CH : 1, true>(solve_f(e, tbits, fill), (unsigned long long*)tab, tbits, steps);
+    if (QT == 3) return solve_fp64q<CH ? CH : 1, true, LOW>(solve_f(e, tbits, fill), (unsigned long long*)tab, tbits, steps);
     return solve_fp64<CH ? CH : 1>(e, (u32*)tab, tbits, steps);
 }
 
@@ -2421,8 +2416,9 @@ __device__ __forceinline__ Solve solve_of(const Entry& g) {
 }
 
 // CH > 0: every entry has p < 2^49 (FP64 solve with CH chains per lane);
-// CH == 0: any p (integer Montgomery solve).
-template <int CH, int QT>
+// CH == 0: any p (integer Montgomery solve).  LOW: every p is below
+// kHashLow.
+template <int CH, int QT, bool LOW = false>
 __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counters* ctr) {
     extern __shared__ __align__(16) u32 smem32[];
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2474,7 +2470,7 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counter
                 e.m = m;
                 e.G = (u32)gt;
                 e.tw = min((u32)(gt >> 32), a.tbits - 1);
-                j = solve_fp64q<CH ? CH : 1, QT == 3>(e, (unsigned long long*)tab, a.tbits, &steps);
+                j = solve_fp64q<CH ? CH : 1, QT == 3, LOW>(e, (unsigned long long*)tab, a.tbits, &steps);
             } else {
                 Solve e;
                 e.p = p;
@@ -2484,7 +2480,7 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counter
                 e.Bm = __shfl_sync(FULL, mine, 4);
                 e.jcount = (u32)jm;
                 e.m = m;
-                j = solve_any<CH, QT>(e, tab, a.tbits, a.load_shift, a.fill, &steps);
+                j = solve_any<CH, QT, LOW>(e, tab, a.tbits, a.load_shift, a.fill, &steps);
             }
             if (lane == 0) {
                 if (j != ~0ull) {
@@ -2509,7 +2505,7 @@ __global__ void __launch_bounds__(256, MPS_BSGS_MINB) k_bsgs(BsgsArgs a, Counter
             return;
         }
         u64 steps = 0;
-        const u64 j = solve_any<CH, QT>(e, tab, a.tbits, a.load_shift, a.fill, &steps);
+        const u64 j = solve_any<CH, QT, LOW>(e, tab, a.tbits, a.load_shift, a.fill, &steps);
         if (lane == 0) {
             if (j != ~0ull) emit_relation(e.p, g.n_first + j * g.L, 0, g.item, a.rel, a.rel_cap, ctr);
             atomicAdd(&ctr->steps, (unsigned long long)((steps & 0xFFFFFFFFull) + (steps >> 32)));
@@ -3104,11 +3100,11 @@ __global__ void k_bsgs_direct(const u64* cases, u64* j_out, u64 count, u32 tbits
         M.init(p);
         const u64 rr = M.r2();
         e.Bm = M.from_mont(M.pow(M.to_mont(e.B, rr), m));
-        if (e.p >= kFp64Limit) result = solve_any<0, 0>(e, smem32, tbits, kDefaultLoadShift, kDefaultFill, nullptr);
-        else if (table_kind == 0) result = solve_any<2, 0>(e, smem32, tbits, kDefaultLoadShift, kDefaultFill, nullptr);
-        else if (table_kind == 2) result = solve_any<2, 2>(e, smem32, tbits, kDefaultLoadShift, kDefaultFill, nullptr);
-        else if (table_kind == 3) result = solve_any<2, 3>(e, smem32, tbits, 0, kDefaultFill, nullptr);
-        else result = solve_any<2, 1>(e, smem32, tbits, kDefaultLoadShift, kDefaultFill, nullptr);
+        if (e.p >= kFp64Limit) result = solve_any<0, 0, false>(e, smem32, tbits, kDefaultLoadShift, kDefaultFill, nullptr);
+        else if (table_kind == 0) result = solve_any<2, 0, false>(e, smem32, tbits, kDefaultLoadShift, kDefaultFill, nullptr);
+        else if (table_kind == 2) result = solve_any<2, 2, false>(e, smem32, tbits, kDefaultLoadShift, kDefaultFill, nullptr);
+        else if (table_kind == 3) result = solve_any<2, 3, false>(e, smem32, tbits, 0, kDefaultFill, nullptr);
+        else result = solve_any<2, 1, false>(e, smem32, tbits, kDefaultLoadShift, kDefaultFill, nullptr);
     }
     if (threadIdx.x == 0) j_out[idx] = result;
 }
@@ -3196,8 +3192,9 @@ cudaError_t bsgs_reserve_smem(size_t smem) {
     if (smem <= done[dev]) return cudaSuccess;
     for (auto kern : {k_bsgs<0, 0>, k_bsgs<1, 0>, k_bsgs<2, 0>, k_bsgs<4, 0>, k_bsgs<1, 1>, k_bsgs<2, 1>,
                       k_bsgs<4, 1>, k_bsgs<1, 2>, k_bsgs<2, 2>, k_bsgs<4, 2>, k_bsgs<1, 3>, k_bsgs<2, 3>,
-                      k_bsgs<4, 3>, k_bsgs_groups<8, 1>,
-                      k_bsgs_groups<8, 2>, k_bsgs_groups<16, 1>, k_bsgs_groups<16, 2>}) {
+                      k_bsgs<4, 3>, k_bsgs<1, 0, true>, k_bsgs<2, 0, true>, k_bsgs<4, 0, true>, k_bsgs<1, 3, true>,
+                      k_bsgs<2, 3, true>, k_bsgs<4, 3, true>, k_bsgs_groups<8, 1>, k_bsgs_groups<8, 2>,
+                      k_bsgs_groups<16, 1>, k_bsgs_groups<16, 2>}) {
         err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return err;
     }
@@ -3221,9 +3218,9 @@ cudaError_t launch_bsgs(const BsgsArgs& a, Counters* ctr, int grid, cudaStream_t
         return a.chains == 1 ? go(k_bsgs_groups<16, 1>) : go(k_bsgs_groups<16, 2>);
     }
     if (a.table_kind == 3) {
-        if (a.chains == 4) return go(k_bsgs<4, 3>);
-        if (a.chains == 1) return go(k_bsgs<1, 3>);
-        return go(k_bsgs<2, 3>);
+        if (a.chains == 4) return a.low ? go(k_bsgs<4, 3, true>) : go(k_bsgs<4, 3>);
+        if (a.chains == 1) return a.low ? go(k_bsgs<1, 3, true>) : go(k_bsgs<1, 3>);
+        return a.low ? go(k_bsgs<2, 3, true>) : go(k_bsgs<2, 3>);
     }
     if (a.table_kind == 2) {
         if (a.chains == 4) return go(k_bsgs<4, 2>);
@@ -3235,9 +3232,9 @@ cudaError_t launch_bsgs(const BsgsArgs& a, Counters* ctr, int grid, cudaStream_t
         if (a.chains == 1) return go(k_bsgs<1, 1>);
         return go(k_bsgs<2, 1>);
     }
-    if (a.chains == 4) return go(k_bsgs<4, 0>);
-    if (a.chains == 1) return go(k_bsgs<1, 0>);
-    return go(k_bsgs<2, 0>);
+    if (a.chains == 4) return a.low ? go(k_bsgs<4, 0, true>) : go(k_bsgs<4, 0>);
+    if (a.chains == 1) return a.low ? go(k_bsgs<1, 0, true>) : go(k_bsgs<1, 0>);
+    return a.low ? go(k_bsgs<2, 0, true>) : go(k_bsgs<2, 0>);
 }
 
 cudaError_t launch_order(const OrderArgs& a, Counters* ctr, int grid, cudaStream_t s) {

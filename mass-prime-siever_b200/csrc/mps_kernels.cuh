@@ -143,6 +143,7 @@ struct BsgsArgs {
     u32 load_shift;            // table kind 2: at most 2^-load_shift of a prime's slots are used
     u32 lanes;                 // table kind 2: lanes per prime, 32 (a warp) or 16 / 8 (groups; every
                                // entry must have p < 2^49, max_p > 0 and < 2^49 or the caller's guarantee)
+    u32 low;                   // 1: every prime is below kHashLow (table kinds 0 and 3: kHashKLow instead of kHashK)
     u32 fill;                  // table kinds 0 and 3: a prime's table has at least m * 256 / fill words
                                // (1..256; 0 counts as 256), within the launch's 2^(tbits-1)
 };

@@ -213,6 +213,7 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     ba.table_kind = 0;
     ba.load_shift = kDefaultLoadShift;
     ba.fill = kDefaultFill;
+    ba.low = hi <= kHashLow;
     ba.max_p = hi;
     OrderArgs oa{};
     oa.rel = rel;
