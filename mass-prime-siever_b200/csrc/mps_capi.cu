@@ -212,7 +212,7 @@ int alloc_entries(mps_ctx* c, Entry** ent, SplitEvent** events, u32** big, u64* 
     *big = nullptr;
     *cap = 0;
     CK(cudaMalloc((void**)ent, need * sizeof(Entry)), "entry buffer");
-    CK(cudaMalloc((void**)events, split_events(split_event_cap(need), split_small_cap(need)) * sizeof(SplitEvent)),
+    CK(cudaMalloc((void**)events, split_events(split_event_cap(need), split_small_cap(need), 2) * sizeof(SplitEvent)),
        "split events");
     CK(cudaMalloc((void**)big, need * sizeof(u32)), "BSGS list");
     *cap = need;
@@ -448,8 +448,7 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     pa.items = c->d_items;
     pa.ent = c->d_ent;
     pa.ent_cap = c->ent_cap;
-    pa.events = c->d_events;
-    pa.ev_cap = split_event_cap(c->ent_cap); pa.ev_small = split_small_cap(c->ent_cap); pa.two_fields = 1;
+    set_event_lists(&pa, c->d_events, split_event_cap(c->ent_cap), split_small_cap(c->ent_cap), 2);
     pa.big = c->d_big;
     pa.rel = c->d_rel;
     pa.rel_cap = c->rel_cap;
@@ -630,8 +629,8 @@ int slot_enqueue(mps_ctx* c, WaveSlot& w, u32 tbits, const LaunchCfg& g, bool ca
     pa.surv = w.d_surv; pa.surv_cap = w.surv_cap; pa.surv_item = w.d_surv_item; pa.item0 = 0;
     pa.surv_split = w.d_surv_split; pa.tables = c->tables();
     pa.items = c->d_items; pa.ent = w.d_ent; pa.ent_cap = w.ent_cap; pa.rel = w.d_rel; pa.rel_cap = w.rel_cap;
-    pa.events = w.d_events; pa.ev_cap = split_event_cap(w.ent_cap); pa.ev_small = split_small_cap(w.ent_cap);
-    pa.two_fields = 1; pa.big = w.d_big;
+    set_event_lists(&pa, w.d_events, split_event_cap(w.ent_cap), split_small_cap(w.ent_cap), 2);
+    pa.big = w.d_big;
     pa.full_mr = c->tun.full_mr;
     pa.m_cap = launch_m_cap(c, g, tbits);
     pa.m_round = g.lanes * g.chains;
@@ -1459,8 +1458,8 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
         pa.surv = c->d_surv; pa.surv_cap = c->surv_cap; pa.item0 = 0; pa.items = c->d_items;
         pa.tables = c->tables();                        // no surv_split: the primes did not come from the sieve
         pa.ent = c->d_ent; pa.ent_cap = c->ent_cap; pa.rel = c->d_rel; pa.rel_cap = c->rel_cap; pa.full_mr = c->tun.full_mr;
-        pa.events = c->d_events; pa.ev_cap = split_event_cap(c->ent_cap); pa.ev_small = split_small_cap(c->ent_cap);
-        pa.two_fields = 1; pa.big = c->d_big;
+        set_event_lists(&pa, c->d_events, split_event_cap(c->ent_cap), split_small_cap(c->ent_cap), 2);
+        pa.big = c->d_big;
         pa.m_cap = launch_m_cap(c, g, tbits);
         pa.m_round = g.lanes * g.chains;
         pa.tbits = tbits;

@@ -795,12 +795,6 @@ __host__ __device__ constexpr u32 split_limit(u32 J) {
 }
 u32 split_primes_for(u64 K) { return split_limit((u32)min(K, (u64)~0u)); }
 
-// The split events' lists: by size (slot_list), those of the second arithmetic after those of the first.
-__device__ __forceinline__ u64 list_cap(const PrepArgs& a, u32 size) { return size == kSplitClasses ? a.ev_small : a.ev_cap; }
-__device__ __forceinline__ u64 list_base(const PrepArgs& a, u32 size, bool second) {
-    return size * a.ev_cap + (second ? kSplitClasses * a.ev_cap + a.ev_small : 0);
-}
-
 // Queues the split events of the warp's entries (idx, lanes with ok) in slots
 // S0 .. S1 - 1: k[slot] is the index + 1 of the entry's l, 0 for none.  One
 // atomic per list and warp; a full list drops the event.
@@ -827,8 +821,9 @@ __device__ __forceinline__ void queue_events(bool ok, u64 idx, u64 p, const u32 
     for (u32 s = S0; s < S1; ++s) {
         const u64 at = __shfl_sync(FULL, at0, slot_list(s) + field) + pos[s];
         if (!ok) continue;
-        const bool in = k[s] != 0 && at < list_cap(a, slot_list(s));
-        if (in) a.events[list_base(a, slot_list(s), field != 0) + at] = SplitEvent{(u32)idx, (k[s] - 1) << 16 | s};
+        const bool in = k[s] != 0 && at < (s < kSplitClasses ? a.ev_cap : a.ev_small);
+        const u32 list = field ? a.ev_at[slot_list(s) + kSplitSizes] : a.ev_at[slot_list(s)];
+        if (in) a.events[list + (u32)at] = SplitEvent{(u32)idx, (k[s] - 1) << 16 | s};
         a.ent[idx].ev[s] = in ? kEvQueued | kEvUnknown : 0u;
         if (s < kSplitClasses) a.ent[idx].k[s] = (unsigned short)(k[s] - 1);
     }
@@ -1318,7 +1313,8 @@ __global__ void __launch_bounds__(256, 4) k_dlog(PrepArgs a, Counters* ctr) {
     u64 count[kSplitLists], total = 0;
 #pragma unroll
     for (u32 i = 0; i < kSplitLists; ++i) {
-        count[i] = min((u64)*(volatile unsigned long long*)&ctr->events[order[i]], list_cap(a, order[i] % kSplitSizes));
+        count[i] = min((u64)*(volatile unsigned long long*)&ctr->events[order[i]],
+                       (u64)(order[i] % kSplitSizes == kSplitClasses ? a.ev_small : a.ev_cap));
         total += (count[i] + 31) / 32;
     }
     // the first unit of a warp is fixed, block by block, so that the longest walks
@@ -1334,7 +1330,7 @@ __global__ void __launch_bounds__(256, 4) k_dlog(PrepArgs a, Counters* ctr) {
         for (u32 i = 0; i < kSplitLists; ++i) {
             const u64 units = (count[i] + 31) / 32;
             if (!placed && k < units) {
-                idx = list_base(a, order[i] % kSplitSizes, order[i] >= kSplitSizes) + k * 32 + lane;
+                idx = a.ev_at[order[i]] + k * 32 + lane;
                 live = k * 32 + lane < count[i];
                 large = i < 4;                         // l > 256
                 placed = true;

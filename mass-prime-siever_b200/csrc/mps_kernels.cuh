@@ -96,8 +96,9 @@ struct PrepArgs {
     const DevItem* items;
     Entry* ent;
     u64 ent_cap;               // < 2^32
-    SplitEvent* events;        // kSplitLists lists, ev_cap events each, ev_small those of the small l
-    u64 ev_cap, ev_small;
+    SplitEvent* events;        // the lists of split events (set_event_lists)
+    u32 ev_at[kSplitLists];    //   the place of each
+    u32 ev_cap, ev_small;      //   events of a size class's list, and of a small-l list
     u32 two_fields;            // 0: kSplitSizes lists only, shared by both arithmetics
     u32* big;                  // ent_cap indices: the entries k_bsgs solves
     RawRelation* rel;
@@ -120,7 +121,16 @@ constexpr u64 entry_cap(u64 odds) { return odds / 8 + (1u << 17); }
 // full list loses splits, never relations.
 constexpr u64 split_event_cap(u64 ent_cap) { return ent_cap / 4; }
 constexpr u64 split_small_cap(u64 ent_cap) { return ent_cap / 4 * 3; }
-constexpr u64 split_events(u64 ev_cap, u64 ev_small) { return kSplitLists / kSplitSizes * (kSplitClasses * ev_cap + ev_small); }
+constexpr u64 split_events(u64 ev_cap, u64 ev_small, u32 fields) { return fields * (kSplitClasses * ev_cap + ev_small); }
+// Lays the lists out in events (split_events of them, below 2^32): the sizes' lists of one arithmetic, then of the other.
+inline void set_event_lists(PrepArgs* a, SplitEvent* events, u64 ev_cap, u64 ev_small, u32 fields) {
+    a->events = events;
+    a->ev_cap = (u32)ev_cap;
+    a->ev_small = (u32)ev_small;
+    a->two_fields = fields == 2;
+    for (u32 c = 0; c < kSplitLists; ++c)
+        a->ev_at[c] = (u32)(c % kSplitSizes * ev_cap + c / kSplitSizes % fields * (kSplitClasses * ev_cap + ev_small));
+}
 // Split primes to look for in the range of an item with K in-class exponents.
 u32 split_primes_for(u64 K);
 constexpr u64 kSievedPrimeBelow = (u64)kSieveMaxPrime * kSieveMaxPrime;

@@ -59,7 +59,7 @@ constexpr size_t kOffSurv = align256(kOffInv + kSievePrimes * sizeof(u64));
 constexpr size_t kOffSplit = align256(kOffSurv + kNoAllocSurv * sizeof(u64));
 constexpr size_t kOffEnt = align256(kOffSplit + kNoAllocSurv * sizeof(u64));
 constexpr size_t kOffEvents = align256(kOffEnt + kNoAllocEntries * sizeof(Entry));
-constexpr size_t kOffBig = align256(kOffEvents + (kSplitClasses * kNoAllocEvents + kNoAllocSmallEvents) * sizeof(SplitEvent));
+constexpr size_t kOffBig = align256(kOffEvents + split_events(kNoAllocEvents, kNoAllocSmallEvents, 1) * sizeof(SplitEvent));
 constexpr size_t kNoAllocUsed = align256(kOffBig + kNoAllocEntries * sizeof(u32));
 constexpr size_t kNoAllocBytes = 8u << 20;
 static_assert(kNoAllocUsed <= kNoAllocBytes, "no-alloc scratch layout exceeds its array");
@@ -189,9 +189,7 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     pa.items = ditem;
     pa.ent = ent;
     pa.ent_cap = kNoAllocEntries;
-    pa.events = (SplitEvent*)(base + kOffEvents);
-    pa.ev_cap = kNoAllocEvents;
-    pa.ev_small = kNoAllocSmallEvents;
+    set_event_lists(&pa, (SplitEvent*)(base + kOffEvents), kNoAllocEvents, kNoAllocSmallEvents, 1);
     pa.big = (u32*)(base + kOffBig);
     pa.rel = rel;
     pa.rel_cap = kNoAllocRelations;
