@@ -78,7 +78,7 @@ __device__ __forceinline__ void emit_relation(u64 p, u64 M, u64 q, u32 item, Raw
 // -------------------------------------------------------------- the sieve --
 
 // A segment is W words of shared-memory bitmap (W * 32 odd numbers); W is a
-// template parameter (1024, 2048 or 4096 words: 4, 8 or 16 KB), chosen per
+// template parameter (256, 512, 1024, 2048 or 4096 words: 1 .. 16 KB), chosen per
 // launch.  kSegWords is the default.
 constexpr u32 kSegWords = 2048;
 constexpr u32 kSieveThreads = 256;
@@ -3124,14 +3124,9 @@ size_t bsgs_smem_bytes(u32 tbits, u32 warps_per_block, u32 table_kind) {
 
 bool valid_seg_words(u32 seg_words) { return seg_words == 1024 || seg_words == 2048 || seg_words == 4096; }
 
-// The segment size of one range: halved (down to 256 words) while the range
-// has fewer segments than kFewSegs, so that a small range reaches every SM
-// (2^20 integers at 10^9: 8 blocks, 40 us; now 64 blocks, 15 us.  Switching at
-// 296 segments instead costs 2^24 integers 48 us against 40: a segment has the
-// same set-up for its 6,541 primes whatever its length).
-constexpr u64 kFewSegs = 148;
+// The segment size of one range.
 u32 range_seg_words(u32 seg_words, u64 n_odds) {
-    while (seg_words > 256 && n_odds < kFewSegs * seg_words * 32) seg_words /= 2;
+    while (seg_words > kLeastSegWords && n_odds < kFewSegs * seg_words * 32) seg_words /= 2;
     return seg_words;
 }
 
@@ -3158,11 +3153,18 @@ cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, const SurvOut
 
 cudaError_t launch_sieve_wave(const WaveDesc* w, const SieveTables& t, const SurvOut& o, Counters* ctr, int grid,
                               cudaStream_t s, u32 seg_words) {
-    if (!valid_seg_words(seg_words)) return cudaErrorInvalidValue;
-    if (seg_words == 1024) k_sieve_wave<1024><<<grid, kSieveThreads, 0, s>>>(w, t, o, ctr);
-    else if (seg_words == 4096) k_sieve_wave<4096><<<grid, kSieveThreads, 0, s>>>(w, t, o, ctr);
-    else k_sieve_wave<2048><<<grid, kSieveThreads, 0, s>>>(w, t, o, ctr);
-    return cudaGetLastError();
+    auto go = [&](auto kern) {
+        kern<<<grid, kSieveThreads, 0, s>>>(w, t, o, ctr);
+        return cudaGetLastError();
+    };
+    switch (seg_words) {
+        case 256: return go(k_sieve_wave<256>);
+        case 512: return go(k_sieve_wave<512>);
+        case 1024: return go(k_sieve_wave<1024>);
+        case 2048: return go(k_sieve_wave<2048>);
+        case 4096: return go(k_sieve_wave<4096>);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 cudaError_t launch_prep(const PrepArgs& a, Counters* ctr, int grid, int num_sms, cudaStream_t s) {

@@ -35,7 +35,13 @@ struct SurvOut {
     u64 cap;
 };
 
-// seg_words: segment bitmap words (1024, 2048 or 4096; 32 odd numbers each)
+// seg_words: segment bitmap words (1024, 2048 or 4096; 32 odd numbers each).  A range or
+// wave of fewer than kFewSegs segments is cut into smaller ones, down to kLeastSegWords
+// (2^20 integers at 10^9 as a chunk: 8 blocks, 40 us of sieve; now 64 blocks, 15 us.
+// Switching at 296 segments instead costs 2^24 integers 48 us against 40: a segment has
+// the same set-up for its 6,541 primes whatever its length).
+constexpr u64 kFewSegs = 148;
+constexpr u32 kLeastSegWords = 256;
 constexpr u32 kDefaultSegWords = 2048;
 cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, const SurvOut& o, Counters* ctr, cudaStream_t s,
                          u32 seg_words = kDefaultSegWords);
@@ -78,7 +84,8 @@ cudaError_t launch_commit(const WaveDesc* w, const RawRelation* rel, const Count
 // A run of an overflowed wave, redone on the host path: p_done = max(p_done, hi),
 // its n relations rel[0..n) appended to the item's state.
 cudaError_t launch_state_add(ItemState* st, u32 item, u64 hi, const RawRelation* rel, u64 n, cudaStream_t s);
-// The wave's runs' seg_begin must count segments of seg_words * 32 odd numbers.
+// The wave's runs' seg_begin must count segments of seg_words * 32 odd numbers (seg_words
+// 256, 512, 1024, 2048 or 4096).
 cudaError_t launch_sieve_wave(const WaveDesc* w, const SieveTables& t, const SurvOut& o, Counters* ctr, int grid,
                               cudaStream_t s, u32 seg_words = kDefaultSegWords);
 
