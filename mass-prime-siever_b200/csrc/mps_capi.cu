@@ -344,11 +344,11 @@ LaunchCfg for_range(LaunchCfg g, u64 hi) {
 }
 
 // The device constants of an item (mps_item.cuh), with this context's split
-// modulus, the item's BSGS configuration (tuned or default) and its
+// modulus (or class_modulus), the item's BSGS configuration (tuned or default) and its
 // baby-step sizing.
-int make_dev_item(mps_ctx* c, const mps_item* it, u32 index, DevItem* d, LaunchCfg* cfg = nullptr) {
+int make_dev_item(mps_ctx* c, const mps_item* it, u32 index, DevItem* d, LaunchCfg* cfg = nullptr, u32 class_modulus = 0) {
     const char* why = "";
-    if (int r = item_constants(it, c->tun.class_modulus, index, d, &why)) return fail(c, r, why);
+    if (int r = item_constants(it, class_modulus ? class_modulus : c->tun.class_modulus, index, d, &why)) return fail(c, r, why);
     const LaunchCfg g = cfg_for(c, d->K, d->cm, it->P0);
     u32 tb = 0, mb = 0;
     table_for(c, g, d->K, &tb, &mb);
@@ -443,6 +443,7 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     pa.surv_cap = c->surv_cap;
     pa.surv_item = nullptr;
     pa.surv_split = c->d_surv_split;
+    pa.split = sa.n_split != 0;
     pa.tables = c->tables();
     pa.item0 = item;
     pa.items = c->d_items;
@@ -520,7 +521,7 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     CK(cudaStreamSynchronize(s), "chunk");
     c->ended = true;
     if (int r = add_stage_times(c, c->evk, c->tun.plain != 0)) return r;
-    c->stats.kernel_launches += 3 + kPrepLaunches;
+    c->stats.kernel_launches += 3 + prep_launches(pa.split, true);
     const Counters h = *c->h_ctr;
     if (h.status & (kStatusSurvivorOverflow | kStatusEntryOverflow)) {
         // a denser range than the buffers were sized for: halve the chunk
@@ -627,7 +628,7 @@ int slot_enqueue(mps_ctx* c, WaveSlot& w, u32 tbits, const LaunchCfg& g, bool ca
     const u32 warps = g.warps;
     PrepArgs pa{};
     pa.surv = w.d_surv; pa.surv_cap = w.surv_cap; pa.surv_item = w.d_surv_item; pa.item0 = 0;
-    pa.surv_split = w.d_surv_split; pa.tables = c->tables();
+    pa.surv_split = w.d_surv_split; pa.split = c->tun.class_modulus == 0; pa.tables = c->tables();
     pa.items = c->d_items; pa.ent = w.d_ent; pa.ent_cap = w.ent_cap; pa.rel = w.d_rel; pa.rel_cap = w.rel_cap;
     set_event_lists(&pa, w.d_events, split_event_cap(w.ent_cap), split_small_cap(w.ent_cap), 2);
     pa.big = w.d_big;
@@ -748,7 +749,7 @@ int slot_finish(mps_ctx* c, WaveSlot& w, std::vector<RawRelation>& out) {
     CK(cudaStreamSynchronize(w.stream), "wave");
     const Counters h = *w.h_ctr;
     if (int r = add_stage_times(c, w.evk)) return r;
-    c->stats.kernel_launches += 4 + kPrepLaunches;
+    c->stats.kernel_launches += 4 + prep_launches(c->tun.class_modulus == 0, true);
     if (h.status & kStatusOrderFailed) return fail(c, MPS_E_CUDA, "order computation did not factor p - 1");
     if (h.status & kStatusBadLaunch) return fail(c, MPS_E_CUDA, "a BSGS entry did not fit the launch's tables");
     if (h.status & (kStatusSurvivorOverflow | kStatusEntryOverflow | kStatusRelationOverflow)) {
@@ -1446,11 +1447,29 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
     }
     if (top >= kTwo62) return fail(c, MPS_E_RANGE, "primes must be below 2^62");
     begin_call(c);
-    if (int r = upload_items(c, &d, 1, false)) return r;
     const u64 chunk = c->tun.chunk_odds;
     std::vector<RawRelation> rel;
+    u64 item_Q = 0;                                     // the item on the device: its split modulus,
+    int item_few = -1;                                  // and whether that is its whole split
     for (size_t off = 0; off < n; off += chunk) {
         const u64 cnt = std::min<u64>(chunk, n - off);
+        // (the arithmetic goes by this chunk's primes: one beyond 2^49 elsewhere in the list costs it nothing)
+        const u64 chunk_top = top < kFp64Limit || cnt == n ? top : *std::max_element(primes + off, primes + off + cnt);
+        const bool low = chunk_top < kFp64Limit;
+        // Few primes are solved side by side, and k_split and k_dlog would take longer than the
+        // steps that they save: lists of 1,000 primes 0.12 .. 0.15 ms with them and 0.08 .. 0.11
+        // without, of 16,000 0.15 .. 0.27 and 0.12 .. 0.27, of 32,000 with 10^7 exponents 0.32
+        // and 0.36.  From 2^49 on a step costs more: 8,000 primes take the same either way, if
+        // the power split then takes 5 .. 19 over (10 primes: 0.18 ms without those, 0.12 with).
+        const bool few = c->tun.class_modulus == 0 && cnt < (low ? 16384u : 8192u);
+        const u64 Q = few ? low ? split_modulus(0, d.cm) : split_modulus_alone(d.cm) : split_modulus(c->tun.class_modulus, d.cm);
+        if (few != item_few || Q != item_Q) {
+            if (int r = make_dev_item(c, item, 0, &d, &g, few ? (u32)Q : 0)) return r;
+            if (split_for(c, d.K) == 0) d.split_more = 0;
+            if (int r = upload_items(c, &d, 1, false)) return r;
+            item_Q = Q;
+            item_few = few;
+        }
         if (int r = ensure(c, &c->d_surv, &c->surv_cap, std::max<u64>(cnt + 16, chunk + 16), "survivor buffer")) return r;
         if (int r = ensure_entries(c, std::max<u64>(cnt, 1 << 16))) return r;
         if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
@@ -1468,6 +1487,7 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
         PrepArgs pa{};
         pa.surv = c->d_surv; pa.surv_cap = c->surv_cap; pa.item0 = 0; pa.items = c->d_items;
         pa.tables = c->tables();                        // no surv_split: the primes did not come from the sieve
+        pa.split = d.split_more;
         pa.ent = c->d_ent; pa.ent_cap = c->ent_cap; pa.rel = c->d_rel; pa.rel_cap = c->rel_cap; pa.full_mr = c->tun.full_mr;
         set_event_lists(&pa, c->d_events, split_event_cap(c->ent_cap), split_small_cap(c->ent_cap), 2);
         pa.big = c->d_big;
@@ -1480,8 +1500,6 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
         ba.tbits = tbits; ba.warps_per_block = warps; ba.persistent = 1; ba.chains = g.chains; ba.table_kind = g.kind;
         ba.load_shift = g.load_shift;
         ba.fill = g.fill;
-        // (the arithmetic goes by this chunk's primes: one beyond 2^49 elsewhere in the list costs it nothing)
-        const u64 chunk_top = top < kFp64Limit || cnt == n ? top : *std::max_element(primes + off, primes + off + cnt);
         ba.lanes = for_range(g, chunk_top + 1).lanes;
         ba.low = chunk_top < kHashLow;
         ba.max_p = chunk_top;
@@ -1500,7 +1518,7 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
             for (u64 i = 0; i < nr; ++i)
                 if (c->h_rel[i].q != ~0ull) rel.push_back(c->h_rel[i]);
         }
-        c->stats.kernel_launches += 3 + kPrepLaunches;
+        c->stats.kernel_launches += 2 + prep_launches(pa.split, false);
         c->stats.entries += c->h_ctr->entries;
         c->stats.bsgs_steps += c->h_ctr->steps;
         c->stats.bsgs_baby_steps += c->h_ctr->baby;

@@ -43,6 +43,16 @@ inline u64 split_modulus(u32 class_modulus, u64 cm) {
     return class_modulus;
 }
 
+// A split modulus that needs no split by single primes: the powers of 2 and 3 and the
+// primes 5 .. 19, or those of them that fit.
+inline u64 split_modulus_alone(u64 cm) {
+    for (u64 base : {232792560ull, 720720ull, 5040ull}) {
+        const u64 l = cm / gcd_host(cm, base) * base;
+        if (l <= kMaxSplit) return l;
+    }
+    return 5040;
+}
+
 // Validates an item the way load_worktodo does (Config.hpp:156-190), plus the
 // GPU path's range P1 <= 2^62, and fills every DevItem field except the
 // baby-step cap max_baby.  Returns MPS_OK, or an MPS_E_* code with *why set.

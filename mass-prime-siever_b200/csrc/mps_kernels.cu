@@ -3169,8 +3169,8 @@ cudaError_t launch_sieve_wave(const WaveDesc* w, const SieveTables& t, const Sur
 
 cudaError_t launch_prep(const PrepArgs& a, Counters* ctr, int grid, int num_sms, cudaStream_t s) {
     k_prep<<<grid, kPrepThreads, 0, s>>>(a, ctr);
-    if (!a.surv_split) k_split<<<num_sms * 2, 256, 0, s>>>(a, ctr);
-    k_dlog<<<num_sms * 4, 256, 0, s>>>(a, ctr);
+    if (a.split && !a.surv_split) k_split<<<num_sms * 2, 256, 0, s>>>(a, ctr);
+    if (a.split) k_dlog<<<num_sms * 4, 256, 0, s>>>(a, ctr);
     k_setup<<<num_sms * 7, kSetupWarps * 32, 0, s>>>(a, ctr);
     return cudaGetLastError();
 }

@@ -98,6 +98,7 @@ struct PrepArgs {
     u64 surv_cap;
     const u32* surv_item;      // nullptr: every survivor belongs to `item0`
     const u64* surv_split;     // the sieve's split primes (SurvOut::split); nullptr: k_split finds them
+    u32 split;                 // 0: no item has split_more, so there are no split events
     SieveTables tables;
     u32 item0;
     const DevItem* items;
@@ -141,7 +142,8 @@ inline void set_event_lists(PrepArgs* a, SplitEvent* events, u64 ev_cap, u64 ev_
 // Split primes to look for in the range of an item with K in-class exponents.
 u32 split_primes_for(u64 K);
 constexpr u64 kSievedPrimeBelow = (u64)kSieveMaxPrime * kSieveMaxPrime;
-constexpr u32 kPrepLaunches = 3;      // kernels of one launch_prep (one more without surv_split)
+// kernels of one launch_prep
+constexpr u32 prep_launches(bool split, bool sieved) { return 2 + (split ? sieved ? 1 : 2 : 0); }
 cudaError_t launch_prep(const PrepArgs& a, Counters* ctr, int grid, int num_sms, cudaStream_t s);
 
 // Exact BSGS, one warp per entry.

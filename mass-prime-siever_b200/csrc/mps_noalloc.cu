@@ -184,6 +184,7 @@ int run_pass(unsigned char* base, u64 lo, u64 hi, const DevItem& d, u32 tbits, i
     pa.surv = surv;
     pa.surv_cap = kNoAllocSurv;
     pa.surv_split = split;
+    pa.split = sa.n_split != 0;
     pa.tables = tables;
     pa.item0 = 0;
     pa.items = ditem;

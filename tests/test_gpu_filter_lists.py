@@ -38,3 +38,19 @@ def test_arithmetic_by_chunk(mps_lib, oracle):
         # in one chunk: the same flags
         mixed = low[:2000] + high + low[2000:3000]
         assert s.filter(mixed, it) == flags[:2000] + flags[4096:] + flags[2000:3000]
+
+
+@pytest.mark.parametrize("P0,counts", [(10**9, (1, 2, 31, 1000, 16383, 16384)), (2**49, (1, 33, 8191, 8192))])
+@pytest.mark.parametrize("mod,res", [(1, 0), (6, 4), (1001, 7), (2**20 - 3, 5)])
+def test_short_and_long_lists(mps_lib, oracle, P0, counts, mod, res):
+    """Lists on both sides of the length from which the primes are split: the oracle's
+    flags, with only the kernels that a list needs (a short one: no split's)."""
+    primes = oracle.primes(P0, P0 + 24 * 16_384 + 100_000, 1 << 16)
+    spec = (3, 2, P0, primes[-1] + 1, 0, 10**7, mod, res)
+    hits = {r[0] for r in oracle.relations(P0, primes[max(counts)] + 1, oracle_item(*spec))}
+    it = mps_lib.make_item(*spec)
+    with mps_lib.Siever(0) as s:
+        for n in counts:
+            assert s.filter(primes[:n], it) == [int(p in hits) for p in primes[:n]]
+            split = n in (16384, 8192) and 10**7 // mod >= 1536
+            assert s.stats()["kernel_launches"] == (6 if split else 4)
