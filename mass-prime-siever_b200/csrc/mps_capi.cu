@@ -123,6 +123,7 @@ struct mps_ctx {
     size_t smem_optin = 227 * 1024;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evb0 = nullptr, evb1 = nullptr;
+    cudaEvent_t items_up = nullptr;    // the items of the call are on the device
     cudaEvent_t evk[kStageEvents] = {};
     bool ended = false;             // ev1 is recorded and reached (the chunk path's last wait)
     mps_tuning tun{};
@@ -381,16 +382,15 @@ int reserve_items(mps_ctx* c, size_t n) {
     return MPS_OK;
 }
 
-// The items to the device.  For the waves (other streams), with their progress
-// reset and waited for; for the chunk path, whose kernels follow on the same
-// stream and touch no progress, the copy alone (it has read the items when it
-// returns: they are pageable memory).
+// The items to the device, their progress reset, in order on the context's stream;
+// run_waves has the waves' streams wait for items_up.  (The copy has read the items
+// when it returns: they are pageable memory.)
 int upload_items(mps_ctx* c, const DevItem* items, size_t n, bool waves = true) {
     if (int r = reserve_items(c, std::max<size_t>(n, 1))) return r;
     CK(cudaMemcpyAsync(c->d_items, items, n * sizeof(DevItem), cudaMemcpyHostToDevice, c->stream), "item upload");
-    if (!waves) return MPS_OK;
+    if (!waves) return MPS_OK;                          // the chunk path touches no progress
     CK(cudaMemsetAsync(c->d_state, 0, n * sizeof(ItemState), c->stream), "item state reset");
-    CK(cudaStreamSynchronize(c->stream), "item upload");
+    CK(cudaEventRecord(c->items_up, c->stream), "event");
     return MPS_OK;
 }
 
@@ -796,8 +796,10 @@ int run_waves(mps_ctx* c, const std::vector<u64>& lo, const std::vector<u64>& hi
             if (int r = slot_alloc(c, w)) return r;
         c->slots_ready = true;
     }
-    for (WaveSlot& w : c->slot)
+    for (WaveSlot& w : c->slot) {
         if (int r = slot_alloc(c, w)) return r;
+        CK(cudaStreamWaitEvent(w.stream, c->items_up, 0), "item upload");
+    }
     const u64 chunk = c->tun.chunk_odds;
     int k = 0;
     WaveSlot* cur = nullptr;
@@ -1343,6 +1345,7 @@ int mps_open(int device, const mps_tuning* tuning, mps_ctx** out) {
         if ((e = cudaEventCreate(ev)) != cudaSuccess) return bail(e, "event");
     for (cudaEvent_t& ev : c->evk)
         if ((e = cudaEventCreate(&ev)) != cudaSuccess) return bail(e, "event");
+    if ((e = cudaEventCreateWithFlags(&c->items_up, cudaEventDisableTiming)) != cudaSuccess) return bail(e, "event");
     const HostTables& t = host_tables();
     const size_t n = t.sp.size();
     if ((e = cudaMalloc((void**)&c->d_sp, n * sizeof(u32))) != cudaSuccess) return bail(e, "tables");
@@ -1368,7 +1371,7 @@ int mps_close(mps_ctx* c) {
         if (p) cudaFree(p);
     if (c->h_ctr) cudaFreeHost(c->h_ctr);
     if (c->h_rel) cudaFreeHost(c->h_rel);
-    for (cudaEvent_t ev : {c->ev0, c->ev1, c->evb0, c->evb1})
+    for (cudaEvent_t ev : {c->ev0, c->ev1, c->evb0, c->evb1, c->items_up})
         if (ev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : c->evk)
         if (ev) cudaEventDestroy(ev);
