@@ -211,7 +211,8 @@ int mps_serve_close(mps_server* sv);
  * chains per lane, warps per block) by the BSGS kernel's CUDA events on a calibration slice of
  * the item (its first 2^25 integers); with the fastest, the table fill and the
  * baby/giant balance (baby_scale) the same way; then the sieve's segment size
- * (1024, 2048 or 4096 words) by the sieve kernel's events;
+ * (1024, 2048 or 4096 words) by the sieve kernel's events on a full wave of
+ * chunk_odds odd numbers;
  * checks that every candidate gives the same relations, and keeps the
  * fastest configuration for the class.  Later calls on items of a tuned class
  * use it (per item; a batched wave uses the configuration of its item with
@@ -229,8 +230,8 @@ typedef struct mps_tune_report {
     uint32_t table_fill;          /* table load chosen (keys per word x 256)             */
     uint32_t baby_scale;          /* baby-step scale chosen (x 256 of the square root)   */
     double   best_ns_per_prime;   /* BSGS time per prime reaching the BSGS, chosen       */
-    double   default_ns_per_prime;/* the same under the context's tuning fields          */
-    double   sieve_best_ms;       /* sieve time of the calibration slice, chosen segment */
+    double   default_ns_per_prime;/* the same with what the class runs untuned           */
+    double   sieve_best_ms;       /* sieve time of a full wave, chosen segment           */
     double   sieve_default_ms;    /* the same with the default segment (2048 words)      */
     uint64_t calib_bsgs_primes;   /* primes of the calibration slice reaching the BSGS   */
 } mps_tune_report;

@@ -266,20 +266,23 @@ u64 tune_key(u64 K, u64 cm, u64 P0) {
     return (kb << 40) | (std::min<u64>(cm, 4095) << 8) | pd;
 }
 
-// The configuration for an item: the tuned one of its class, else the default,
-// with four chains per lane instead of two for an item of at least 2^20
-// exponents when the tuning leaves the chains open.  Four chains spread the
-// loop's own instructions over twice the steps, but the last iteration of each
-// loop is then half empty on average: BSGS of 2^27 integers, two and four chains,
-// K = 10^7 5.63 and 5.26 ms, K = 1.7 * 10^6 1.32 and 1.28, K = 7 * 10^5 equal, K =
-// 10^4 0.19 and 0.23.
+// The configuration of an item of an untuned class: the default, with four chains
+// per lane instead of two for an item of at least 2^20 exponents when the tuning
+// leaves the chains open.  Four chains spread the loop's own instructions over twice
+// the steps, but the last iteration of each loop is then half empty on average: BSGS
+// of 2^27 integers, two and four chains, K = 10^7 5.63 and 5.26 ms, K = 1.7 * 10^6
+// 1.32 and 1.28, K = 7 * 10^5 equal, K = 10^4 0.19 and 0.23.
 constexpr u64 kFourChainsK = 1ull << 20;
-LaunchCfg cfg_for(const mps_ctx* c, u64 K, u64 cm, u64 P0) {
-    auto it = c->tuned.find(tune_key(K, cm, P0));
-    if (it != c->tuned.end()) return it->second.cfg;
+LaunchCfg untuned_cfg(const mps_ctx* c, u64 K) {
     LaunchCfg g = default_cfg(c);
     if (c->tun.chains == 0 && g.kind == 3 && K >= kFourChainsK) g.chains = 4;
     return g;
+}
+
+// The configuration for an item: the tuned one of its class, if there is one.
+LaunchCfg cfg_for(const mps_ctx* c, u64 K, u64 cm, u64 P0) {
+    auto it = c->tuned.find(tune_key(K, cm, P0));
+    return it != c->tuned.end() ? it->second.cfg : untuned_cfg(c, K);
 }
 
 // log2 of the primes a warp solves at once (lanes per prime 32, 16 or 8).
@@ -1275,6 +1278,62 @@ void sort_by_p(std::vector<RawRelation>& rel) {
     rel.swap(sorted);
 }
 
+// The BSGS configurations that the tuner times, the class's own first.
+std::vector<LaunchCfg> tune_candidates(const LaunchCfg& base) {
+    std::vector<LaunchCfg> cands{base};
+    for (u32 kind : {0u, 3u})
+        for (u32 ch : {1u, 2u, 4u})
+            for (u32 w : {4u, 8u}) {
+                LaunchCfg g;
+                g.kind = kind;
+                g.chains = ch;
+                g.warps = w;
+                if (g != base) cands.push_back(g);
+            }
+    // lanes per prime: groups of 16 or 8 lanes (table kind 2, 1 or 2 chains)
+    for (u32 lanes : {16u, 8u})
+        for (u32 ch : {1u, 2u})
+            for (u32 w : {4u, 8u}) {
+                LaunchCfg g;
+                g.kind = 2;
+                g.load_shift = 2;
+                g.chains = ch;
+                g.warps = w;
+                g.lanes = lanes;
+                cands.push_back(g);
+            }
+    return cands;
+}
+
+// Device time of the sieve of a full wave (chunk_odds odd numbers from lo) in segments of
+// that many words, none of them cut smaller: the best of three after a first run.  (On
+// the calibration slice 4096 words make fewer segments than there are SMs and 2048
+// leave the last round half empty, so that 1024 always won; on 2^26 odd numbers 1024,
+// 2048 and 4096 words take 0.216, 0.194 and 0.215 ms.  Two waves overlap in an item
+// call, and its time is the same with 1024 and 2048 to 0.3%.)
+int time_sieve(mps_ctx* c, u64 lo, u64 K, u32 words, double* ms) {
+    SieveArgs sa{};
+    sa.lo_odd = std::max<u64>(lo, 3) | 1ull;
+    sa.n_odds = std::min<u64>(c->tun.chunk_odds, (kTwo62 - sa.lo_odd) / 2);
+    sa.hi = sa.lo_odd + 2 * sa.n_odds;
+    sa.n_primes = sieve_prime_count(sa.hi);
+    sa.n_split = split_for(c, K);
+    if (int r = ensure(c, &c->d_surv, &c->surv_cap, c->tun.chunk_odds + 16, "survivor buffer")) return r;
+    if (int r = ensure(c, &c->d_surv_split, &c->surv_split_cap, c->surv_cap, "split primes")) return r;
+    const SurvOut out{c->d_surv, nullptr, c->d_surv_split, c->surv_cap};
+    for (int rep = 0; rep < 4; ++rep) {
+        CK(cudaMemsetAsync(c->d_ctr, 0, sizeof(Counters), c->stream), "counter reset");
+        CK(cudaEventRecord(c->evb0, c->stream), "event");
+        CK(launch_sieve(sa, c->tables(), out, c->d_ctr, c->stream, words, false), "sieve launch");
+        CK(cudaEventRecord(c->evb1, c->stream), "event");
+        CK(cudaEventSynchronize(c->evb1), "sieve");
+        float t = 0;
+        CK(cudaEventElapsedTime(&t, c->evb0, c->evb1), "event time");
+        if (rep == 1 || (rep > 1 && t < *ms)) *ms = t;
+    }
+    return MPS_OK;
+}
+
 // Keeps rel as the context's last relations and copies them out.
 int copy_out(mps_ctx* c, std::vector<RawRelation>& kept, mps_relation* out, uint32_t* out_item, size_t cap,
              size_t* n_out) {
@@ -1839,29 +1898,6 @@ int mps_autotune(mps_ctx* c, const mps_item* items, size_t n_items, mps_tune_rep
     if (!items && n_items) return fail(c, MPS_E_ARG, "items is NULL");
     if (!out && cap) return fail(c, MPS_E_ARG, "out is NULL");
     constexpr u64 kCalibSpan = 1ull << 25;
-    const LaunchCfg base = default_cfg(c);
-    std::vector<LaunchCfg> cands{base};
-    for (u32 kind : {0u, 3u})
-        for (u32 ch : {1u, 2u, 4u})
-            for (u32 w : {4u, 8u}) {
-                LaunchCfg g;
-                g.kind = kind;
-                g.chains = ch;
-                g.warps = w;
-                if (g != base) cands.push_back(g);
-            }
-    // lanes per prime: groups of 16 or 8 lanes (table kind 2, 1 or 2 chains)
-    for (u32 lanes : {16u, 8u})
-        for (u32 ch : {1u, 2u})
-            for (u32 w : {4u, 8u}) {
-                LaunchCfg g;
-                g.kind = 2;
-                g.load_shift = 2;
-                g.chains = ch;
-                g.warps = w;
-                g.lanes = lanes;
-                cands.push_back(g);
-            }
     std::vector<mps_tune_report> reps;
     std::set<u64> seen;
     for (size_t i = 0; i < n_items; ++i) {
@@ -1870,25 +1906,25 @@ int mps_autotune(mps_ctx* c, const mps_item* items, size_t n_items, mps_tune_rep
         if (int r = item_constants(&items[i], c->tun.class_modulus, 0, &d, &why)) return fail(c, r, why);
         const u64 key = tune_key(d.K, d.cm, items[i].P0);
         if (!seen.insert(key).second || !d.has_work) continue;
+        const LaunchCfg base = untuned_cfg(c, d.K);
+        const std::vector<LaunchCfg> cands = tune_candidates(base);
         const u64 lo = items[i].P0, hi = std::min<u64>(items[i].P1, items[i].P0 + kCalibSpan);
         double best_ms = 0, base_ms = 0, sieve_base_ms = 0, sieve_best_ms = 0;
         u64 entries = 0;
         LaunchCfg best = base;
         std::vector<RawRelation> first;
         // phase 1: the BSGS configuration by the BSGS kernel's time; phase 2: with
-        // it, the table fill and the baby-step scale (fingerprint words only);
-        // phase 3: the sieve's segment size by the sieve kernel's time
+        // it, the table fill and the baby-step scale (fingerprint words only)
         constexpr u32 kFills[] = {224u, 192u, 160u, 128u};
         constexpr u32 kScales[] = {224u, 192u, 160u, 128u};
         const size_t n_bsgs = cands.size();
         const size_t n_fill = n_bsgs + (sizeof(kFills) / sizeof(kFills[0])) * (sizeof(kScales) / sizeof(kScales[0]));
-        const size_t n_all = n_fill + 3;
         size_t timed = 0;
-        for (size_t k = 0; k < n_all; ++k) {
+        for (size_t k = 0; k < n_fill; ++k) {
             LaunchCfg g;
             if (k < n_bsgs) {
                 g = cands[k];
-            } else if (k < n_fill) {                            // phase 2 keeps the chosen BSGS settings
+            } else {                                            // phase 2 keeps the chosen BSGS settings
                 if (best.kind != 0 && best.kind != 3) continue;
                 const size_t f = (k - n_bsgs) / (sizeof(kScales) / sizeof(kScales[0]));
                 const size_t sc = (k - n_bsgs) % (sizeof(kScales) / sizeof(kScales[0]));
@@ -1896,9 +1932,6 @@ int mps_autotune(mps_ctx* c, const mps_item* items, size_t n_items, mps_tune_rep
                 g.fill = kFills[f];
                 g.scale = kScales[sc];
                 if (g == best) continue;
-            } else {                                            // phase 3 keeps the chosen BSGS settings
-                g = best;
-                g.seg_words = 1024u << (k - n_fill);
             }
             if (g.lanes != 32 && hi > kFp64Limit) continue;    // groups run the FP64 solve only
             u32 tb, mb;
@@ -1908,13 +1941,12 @@ int mps_autotune(mps_ctx* c, const mps_item* items, size_t n_items, mps_tune_rep
             if (bsgs_smem_bytes(tb, g.warps, g.kind) > c->smem_optin) continue;
             if (int r = upload_items(c, &d, 1)) return r;
             ++timed;
-            double ms = 0, sms = 0;
+            double ms = 0;
             for (int rep = 0; rep < 2; ++rep) {                 // the second run is timed
                 std::vector<RawRelation> rel;
                 std::memset(&c->stats, 0, sizeof(c->stats));
                 if (int r = run_chunk(c, lo, hi, 0, d.K, g, rel)) return r;
                 ms = c->stats.bsgs_ms;
-                sms = c->stats.sieve_ms;
                 entries = c->stats.entries;
                 sort_by_p(rel);
                 if (k == 0 && rep == 0) {
@@ -1926,18 +1958,21 @@ int mps_autotune(mps_ctx* c, const mps_item* items, size_t n_items, mps_tune_rep
                     return fail(c, MPS_E_CUDA, "tuning candidates gave different relations");
                 }
             }
-            if (k < n_fill) {
-                if (k == 0) base_ms = ms;
-                if (k == 0 || ms < best_ms) {
-                    best_ms = ms;
-                    best = g;
-                }
-            } else {
-                if (g.seg_words == base.seg_words) sieve_base_ms = sms;
-                if (k == n_fill || sms < sieve_best_ms) {
-                    sieve_best_ms = sms;
-                    best.seg_words = g.seg_words;
-                }
+            if (k == 0) base_ms = ms;
+            if (k == 0 || ms < best_ms) {
+                best_ms = ms;
+                best = g;
+            }
+        }
+        // phase 3: the sieve's segment size, by the sieve of one full wave
+        for (u32 words : {1024u, 2048u, 4096u}) {
+            double ms = 0;
+            if (int r = time_sieve(c, lo, d.K, words, &ms)) return r;
+            ++timed;
+            if (words == base.seg_words) sieve_base_ms = ms;
+            if (sieve_best_ms == 0 || ms < sieve_best_ms) {
+                sieve_best_ms = ms;
+                best.seg_words = words;
             }
         }
         const double per = entries ? 1e6 / (double)entries : 0.0;

@@ -3131,9 +3131,9 @@ u32 range_seg_words(u32 seg_words, u64 n_odds) {
 }
 
 cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, const SurvOut& o, Counters* ctr, cudaStream_t s,
-                         u32 seg_words) {
+                         u32 seg_words, bool fit) {
     if (!valid_seg_words(seg_words)) return cudaErrorInvalidValue;
-    seg_words = range_seg_words(seg_words, a.n_odds);
+    if (fit) seg_words = range_seg_words(seg_words, a.n_odds);
     const u64 seg_odds = (u64)seg_words * 32;
     const u64 segs = (a.n_odds + seg_odds - 1) / seg_odds;
     if (segs == 0 && !a.include_two) return cudaSuccess;

@@ -44,7 +44,7 @@ constexpr u64 kFewSegs = 148;
 constexpr u32 kLeastSegWords = 256;
 constexpr u32 kDefaultSegWords = 2048;
 cudaError_t launch_sieve(const SieveArgs& a, const SieveTables& t, const SurvOut& o, Counters* ctr, cudaStream_t s,
-                         u32 seg_words = kDefaultSegWords);
+                         u32 seg_words = kDefaultSegWords, bool fit = true);   // fit: cut a short range smaller
 
 // A wave: several runs (odd ranges of possibly different items) sieved by
 // one launch; kept in device memory so that a captured graph is replayable.
