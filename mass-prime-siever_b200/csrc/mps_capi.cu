@@ -168,6 +168,7 @@ int fail(mps_ctx* c, int code, const std::string& msg) {
 }
 
 int cuda_fail(mps_ctx* c, cudaError_t e, const char* what) {
+    cudaGetLastError();             // (out of memory: the next launch's check must not see it)
     c->poisoned = (e == cudaErrorIllegalAddress || e == cudaErrorLaunchFailure || e == cudaErrorIllegalInstruction ||
                    e == cudaErrorMisalignedAddress || e == cudaErrorHardwareStackError);
     return fail(c, MPS_E_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
@@ -380,8 +381,12 @@ int reserve_items(mps_ctx* c, size_t n) {
     if (c->d_state) CK(cudaFree(c->d_state), "cudaFree");
     c->d_state = nullptr;
     const u64 cap = std::max<u64>(n, 64);
+    c->items_cap = 0;
     if (int r = ensure(c, &c->d_items, &c->items_cap, cap, "item buffer")) return r;
-    CK(cudaMalloc((void**)&c->d_state, cap * sizeof(ItemState)), "item state");
+    if (cudaError_t e = cudaMalloc((void**)&c->d_state, cap * sizeof(ItemState)); e != cudaSuccess) {
+        c->items_cap = 0;
+        return cuda_fail(c, e, "item state");
+    }
     return MPS_OK;
 }
 
@@ -581,32 +586,37 @@ void drop_graphs(WaveSlot& w) {
 
 int slot_alloc(mps_ctx* c, WaveSlot& w) {
     const u64 chunk = c->tun.chunk_odds;
-    if (!w.stream) {
-        CK(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking), "stream");
-        for (cudaEvent_t& ev : w.evk) CK(cudaEventCreate(&ev), "event");
-        CK(cudaMalloc((void**)&w.d_ctr, sizeof(Counters)), "counters");
-        CK(cudaMallocHost((void**)&w.h_ctr, sizeof(Counters)), "counters");
-        CK(cudaMalloc((void**)&w.d_wave, sizeof(WaveDesc)), "wave descriptor");
-        CK(cudaMallocHost((void**)&w.h_wave, sizeof(WaveDesc)), "wave descriptor");
-    }
-    if (w.surv_cap < chunk + kMaxRuns + 16) {
-        if (w.d_surv) CK(cudaFree(w.d_surv), "cudaFree");
-        if (w.d_surv_item) CK(cudaFree(w.d_surv_item), "cudaFree");
-        if (w.d_surv_split) CK(cudaFree(w.d_surv_split), "cudaFree");
-        w.surv_cap = chunk + kMaxRuns + 16;
-        CK(cudaMalloc((void**)&w.d_surv, w.surv_cap * sizeof(u64)), "survivor buffer");
-        CK(cudaMalloc((void**)&w.d_surv_item, w.surv_cap * sizeof(u32)), "survivor items");
-        CK(cudaMalloc((void**)&w.d_surv_split, w.surv_cap * sizeof(u64)), "split primes");
+    if (!w.stream) CK(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking), "stream");
+    for (cudaEvent_t& ev : w.evk)
+        if (!ev) CK(cudaEventCreate(&ev), "event");
+    if (!w.d_ctr) CK(cudaMalloc((void**)&w.d_ctr, sizeof(Counters)), "counters");
+    if (!w.h_ctr) CK(cudaMallocHost((void**)&w.h_ctr, sizeof(Counters)), "counters");
+    if (!w.d_wave) CK(cudaMalloc((void**)&w.d_wave, sizeof(WaveDesc)), "wave descriptor");
+    if (!w.h_wave) CK(cudaMallocHost((void**)&w.h_wave, sizeof(WaveDesc)), "wave descriptor");
+    // (a capacity is set once its buffers are there: a call that ran out of memory
+    // leaves none, and the next one allocates again)
+    const u64 surv = chunk + kMaxRuns + 16;
+    if (w.surv_cap < surv) {
         drop_graphs(w);
+        w.surv_cap = 0;
+        for (void* p : {(void*)w.d_surv, (void*)w.d_surv_item, (void*)w.d_surv_split})
+            if (p) CK(cudaFree(p), "cudaFree");
+        w.d_surv = w.d_surv_split = nullptr;
+        w.d_surv_item = nullptr;
+        CK(cudaMalloc((void**)&w.d_surv, surv * sizeof(u64)), "survivor buffer");
+        CK(cudaMalloc((void**)&w.d_surv_item, surv * sizeof(u32)), "survivor items");
+        CK(cudaMalloc((void**)&w.d_surv_split, surv * sizeof(u64)), "split primes");
+        w.surv_cap = surv;
     }
     if (w.ent_cap < entry_cap(chunk)) {
-        if (int r = alloc_entries(c, &w.d_ent, &w.d_events, &w.d_big, &w.ent_cap, entry_cap(chunk))) return r;
         drop_graphs(w);
+        if (int r = alloc_entries(c, &w.d_ent, &w.d_events, &w.d_big, &w.ent_cap, entry_cap(chunk))) return r;
     }
-    if (w.rel_cap < (1u << 16)) {
-        w.rel_cap = 1u << 16;
-        CK(cudaMalloc((void**)&w.d_rel, w.rel_cap * sizeof(RawRelation)), "relation buffer");
-        CK(cudaMallocHost((void**)&w.h_rel, w.rel_cap * sizeof(RawRelation)), "relation buffer");
+    constexpr u64 kSlotRelations = 1u << 16;
+    if (w.rel_cap < kSlotRelations) {
+        if (!w.d_rel) CK(cudaMalloc((void**)&w.d_rel, kSlotRelations * sizeof(RawRelation)), "relation buffer");
+        if (!w.h_rel) CK(cudaMallocHost((void**)&w.h_rel, kSlotRelations * sizeof(RawRelation)), "relation buffer");
+        w.rel_cap = kSlotRelations;
     }
     return MPS_OK;
 }

@@ -27,3 +27,21 @@ def test_every_prime_of_the_densest_chunk_fits(mps_lib, odds):
         s.chunk_relations(3, 3 + 2 * odds, it)
         st = s.stats()
         assert st["chunks"] == 1 and st["entries"] > 0.9 * s.count_primes(1000, 3 + 2 * odds)
+
+
+def test_a_context_that_runs_out_of_memory(mps_lib, siever, oracle):
+    """Chunks larger than the device: every call fails for want of the same buffer (none
+    goes on with what the failed one left), and other contexts are unaffected."""
+    from oracle.oracle import make_item as oracle_item
+
+    spec = (2, -25, 10**6, 2 * 10**6, 0, 1000, 2, 1)
+    it = mps_lib.make_item(*spec)
+    want = oracle.relations(spec[2], spec[3], oracle_item(*spec))
+    with mps_lib.Siever(0, chunk_odds=1 << 36) as s:
+        for call in (s.item_relations, lambda i: s.batch_relations([i, i])):
+            for _ in range(2):
+                with pytest.raises(mps_lib.MpsError, match="survivor buffer") as e:
+                    call(it)
+                assert e.value.code == mps_lib.MPS_E_CUDA
+                assert siever.chunk_relations(spec[2], spec[3], it) == want
+    assert siever.item_relations(it) == want
