@@ -68,13 +68,18 @@ typedef struct mps_tuning {
     uint32_t bsgs_warps;        /* warps per BSGS block (0: 4)                                 */
     uint32_t class_modulus;     /* Q of the power-residue split g = gcd(Q, p-1), even, <= 2^28
                                    (0: lcm(mod, 144), else lcm(mod, 24), the first within
-                                    2^28, else 144, and a further split by every prime
-                                    5..4261 that divides p - 1;
+                                    2^28, else 144, and a further split of the primes with
+                                    1,536 exponents left or more by primes l that divide
+                                    p - 1: 5 .. 19, and one l each of 23 .. 61, 67 .. 251,
+                                    257 .. 1021 and 1031 .. 4259, the larger ones for larger
+                                    counts; mps_filter on fewer than 16,384 primes (8,192
+                                    from 2^49 on) has no further split;
                                     1: lcm(mod, 2), the reference's plain-method filter)       */
     uint32_t full_mr;           /* 1: 12-base Miller-Rabin on every filter survivor (eager)    */
     uint32_t plain;             /* 1: plain per-chunk path (host sync between stages)          */
     uint32_t chains;            /* BSGS chains per lane, 1, 2 or 4 (0: 2, or 4 for an item of at
-                                   least 2^20 in-class exponents)                               */
+                                   least 2^20 in-class exponents; a batched wave takes 4 when
+                                   all its items do, a served wave always 2)                    */
     uint32_t graphs_off;        /* 1: launch waves directly instead of replaying CUDA graphs   */
     uint32_t table_kind;        /* BSGS table: 0 = four 16-bit fingerprints per 64-bit word,
                                    inserted by compare-and-swap, 1 = one 32-bit key per slot,
@@ -102,7 +107,10 @@ typedef struct mps_stats {
     double   bsgs_ms;           /* device time of the BSGS kernel               */
     uint64_t bsgs_launches;
     uint64_t kernel_launches;   /* kernels of this library launched             */
-    uint64_t bsgs_steps;        /* baby + giant steps (modular multiplies) of the BSGS kernel */
+    uint64_t bsgs_steps;        /* baby + giant steps (modular multiplies) of the BSGS kernel; of
+                                   two l of one size class a prime is split by either one, so
+                                   that two runs of a call may differ by some hundredths of a
+                                   per cent (their relations do not)                          */
     double   sieve_ms;          /* device time of the sieve kernel (CUDA events)  */
     double   prep_ms;           /* device time of the prep kernels (prep, splits, set-up) */
     double   order_ms;          /* device time of the order kernel                */

@@ -31,8 +31,9 @@ constexpr u64 kHashLow = 1ull << 30;
 // Largest baby-step count of one prime (a table of 2^13 slots at load 1/2).
 constexpr u32 kMaxBaby = 4096;
 // Measured on the B200 (C2 and C3 slices): a baby step (hash, insert) costs
-// about twice a giant step (hash, probe), so m = 0.625 sqrt(jcount) beats the
-// square root, and words filled to 0.625 keys overflow rarely enough.
+// more than a giant step (hash, probe; 36 and 27 warp instructions), so m = 0.625
+// sqrt(jcount) beats the square root, and words filled to 0.625 keys overflow rarely
+// enough.
 constexpr u32 kDefaultBabyScale = 160;   // m = ceil(sqrt(jcount)) x 160/256
 constexpr u32 kDefaultFill = 160;        // fingerprint words: 0.625 keys per word on average
 
@@ -69,7 +70,7 @@ struct DevItem {
 };
 
 // The split by primes l | p - 1 outside the split modulus: the kSplitPrimes
-// sieving primes from 5 (to 4261); k is an l's index among them.  The first
+// sieving primes from 5 to kSplitLast; k is an l's index among them.  The first
 // kSplitSmall (5 .. 19) have a slot of an entry each; the sieve finds the others,
 // one of each of kSplitClasses size classes, a slot a class.  Events queue in
 // lists by size, the classes' and one for the small l, for each of the two
@@ -80,6 +81,21 @@ constexpr u32 kSplitClasses = 4, kSplitSizes = kSplitClasses + 1, kSplitLists = 
 __host__ __device__ constexpr u32 split_class(u32 k) {       // k >= kSplitSmall; l < 64, 256, 1024
     return k < 16 ? 0u : k < 52 ? 1u : k < 170 ? 2u : 3u;
 }
+constexpr u32 kSplitLast = 4259;
+constexpr u32 primes_from_5(u32 below) {                     // number of primes 5 <= q < below
+    u32 n = 0;
+    for (u32 q = 5; q < below; q += 2) {
+        bool prime = true;
+        for (u32 d = 3; d * d <= q && prime; d += 2) prime = q % d != 0;
+        n += prime;
+    }
+    return n;
+}
+static_assert(primes_from_5(kSplitLast) == kSplitPrimes - 1 && primes_from_5(kSplitLast + 1) == kSplitPrimes, "the last split prime");
+static_assert(primes_from_5(20) == kSplitSmall, "5 .. 19");
+static_assert(split_class(primes_from_5(64)) == 1 && split_class(primes_from_5(64) - 1) == 0 && split_class(primes_from_5(256)) == 2 &&
+                  split_class(primes_from_5(256) - 1) == 1 && split_class(primes_from_5(1024)) == 3 &&
+                  split_class(primes_from_5(1024) - 1) == 2, "the size classes");
 __host__ __device__ constexpr u32 slot_list(u32 slot) { return slot < kSplitClasses ? slot : kSplitClasses; }
 
 // One prime that reached the discrete-log stages: the candidates left are

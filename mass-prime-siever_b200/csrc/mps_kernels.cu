@@ -7,7 +7,7 @@
 //            power-residue split over g = gcd(Q, p - 1) (Gpu.hpp:465-589,
 //            Math.hpp:410-433), class combination; staged through shared-memory
 //            queues so that every stage runs with full warps
-//   k_dlog   per prime and l | p - 1 (5 .. 4261, found by the sieve, or by
+//   k_dlog   per prime and l | p - 1 (5 .. 4259, found by the sieve, or by
 //            k_split for given primes): the candidates' residue mod l
 //   k_setup  applies those, sets the solve up, and solves entries with few
 //            candidates left, one lane each
@@ -775,7 +775,7 @@ __device__ __forceinline__ bool combine_class(u64 p, const DevItem& it, u32 d, u
 // w = b^((p-1)/l) and u = t^((p-1)/l), b^n == t forces w^n == u, so n is known
 // mod l (or, when b is an l-th power residue, t has to be one too).  One
 // discrete logarithm in a group of l elements divides the candidates by l and
-// the baby and giant steps by sqrt(l); a prime has an l of 5 .. 4261 with
+// the baby and giant steps by sqrt(l); a prime has an l of 5 .. 4259 with
 // chance 1/(l-1), 1.7 in all.  Those of 5 .. 19 are tried on each entry, finding
 // the others costs a second walk of the sieve's bitmap (sieve_segment); a
 // logarithm costs about 700 lane instructions for the powers and 1.2 l for the
@@ -889,11 +889,6 @@ __device__ __noinline__ u32 lane_rest(F f, typename F::V t, typename F::V B, typ
 }
 
 template <class F>
-__device__ __forceinline__ u32 lane_match32(F f, typename F::V t, typename F::V B, typename F::V g, u32 base) {
-    return lane_match<32>(f, t, B, g, base);
-}
-
-template <class F>
 __device__ __forceinline__ u32 lane_solve16(const F& f, typename F::V t, typename F::V G0, typename F::V B, u32 J) {
     typedef typename F::V V;
     constexpr u32 M = 16;
@@ -956,7 +951,7 @@ __device__ __forceinline__ u32 lane_solve32(const F& f, typename F::V t, typenam
         for (u32 i = 0; i < M / 2; ++i) z |= equal_halves(key[i], rep);
         if (z) {
             if (n == 2) {
-                best = lane_match32(f, t, B, g0, b0);
+                best = lane_match<32>(f, t, B, g0, b0);
                 if (best != ~0u) break;
                 g0 = g1;
                 b0 = b1;
@@ -974,8 +969,8 @@ __device__ __forceinline__ u32 lane_solve32(const F& f, typename F::V t, typenam
         g = next;
     }
     __syncwarp(together);
-    if (best == ~0u && n > 0) best = lane_match32(f, t, B, g0, b0);
-    if (best == ~0u && n > 1) best = lane_match32(f, t, B, g1, b1);
+    if (best == ~0u && n > 0) best = lane_match<32>(f, t, B, g0, b0);
+    if (best == ~0u && n > 1) best = lane_match<32>(f, t, B, g1, b1);
     return best < J ? best : ~0u;
 }
 
@@ -1101,7 +1096,7 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep(PrepArgs a, Counters* 
                 // the primes l | p - 1 to split by: 5 .. 19 here, the others from the sieve
                 u32 k[kSplitSlots] = {};
                 if (ok && a.items[e.item].split_more) {
-                    const u32 limit = split_limit(e.jcount), Q = a.items[e.item].Q;
+                    const u32 limit = split_limit(e.jcount), modulus = a.items[e.item].Q;
                     const u64 found = a.surv_split ? a.surv_split[sv] : 0;
 #pragma unroll
                     for (u32 c = 0; c < kSplitClasses; ++c) {
@@ -1119,7 +1114,7 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep(PrepArgs a, Counters* 
                     }
 #pragma unroll
                     for (u32 s = 0; s < kSplitSlots; ++s)
-                        if (k[s] && Q % a.tables.sp[kSplitBase + k[s] - 1] == 0) k[s] = 0;   // Q splits by it
+                        if (k[s] && modulus % a.tables.sp[kSplitBase + k[s] - 1] == 0) k[s] = 0;   // Q splits by it
                 }
                 queue_events<0, kSplitSlots>(ok, slot, ok ? e.p : 0, k, a, ctr);
             }
@@ -1502,7 +1497,10 @@ __global__ void __launch_bounds__(kSetupWarps * 32, 7) k_setup(PrepArgs a, Count
         if (q < kLaneQueues) {
 #pragma unroll
             for (u32 k = 0; k < kLaneQueues; ++k)
-                if (k == q) idx = Q[k][n[k] -= 32, n[k] + lane];
+                if (k == q) {
+                    n[k] -= 32;
+                    idx = Q[k][n[k] + lane];
+                }
         } else if (!inputs) {
             u32 taken = 0;
 #pragma unroll
