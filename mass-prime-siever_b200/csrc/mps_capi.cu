@@ -427,10 +427,13 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     if (n_odds == 0 && !include_two) return MPS_OK;
     const u64 chunk = c->tun.chunk_odds;
     const u64 need_surv = n_odds + 16;
+    // (The relations' buffer comes first, beside the tables that k_order reads with it: behind
+    // the large buffers k_order took 37, 41 or 49 us for 50 relations of 2^24 integers at
+    // 10^10, by their sizes alone.)
+    if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
     if (int r = ensure(c, &c->d_surv, &c->surv_cap, std::max<u64>(need_surv, chunk + 16), "survivor buffer")) return r;
     if (int r = ensure(c, &c->d_surv_split, &c->surv_split_cap, c->surv_cap, "split primes")) return r;
     if (int r = ensure_entries(c, entry_cap(chunk))) return r;
-    if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
 
     u32 tbits, max_baby;
     table_for(c, g, K, &tbits, &max_baby);
@@ -595,6 +598,12 @@ int slot_alloc(mps_ctx* c, WaveSlot& w) {
     if (!w.h_wave) CK(cudaMallocHost((void**)&w.h_wave, sizeof(WaveDesc)), "wave descriptor");
     // (a capacity is set once its buffers are there: a call that ran out of memory
     // leaves none, and the next one allocates again)
+    constexpr u64 kSlotRelations = 1u << 16;
+    if (w.rel_cap < kSlotRelations) {
+        if (!w.d_rel) CK(cudaMalloc((void**)&w.d_rel, kSlotRelations * sizeof(RawRelation)), "relation buffer");
+        if (!w.h_rel) CK(cudaMallocHost((void**)&w.h_rel, kSlotRelations * sizeof(RawRelation)), "relation buffer");
+        w.rel_cap = kSlotRelations;
+    }
     const u64 surv = chunk + kMaxRuns + 16;
     if (w.surv_cap < surv) {
         drop_graphs(w);
@@ -611,12 +620,6 @@ int slot_alloc(mps_ctx* c, WaveSlot& w) {
     if (w.ent_cap < entry_cap(chunk)) {
         drop_graphs(w);
         if (int r = alloc_entries(c, &w.d_ent, &w.d_events, &w.d_big, &w.ent_cap, entry_cap(chunk))) return r;
-    }
-    constexpr u64 kSlotRelations = 1u << 16;
-    if (w.rel_cap < kSlotRelations) {
-        if (!w.d_rel) CK(cudaMalloc((void**)&w.d_rel, kSlotRelations * sizeof(RawRelation)), "relation buffer");
-        if (!w.h_rel) CK(cudaMallocHost((void**)&w.h_rel, kSlotRelations * sizeof(RawRelation)), "relation buffer");
-        w.rel_cap = kSlotRelations;
     }
     return MPS_OK;
 }
@@ -1542,9 +1545,9 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
             item_Q = Q;
             item_few = few;
         }
+        if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
         if (int r = ensure(c, &c->d_surv, &c->surv_cap, std::max<u64>(cnt + 16, chunk + 16), "survivor buffer")) return r;
         if (int r = ensure_entries(c, std::max<u64>(cnt, 1 << 16))) return r;
-        if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
         u32 tbits, mb;
         table_for(c, g, d.K, &tbits, &mb);
         const u32 warps = g.warps;
