@@ -426,14 +426,14 @@ int run_chunk(mps_ctx* c, u64 lo, u64 hi, u32 item, u64 K, const LaunchCfg& g_it
     const u32 include_two = (lo <= 2 && hi > 2) ? 1 : 0;
     if (n_odds == 0 && !include_two) return MPS_OK;
     const u64 chunk = c->tun.chunk_odds;
-    const u64 need_surv = n_odds + 16;
+    const u64 room = entry_cap(std::max<u64>(n_odds, chunk));
     // (The relations' buffer comes first, beside the tables that k_order reads with it: behind
     // the large buffers k_order took 37, 41 or 49 us for 50 relations of 2^24 integers at
     // 10^10, by their sizes alone.)
     if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
-    if (int r = ensure(c, &c->d_surv, &c->surv_cap, std::max<u64>(need_surv, chunk + 16), "survivor buffer")) return r;
+    if (int r = ensure(c, &c->d_surv, &c->surv_cap, room, "survivor buffer")) return r;
     if (int r = ensure(c, &c->d_surv_split, &c->surv_split_cap, c->surv_cap, "split primes")) return r;
-    if (int r = ensure_entries(c, entry_cap(chunk))) return r;
+    if (int r = ensure_entries(c, room)) return r;
 
     u32 tbits, max_baby;
     table_for(c, g, K, &tbits, &max_baby);
@@ -604,7 +604,7 @@ int slot_alloc(mps_ctx* c, WaveSlot& w) {
         if (!w.h_rel) CK(cudaMallocHost((void**)&w.h_rel, kSlotRelations * sizeof(RawRelation)), "relation buffer");
         w.rel_cap = kSlotRelations;
     }
-    const u64 surv = chunk + kMaxRuns + 16;
+    const u64 surv = entry_cap(chunk);
     if (w.surv_cap < surv) {
         drop_graphs(w);
         w.surv_cap = 0;
@@ -1331,7 +1331,7 @@ int time_sieve(mps_ctx* c, u64 lo, u64 K, u32 words, double* ms) {
     sa.hi = sa.lo_odd + 2 * sa.n_odds;
     sa.n_primes = sieve_prime_count(sa.hi);
     sa.n_split = split_for(c, K);
-    if (int r = ensure(c, &c->d_surv, &c->surv_cap, c->tun.chunk_odds + 16, "survivor buffer")) return r;
+    if (int r = ensure(c, &c->d_surv, &c->surv_cap, entry_cap(c->tun.chunk_odds), "survivor buffer")) return r;
     if (int r = ensure(c, &c->d_surv_split, &c->surv_split_cap, c->surv_cap, "split primes")) return r;
     const SurvOut out{c->d_surv, nullptr, c->d_surv_split, c->surv_cap};
     for (int rep = 0; rep < 4; ++rep) {
@@ -1546,7 +1546,7 @@ int mps_filter(mps_ctx* c, const uint64_t* primes, size_t n, const mps_item* ite
             item_few = few;
         }
         if (int r = ensure_rel(c, std::max<u64>(c->rel_cap, 1 << 18))) return r;
-        if (int r = ensure(c, &c->d_surv, &c->surv_cap, std::max<u64>(cnt + 16, chunk + 16), "survivor buffer")) return r;
+        if (int r = ensure(c, &c->d_surv, &c->surv_cap, std::max<u64>(cnt, entry_cap(chunk)), "survivor buffer")) return r;
         if (int r = ensure_entries(c, std::max<u64>(cnt, 1 << 16))) return r;
         u32 tbits, mb;
         table_for(c, g, d.K, &tbits, &mb);
@@ -1860,7 +1860,7 @@ int mps_count_primes(mps_ctx* c, uint64_t lo, uint64_t hi, uint64_t* count) {
         u64 b = hi;
         if (lo_odd < hi && (hi - lo_odd + 1) / 2 > chunk) b = lo_odd + 2 * chunk;
         const u64 n_odds = lo_odd < b ? (b - lo_odd + 1) / 2 : 0;
-        if (int r = ensure(c, &c->d_surv, &c->surv_cap, chunk + 16, "survivor buffer")) return r;
+        if (int r = ensure(c, &c->d_surv, &c->surv_cap, entry_cap(chunk), "survivor buffer")) return r;
         SieveArgs sa{};
         sa.lo_odd = lo_odd; sa.n_odds = n_odds; sa.hi = b; sa.include_two = (a <= 2 && b > 2);
         sa.n_primes = sieve_prime_count(b);

@@ -118,10 +118,11 @@ struct PrepArgs {
     u64 prime_below;           // survivors below this are prime (sieved by every prime up to their
                                // square root: 65521^2 for the sieve's survivors, 0 for caller-given numbers)
 };
-// Entries for a range of that many odd numbers: the primes of any such range (the
-// first one holds the most: pi(2 odds) stays below this, by 2% at 2^24 .. 2^26).
-// 168 B an entry (Entry, events, BSGS list): 21 B an odd number, and 16 B more
-// for the survivors and their split primes.
+// Survivors of the sieve and entries of a range of that many odd numbers: the primes of
+// any such range (the first one holds the most: pi(2 odds) stays below this, by 2% at
+// 2^24 .. 2^26).  Beyond 65521^2 the survivors are 0.101 of the odd numbers.  168 B an
+// entry (Entry, events, BSGS list) and 16 a survivor: 23 B an odd number.  (A range
+// that has more all the same is halved.)
 constexpr u64 entry_cap(u64 odds) { return odds / 8 + (1u << 17); }
 // Events of a size class's list and of a small-l list for ent_cap entries: a prime has
 // an l of a class with chance 1/4 at most (0.25 for 67 .. 251) and 0.72 small l on
